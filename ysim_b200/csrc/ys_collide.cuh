@@ -172,70 +172,50 @@ __device__ __forceinline__ bool root_overlap(const Node* __restrict__ a, const N
 }
 
 // ------------------------------------------------------------- H1 self rows
-// pointTriSq (spatial_hash.hpp:1659-1711).
+// pointTriSq (spatial_hash.hpp:1659-1711).  The seven regions share one
+// evaluation: all the products first, the region by the reference's tests in
+// its order, then q = base + t1 dir1 (+ t2 dir2) with the region's operands
+// -- each region's own expression, operation for operation -- so the lanes of
+// a warp run it together instead of one region after another.
 __device__ __forceinline__ float point_tri_sq(const float p[3], const float a[3], const float b[3], const float c[3]) {
-    float ab[3], ac[3], ap[3], q[3];
+    float ab[3], ac[3], ap[3], bp[3], cp[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) { ab[i] = b[i] - a[i]; ac[i] = c[i] - a[i]; ap[i] = p[i] - a[i]; }
+    for (int i = 0; i < 3; ++i) {
+        ab[i] = b[i] - a[i]; ac[i] = c[i] - a[i]; ap[i] = p[i] - a[i];
+        bp[i] = p[i] - b[i]; cp[i] = p[i] - c[i];
+    }
     const float d1 = ab[0] * ap[0] + ab[1] * ap[1] + ab[2] * ap[2];
     const float d2 = ac[0] * ap[0] + ac[1] * ap[1] + ac[2] * ap[2];
-    if (d1 <= 0.f && d2 <= 0.f) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) q[i] = a[i];
-    } else {
-        float bp[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) bp[i] = p[i] - b[i];
-        const float d3 = ab[0] * bp[0] + ab[1] * bp[1] + ab[2] * bp[2];
-        const float d4 = ac[0] * bp[0] + ac[1] * bp[1] + ac[2] * bp[2];
-        if (d3 >= 0.f && d4 <= d3) {
-#pragma unroll
-            for (int i = 0; i < 3; ++i) q[i] = b[i];
-        } else {
-            const float vc = d1 * d4 - d3 * d2;
-            if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) {
-                const float den = d1 - d3;
-                const float vv = (den != 0.f) ? d1 / den : 0.f;
-#pragma unroll
-                for (int i = 0; i < 3; ++i) q[i] = a[i] + vv * ab[i];
-            } else {
-                float cp[3];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) cp[i] = p[i] - c[i];
-                const float d5 = ab[0] * cp[0] + ab[1] * cp[1] + ab[2] * cp[2];
-                const float d6 = ac[0] * cp[0] + ac[1] * cp[1] + ac[2] * cp[2];
-                if (d6 >= 0.f && d5 <= d6) {
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) q[i] = c[i];
-                } else {
-                    const float vb = d5 * d2 - d1 * d6;
-                    if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) {
-                        const float den = d2 - d6;
-                        const float w = (den != 0.f) ? d2 / den : 0.f;
-#pragma unroll
-                        for (int i = 0; i < 3; ++i) q[i] = a[i] + w * ac[i];
-                    } else {
-                        const float va = d3 * d6 - d5 * d4;
-                        if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
-                            const float den = (d4 - d3) + (d5 - d6);
-                            const float w = (den != 0.f) ? (d4 - d3) / den : 0.f;
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) q[i] = b[i] + w * (c[i] - b[i]);
-                        } else {
-                            const float den = va + vb + vc;
-                            const float vv = (den != 0.f) ? vb / den : 0.f;
-                            const float w = (den != 0.f) ? vc / den : 0.f;
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) q[i] = a[i] + ab[i] * vv + ac[i] * w;
-                        }
-                    }
-                }
-            }
-        }
-    }
+    const float d3 = ab[0] * bp[0] + ab[1] * bp[1] + ab[2] * bp[2];
+    const float d4 = ac[0] * bp[0] + ac[1] * bp[1] + ac[2] * bp[2];
+    const float d5 = ab[0] * cp[0] + ab[1] * cp[1] + ab[2] * cp[2];
+    const float d6 = ac[0] * cp[0] + ac[1] * cp[1] + ac[2] * cp[2];
+    const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    const float e43 = d4 - d3, e56 = d5 - d6;
+    enum { A_, B_, AB_, C_, AC_, BC_, IN_ };
+    const int r = (d1 <= 0.f && d2 <= 0.f)                   ? A_
+                  : (d3 >= 0.f && d4 <= d3)                  ? B_
+                  : (vc <= 0.f && d1 >= 0.f && d3 <= 0.f)    ? AB_
+                  : (d6 >= 0.f && d5 <= d6)                  ? C_
+                  : (vb <= 0.f && d2 >= 0.f && d6 <= 0.f)    ? AC_
+                  : (va <= 0.f && e43 >= 0.f && e56 >= 0.f)  ? BC_
+                                                             : IN_;
+    const float num = r == AB_ ? d1 : r == AC_ ? d2 : r == BC_ ? e43 : vb;
+    const float den = r == AB_ ? d1 - d3 : r == AC_ ? d2 - d6 : r == BC_ ? e43 + e56 : va + vb + vc;
+    const float t1 = (den != 0.f) ? num / den : 0.f;
+    float t2 = 0.f;
+    if (r == IN_) t2 = (den != 0.f) ? vc / den : 0.f;
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) { const float e = p[i] - q[i]; s += e * e; }
+    for (int i = 0; i < 3; ++i) {
+        const float base = (r == B_ || r == BC_) ? b[i] : r == C_ ? c[i] : a[i];
+        const float dir = r == AC_ ? ac[i] : r == BC_ ? c[i] - b[i] : ab[i];
+        float q = base + t1 * dir;
+        if (r == IN_) q = q + ac[i] * t2;
+        if (r == A_ || r == B_ || r == C_) q = base;
+        const float e = p[i] - q;
+        s += e * e;
+    }
     return s;
 }
 
@@ -292,24 +272,38 @@ __device__ __forceinline__ void h1_query_box(const H1Vertex& h, float m, f3& qmn
 // span_check = false skips the face's 64-cell test, for callers whose cell
 // size is this mesh's largest key-box extent computed from the same positions
 // (the refit's H1 extent): every key box then spans at most two cells.
-__device__ __forceinline__ bool h1_face_at(f3 P0, f3 P1, f3 P2, float m, float inv, const H1Vertex& h,
-                                           bool span_check) {
+// h1_key_box: the face's key box (false: a corner is not finite, the face
+// never entered the grid); h1_near: the distance test of a face whose key
+// box meets the vertex's.
+__device__ __forceinline__ bool h1_key_box(f3 P0, f3 P1, f3 P2, float m, float4& lo, float4& hi) {
     const float A[3] = {P0.x, P0.y, P0.z}, B[3] = {P1.x, P1.y, P1.z}, C[3] = {P2.x, P2.y, P2.z};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (!isfinite(A[a]) || !isfinite(B[a]) || !isfinite(C[a])) return false;
-    }
     float bmn[3], bmx[3];
+    bool finite = true;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        if (!isfinite(A[a]) || !isfinite(B[a]) || !isfinite(C[a])) finite = false;
         // std::min(p0, std::min(p1, p2))
         float mn12 = (C[a] < B[a]) ? C[a] : B[a];
-        float lo = (mn12 < A[a]) ? mn12 : A[a];
+        float l = (mn12 < A[a]) ? mn12 : A[a];
         float mx12 = (B[a] < C[a]) ? C[a] : B[a];
-        float hi = (A[a] < mx12) ? mx12 : A[a];
-        bmn[a] = lo - m;
-        bmx[a] = hi + m;
+        float h = (A[a] < mx12) ? mx12 : A[a];
+        bmn[a] = l - m;
+        bmx[a] = h + m;
     }
+    lo.x = bmn[0]; lo.y = bmn[1]; lo.z = bmn[2];
+    hi.x = bmx[0]; hi.y = bmx[1]; hi.z = bmx[2];
+    return finite;
+}
+__device__ __forceinline__ bool h1_near(f3 P0, f3 P1, f3 P2, float m, const H1Vertex& h) {
+    const float A[3] = {P0.x, P0.y, P0.z}, B[3] = {P1.x, P1.y, P1.z}, C[3] = {P2.x, P2.y, P2.z};
+    const float m2 = m * m;
+    return !(point_tri_sq(h.pc, A, B, C) > m2 && point_tri_sq(h.pp, A, B, C) > m2);
+}
+__device__ __forceinline__ bool h1_face_at(f3 P0, f3 P1, f3 P2, float m, float inv, const H1Vertex& h,
+                                           bool span_check) {
+    float4 lo, hi;
+    if (!h1_key_box(P0, P1, P2, m, lo, hi)) return false;
+    const float bmn[3] = {lo.x, lo.y, lo.z}, bmx[3] = {hi.x, hi.y, hi.z};
     if (span_check) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -320,9 +314,7 @@ __device__ __forceinline__ bool h1_face_at(f3 P0, f3 P1, f3 P2, float m, float i
     if (h.hi[0] < bmn[0] || h.lo[0] > bmx[0] || h.hi[1] < bmn[1] || h.lo[1] > bmx[1] || h.hi[2] < bmn[2] ||
         h.lo[2] > bmx[2])
         return false;
-    const float m2 = m * m;
-    if (point_tri_sq(h.pc, A, B, C) > m2 && point_tri_sq(h.pp, A, B, C) > m2) return false;
-    return true;
+    return h1_near(P0, P1, P2, m, h);
 }
 __device__ __forceinline__ bool h1_face(const float4* __restrict__ X, u32 voff, uint4 tri, u32 v, float m, float inv,
                                         const H1Vertex& h, bool span_check = true) {
@@ -350,12 +342,10 @@ __device__ __forceinline__ bool point_in_tri(f3 p, f3 e0, f3 e1) {
 }
 // narrow_pt_tri (bruteforce.metal:41-178) for one candidate: swept segment
 // xPrev -> x against the triangle plane; rsqrt written as 1/sqrt (IEEE).
-__device__ __forceinline__ bool narrow_one(f3 qcur, f3 qprev, f3 t0, f3 t1, f3 t2, float band, f3& nout, float& dout) {
-    f3 e0 = t1 - t0, e1 = t2 - t0;
-    f3 n = cross(e0, e1);
-    float nl2 = dot(n, n);
-    if (nl2 < 1e-12f) return false;
-    n = n * (1.0f / sqrtf(nl2));
+// narrow_plane is the part after the unit normal n.
+__device__ __forceinline__ bool narrow_plane(f3 qcur, f3 qprev, f3 t0, f3 t1, f3 t2, f3 n, float band, f3& nout,
+                                             float& dout) {
+    const f3 e0 = t1 - t0, e1 = t2 - t0;
     float dp = dot(n, qprev - t0), dc = dot(n, qcur - t0);
     float dref = (dp != 0.0f) ? dp : dc;
     if (dref < 0.0f) { n = -n; dp = -dp; dc = -dc; }
@@ -375,6 +365,12 @@ __device__ __forceinline__ bool narrow_one(f3 qcur, f3 qprev, f3 t0, f3 t1, f3 t
     nout = n;
     dout = dc;
     return true;
+}
+__device__ __forceinline__ bool narrow_one(f3 qcur, f3 qprev, f3 t0, f3 t1, f3 t2, float band, f3& nout, float& dout) {
+    const f3 n = cross(t1 - t0, t2 - t0);
+    const float nl2 = dot(n, n);
+    if (nl2 < 1e-12f) return false;
+    return narrow_plane(qcur, qprev, t0, t1, t2, n * (1.0f / sqrtf(nl2)), band, nout, dout);
 }
 
 // ------------------------------------------------------------- F / I

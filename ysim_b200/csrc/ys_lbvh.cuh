@@ -222,6 +222,53 @@ cudaError_t launch_range_lists(const RefitJob* jobsDev, u32 numJobs, u32 totalLe
 cudaError_t refit_levels_prepare();
 void launch_refit_levels(const RefitJob* jobsDev, const uint2* list, const u32* hoffDev, const u32* hostOff,
                          u32 top, cudaStream_t s);
+// ---- sorted-leaf groups: what the fused substep descends in the cube layout.
+// The leaves of a tree in sorted (Morton) order, and the boxes of every run
+// of 32, 1024 and 32768 of them: a 32-wide tree without child pointers, in
+// which a warp tests the 32 children of a node with one coalesced load.  A
+// box is two float4 (minimum, maximum); the runs of 32768 ("tops") and the
+// whole-mesh boxes ("roots") are 8 words each, six of them order-preserving
+// integers that only ever grow (~ford(min), ford(max); 0 = empty), so that
+// blocks reduce into them by atomicMax after one clear.
+//
+// A job is one mesh: GJ_KEY writes the key boxes of the CPU-hash self rows
+// (AABB +- margin, an empty box for a face with a non-finite corner), GJ_BOX
+// the boxes of the point queries (swept by v dt with GJ_SWEPT), each with its
+// own runs; GJ_REC the records of the candidate tests, per leaf {corner 0,
+// face}, {corner 1, -}, {corner 2, -}, {unit normal, 0 if the face is
+// degenerate}; GJ_ROOT the root box by faces; GJ_VERTS (alone) the root box
+// by vertices, for a mesh whose every vertex is on a face (the same set of
+// points then).
+enum : u32 { GJ_KEY = 1, GJ_BOX = 2, GJ_SWEPT = 4, GJ_REC = 8, GJ_ROOT = 16, GJ_VERTS = 32 };
+struct GroupJob {
+    const uint4* lvid;     // per sorted leaf (vertex ids, face), or null: leaf i is face i of facets
+    const u32* facets;
+    u32* maxExt;           // GJ_KEY: the H1 grid extent
+    u32 flags, voff, n;    // n leaves (GJ_VERTS: vertices)
+    u32 block0;            // first block of the launch working on this job
+    u32 keyL0, keyTop, boxL0, boxTop, rec, root;
+    float dt, margin;
+};
+struct GroupBufs {
+    float4 *l0, *l1, *l2;  // boxes of leaves, runs of 32 and of 1024 (pairs; a tree's first leaf is a multiple of 1024)
+    float4* rec;           // 4 per leaf
+    u32 *top, *root;       // 8 words per run of 32768 / per mesh
+};
+static constexpr u32 GROUP_BLOCK = 1024;    // leaves (or vertices) per block
+static constexpr u32 GROUP_TOP = 32768;
+__device__ __forceinline__ void group_acc_box(const u32* a, float lo[3], float hi[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const u32 l = a[k], h = a[3 + k];
+        lo[k] = l ? funord(~l) : __int_as_float(0x7F800000);
+        hi[k] = h ? funord(h) : -__int_as_float(0x7F800000);
+    }
+}
+// One launch over the jobs' blocks (blkJob: the job of each block).  The tops
+// and roots the jobs write were cleared before.
+void launch_refit_groups(const GroupJob* jobs, const u32* blkJob, u32 numBlocks, const float4* x, const float4* v,
+                         GroupBufs B, cudaStream_t s);
+
 // Leaves + bottom-up for every job (jobs in device memory, jobsHost mirrors
 // them for the launch size).
 void launch_refit(const RefitJob* jobsDev, u32 numJobs, u32 totalLeaves, u32* status, cudaStream_t s);

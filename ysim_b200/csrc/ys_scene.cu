@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ys_analytic.cuh"
@@ -58,7 +59,10 @@ struct MeshDev {
     u32 w4_off, w4_cap;  // wide nodes of this mesh's tree (cube layout)
     u32 shape;           // analytic collider: slot in the shape table
     u32 tmap;            // FastGridCloth: first of its 5 tensor maps (X[0..2], V[0..1]) or NO_PAIR
-    u32 pad[2];
+    // sorted-leaf groups (cube layout): first leaf and first top of the key
+    // boxes (CPU-hash self rows) and of the query boxes, first record, slot of
+    // the root box
+    u32 keyL0, keyTop, boxL0, boxTop, rec, root;
 };
 static constexpr u32 NO_SPRINGS = 0xFFFFFFFFu;
 static constexpr u32 NO_PAIR = 0xFFFFFFFFu;
@@ -84,8 +88,12 @@ struct StepArgs {
     // mask A; a vertex whose faces do not fit has both masks 0
     const uint2* own;
     const Node* nodes;
-    const Wide4* w4;  // 4-wide form of the trees (wide != 0)
+    const Wide4* w4;  // 4-wide form of the trees (wide != 0; the staged path descends it)
     u32 wide;
+    // sorted-leaf groups (wide != 0; the fused path descends them), the
+    // sorted leaves' (vertex ids, face) by mesh
+    GroupBufs grp;
+    const uint4* lvid;
     const u32* spr_off;
     const u32* spr_split;
     const u32* spr_nbr;
@@ -441,19 +449,32 @@ __device__ __forceinline__ void warp_count(unsigned long long* ctr, u32 v) {
 }
 
 // ------------------------------------------------------------------ fused
-// One thread per vertex, but the per-candidate work (the H1 face test with its
-// two point-triangle distances, and the narrow test) is not done inside the
-// thread's own tree descent, where a warp would run it with the few lanes that
-// reached a leaf on that iteration.  Descents only push (owner lane, mesh,
-// face) into a per-warp queue in shared memory; whenever 32 candidates wait,
-// the whole warp takes one each, fetching the owner's positions by shuffle.
-// Contacts go back to their owner through a per-warp buffer and are inserted
-// into the owner's sorted list, which keeps the MAXC smallest (mesh, face)
-// keys whatever the arrival order -- so results are those of a per-vertex
-// loop over candidates in descent order.
+// One lane per vertex, but neither the tree descents nor the per-candidate
+// work run in a lane's own control flow.
+//
+// Descent (cube layout): the warp descends each tree once for its vertices,
+// over the sorted-leaf groups: the boxes of runs of 32768, 1024 and 32 sorted
+// leaves.  At a node, lane c tests child c of 32 against the union of the
+// boxes of the vertices that meet the node -- one coalesced load for 32
+// boxes, and a warp whose vertices lie in several places goes on with a tight
+// union in each.  At a run of 32 leaves, lane = leaf, and each vertex whose
+// box meets the run's tests the 32 leaves at once.  (One descent per lane
+// over 4-wide nodes ran 17.3k warp instructions per warp on the
+// self-colliding 262k-vertex cloth at 18 of 32 lanes, its time the steps of
+// the slowest lane: 0.369 ms per substep in its contact phase, 0.280 ms so.)
+//
+// Candidates (record, mesh, owner lane) wait in a per-warp queue; whenever 32
+// do, the whole warp takes one each, fetching the owner's positions by
+// shuffle.  Contacts go back to their owner through a per-warp buffer and
+// are inserted into the owner's sorted list, which keeps the MAXC smallest
+// (mesh, face) keys whatever the arrival order -- so results are those of a
+// per-vertex loop over candidates in descent order.
+//
+// The binary trees of the reference layout (a leaf can be reached by several
+// paths there, once per path in the rows) keep one descent per lane.
 static constexpr int FUSED_WARPS = 4;  // 128-thread blocks
-static constexpr u32 WQ_CAP = 160;     // candidate queue: < 32 left over + up to 4 leaves per lane
-static constexpr u32 WC_CAP = 64;      // contact buffer between flushes
+static constexpr u32 WQ_CAP = 64;      // candidate queue: < 32 left over + up to one per lane
+static constexpr u32 WC_CAP = 32;      // contact buffer between flushes
 static constexpr u32 KEY_SELF = 32u;   // queue key: (mesh << 6) | KEY_SELF? | owner lane
 static constexpr unsigned FULL_MASK = 0xFFFFFFFFu;
 
@@ -462,7 +483,40 @@ struct WarpWork {
     u32 qk[WQ_CAP];
     VContact cb[WC_CAP];
     unsigned char co[WC_CAP];
+    float4 vlo[32], vhi[32];  // groups: per lane the box its candidates must meet; w of vlo = mesh-local vertex id
+    float tile[90];           // the rest of the warp's share of the tile's spring table
 };
+
+// The lanes' boxes as order-preserving integers, for unions over subsets.
+struct LaneBox {
+    u32 lo[3], hi[3];
+};
+__device__ __forceinline__ LaneBox lane_box(f3 lo, f3 hi) {
+    const u32 NEG = ford(-__int_as_float(0x7F800000)), POS = ford(__int_as_float(0x7F800000));
+    // a NaN coordinate meets every box: unbounded
+    return LaneBox{{lo.x != lo.x ? NEG : ford(lo.x), lo.y != lo.y ? NEG : ford(lo.y), lo.z != lo.z ? NEG : ford(lo.z)},
+                   {hi.x != hi.x ? POS : ford(hi.x), hi.y != hi.y ? POS : ford(hi.y), hi.z != hi.z ? POS : ford(hi.z)}};
+}
+__device__ __forceinline__ void lane_union(const LaneBox& L, bool on, f3& lo, f3& hi) {
+    u32 r[6];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        r[k] = __reduce_min_sync(FULL_MASK, on ? L.lo[k] : 0xFFFFFFFFu);
+        r[3 + k] = __reduce_max_sync(FULL_MASK, on ? L.hi[k] : 0u);
+    }
+    lo = mk(funord(r[0]), funord(r[1]), funord(r[2]));
+    hi = mk(funord(r[3]), funord(r[4]), funord(r[5]));
+}
+// overlap() without branches
+__device__ __forceinline__ bool meets(f3 qmn, f3 qmx, float4 n0, float4 n1) {
+    return !((qmx.x < n0.x) | (qmn.x > n1.x) | (qmx.y < n0.y) | (qmn.y > n1.y) | (qmx.z < n0.z) | (qmn.z > n1.z));
+}
+// The root box of a mesh (cube layout) from its accumulators.
+__device__ __forceinline__ Node root_box(const StepArgs& A, const MeshDev* M) {
+    float lo[3], hi[3];
+    group_acc_box(A.grp.root + 8 * (size_t)M->root, lo, hi);
+    return Node{lo[0], lo[1], lo[2], 0, hi[0], hi[1], hi[2], 0};
+}
 
 __device__ __forceinline__ void insert_contact(VContact (&buf)[MAXC], int& nc, u32& st, const VContact& c) {
     if (nc == MAXC) {
@@ -483,10 +537,9 @@ __device__ __forceinline__ void insert_contact(VContact (&buf)[MAXC], int& nc, u
 // (PackedCollisionData::endAnalyticPairs, scene.hpp:485-530).  The cloth's
 // first vertex records this detect's mark for the next; the flags of the two
 // detects alternate between two slots by substep parity.
-__device__ __forceinline__ bool analytic_live(const StepArgs& A, const DShape& S, const Node* root, u32 p, bool writer) {
+__device__ __forceinline__ bool analytic_live(const StepArgs& A, const DShape& S, const Node& r, u32 p, bool writer) {
     bool fresh = true;
     if (S.lo.w != 0.f) {
-        const Node r = *root;
         fresh = !(S.hi.x < r.mnx || S.lo.x > r.mxx || S.hi.y < r.mny || S.lo.y > r.mxy || S.hi.z < r.mnz ||
                   S.lo.z > r.mxz);
     }
@@ -507,7 +560,7 @@ __device__ __noinline__ bool analytic_contact(const DShape* S, f3 pcur, f3 pprev
     return true;
 }
 
-// WIDE: descend the 4-wide form of the trees (cube layout), else the binary one.
+// GROUPS: descend the sorted-leaf groups (cube layout), else the binary trees.
 // MINB: CTAs per SM the registers are capped for (8: 64 registers, 7: 72,
 // 4: no cap); the results do not depend on it (ys_scene_autotune picks one).
 // ANA: the scene has analytic colliders (without them the kernel carries no
@@ -516,7 +569,7 @@ static constexpr u32 NO_VERTEX = 0xFFFFFFFFu;  // a padding slot of the thread o
 static_assert(sizeof(WarpWork) * FUSED_WARPS >= 3 * TILE_SPRINGS * sizeof(float),
               "the tile's spring table reuses the warps' queues");
 
-template <bool WIDE, int MINB, bool ANA>
+template <bool GROUPS, int MINB, bool ANA>
 __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
     __shared__ WarpWork wq[FUSED_WARPS];
     __shared__ unsigned long long tile_bar;
@@ -556,89 +609,9 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
     const f3 xpv = query ? ld(A.xp, g) : xc;
     const float mg = A.margin;
     u32 st = 0, rows = 0;
-    // own faces of this vertex: never a self row, dropped before the queue
-    const uint2 ownw = (query && A.own) ? A.own[g] : make_uint2(0u, 0u);
-    auto own_face = [&](u32 f) -> bool {
-        const u32 da = f - ownw.x, db = da - (ownw.y >> 16);
-        return (da < 8u && ((ownw.y >> da) & 1u)) || (db < 8u && ((ownw.y >> (8u + db)) & 1u));
-    };
-
-    // ---- descent state: the own tree first (set up here), then the targets
-    int stack[STACK_DEPTH];
-    int sp = 0;
-    auto push = [&](int v) -> bool {
-        if (sp >= STACK_DEPTH) return false;
-        stack[sp++] = v;
-        return true;
-    };
-    auto pop = [&]() -> int { return stack[--sp]; };
-    u32 visited = 0, nn = 0, key = 0;
-    const Node* nodes = A.nodes;  // binary form
-    const Wide4* wn = A.w4;       // wide form
-    f3 qmn = xc, qmx = xc;
-    float inv = 0.f;
-    // start a descent of mesh t's tree unless the query misses its root box
-    auto start = [&](u32 t, u32 k) {
-        const MeshDev* T = A.meshes + t;
-        key = k;
-        visited = 0;
-        if (WIDE) {
-            const float4* r = reinterpret_cast<const float4*>(A.nodes + T->node_off);
-            if (!overlap(qmn, qmx, __ldg(r), __ldg(r + 1))) return;
-            wn = A.w4 + T->w4_off;
-            nn = T->w4_cap;
-        } else {
-            nodes = A.nodes + T->node_off;
-            nn = 2 * T->nF - 1;
-        }
-        sp = 0;
-        push(0);
-    };
-    if (query && Mp->nF) {
-        bool selfOK = false;
-        if (A.self_mode == YS_SELF_HASH && (mflags & MF_CLOTH) && (mflags & MF_SELF)) {
-            float mx = __uint_as_float(A.maxext[m]);
-            float cs = (mx > 1e-5f) ? mx : 1e-5f;
-            inv = 1.f / cs;
-            H1Vertex h;
-            if (h1_vertex(xc, xpv, inv, h)) { selfOK = true; h1_query_box(h, mg, qmn, qmx); }
-        } else if (A.self_mode == YS_SELF_BVH && !(mflags & MF_ANALYTIC)) {
-            selfOK = true;
-            qmn = xc - mk(mg, mg, mg);
-            qmx = xc + mk(mg, mg, mg);
-        }
-        if (selfOK) start(m, (m << 6) | KEY_SELF | lane);
-    }
     VContact buf[MAXC];
     int nc = 0;
-    const u32 te = query ? Mp->tgt_end : 0u;
-    u32 tk = query ? Mp->tgt_begin : 0u;  // next target
-    auto next_tree = [&]() -> bool {
-        while (tk < te) {
-            const u32 k = tk++;
-            const u32 t = A.targets[k];
-            if (ANA && (A.meshes[t].flags & MF_ANALYTIC)) {
-                // narrowAnalytic for a marked (cloth, collider) pair: this
-                // vertex against the shape, no descent
-                const u32 p = A.tpair[k];
-                if (p == NO_PAIR) continue;
-                const DShape* S = A.shapes + A.meshes[t].shape;
-                VContact c;
-                if (analytic_live(A, *S, A.nodes + Mp->node_off, p, g == Mp->voff) &&
-                    analytic_contact(S, xc, xpv, A.radius, mg, &c))
-                    insert_contact(buf, nc, st, c);
-                continue;
-            }
-            if (ANA && (mflags & MF_ANALYTIC)) continue;  // no queries from an analytic collider
-            const u32 tno = A.meshes[t].node_off, tnf = A.meshes[t].nF;
-            if (tnf == 0 || !root_overlap(A.nodes + Mp->node_off, A.nodes + tno)) continue;
-            qmn = xc - mk(mg, mg, mg);
-            qmx = xc + mk(mg, mg, mg);
-            start(t, (t << 6) | lane);
-            if (sp) return true;
-        }
-        return false;
-    };
+    float inv = 0.f;
 
     u32 qn = 0, cn = 0;  // warp-uniform fill of the queue and of the contact buffer
 
@@ -667,31 +640,45 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
         VContact c;
         if (has) {
             const u32 t = k >> 6;
-            // the face's vertices in one 48-byte record (ids in w)
-            const float4* fp = A.fpos + 3 * (size_t)(A.meshes[t].foff + f);
-            const float4 q0 = __ldg(fp), q1 = __ldg(fp + 1), q2 = __ldg(fp + 2);
-            const f3 P0 = mk(q0.x, q0.y, q0.z), P1 = mk(q1.x, q1.y, q1.z), P2 = mk(q2.x, q2.y, q2.z);
             bool row = true;
-            if (k & KEY_SELF) {
-                const u32 lid = og - A.meshes[t].voff;
-                row = !(__float_as_uint(q0.w) == lid || __float_as_uint(q1.w) == lid || __float_as_uint(q2.w) == lid);
-                if (row && A.self_mode == YS_SELF_HASH) {
-                    // the owner passed its 64-cell check; the cell size is the
-                    // extent the refit just took from these positions
+            f3 n;
+            float d;
+            if (GROUPS) {
+                // f is a record; the descent queues a self face only when the
+                // owner is not one of its corners and its key box (or leaf
+                // box) meets the owner's box
+                const float4* fp = A.grp.rec + 4 * (size_t)f;
+                const float4 q0 = __ldg(fp), q1 = __ldg(fp + 1), q2 = __ldg(fp + 2), q3 = __ldg(fp + 3);
+                const f3 P0 = mk(q0.x, q0.y, q0.z), P1 = mk(q1.x, q1.y, q1.z), P2 = mk(q2.x, q2.y, q2.z);
+                if ((k & KEY_SELF) && A.self_mode == YS_SELF_HASH) {
                     H1Vertex h;
                     h1_vertex_box(oxc, oxp, h);
-                    row = h1_face_at(P0, P1, P2, mg, oinv, h, false);
+                    row = h1_near(P0, P1, P2, mg, h);
                 }
-            }
-            if (row) {
-                ++rows;
-                f3 n;
-                float d;
-                if (narrow_one(oxc, oxp, P0, P1, P2, A.band, n, d)) {
-                    hit = true;
-                    c = VContact{t, f, n.x, n.y, n.z, d};
+                rows += row ? 1u : 0u;
+                f = __float_as_uint(q0.w);
+                hit = row && q3.w != 0.f && narrow_plane(oxc, oxp, P0, P1, P2, mk(q3.x, q3.y, q3.z), A.band, n, d);
+            } else {
+                // the face's vertices in one 48-byte record (ids in w)
+                const float4* fp = A.fpos + 3 * (size_t)(A.meshes[t].foff + f);
+                const float4 q0 = __ldg(fp), q1 = __ldg(fp + 1), q2 = __ldg(fp + 2);
+                const f3 P0 = mk(q0.x, q0.y, q0.z), P1 = mk(q1.x, q1.y, q1.z), P2 = mk(q2.x, q2.y, q2.z);
+                if (k & KEY_SELF) {
+                    const u32 lid = og - A.meshes[t].voff;
+                    row = !(__float_as_uint(q0.w) == lid || __float_as_uint(q1.w) == lid ||
+                            __float_as_uint(q2.w) == lid);
+                    if (row && A.self_mode == YS_SELF_HASH) {
+                        // the owner passed its 64-cell check; the cell size is the
+                        // extent the refit just took from these positions
+                        H1Vertex h;
+                        h1_vertex_box(oxc, oxp, h);
+                        row = h1_face_at(P0, P1, P2, mg, oinv, h, false);
+                    }
                 }
+                rows += row ? 1u : 0u;
+                hit = row && narrow_one(oxc, oxp, P0, P1, P2, A.band, n, d);
             }
+            if (hit) c = VContact{t, f, n.x, n.y, n.z, d};
         }
         const unsigned hm = __ballot_sync(FULL_MASK, hit);
         if (hm) {
@@ -705,42 +692,222 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
         }
         __syncwarp();
     };
-    // warp-aggregated append of this lane's leaf (face >= 0) to the queue
-    auto enqueue = [&](int face) {
-        const unsigned lm = __ballot_sync(FULL_MASK, face >= 0);
-        if (lm) {
-            if (face >= 0) {
-                const u32 slot = qn + (u32)__popc(lm & ((1u << lane) - 1u));
-                Q.qf[slot] = (u32)face;
-                Q.qk[slot] = key;
-            }
-            qn += (u32)__popc(lm);
-        }
-    };
 
-    bool active = sp > 0 || next_tree();
-    while (true) {
-        if (active && sp == 0) active = next_tree();
-        if (!__ballot_sync(FULL_MASK, active)) break;
-        if (WIDE) {
-            int lf[4] = {-1, -1, -1, -1};
-            if (active) {
-                if (++visited > VISIT_CAP) {
-                    st |= ST_STACK_OVF;
-                    sp = 0;
+    if constexpr (GROUPS) {
+        // the warp's meshes one after another (a warp at the seam of two
+        // meshes has both); for each mesh its own tree, then its targets
+        unsigned todo = __ballot_sync(FULL_MASK, query && Mp->nF);
+        while (todo) {
+            const u32 gm = __shfl_sync(FULL_MASK, m, __ffs(todo) - 1);
+            const bool mine = ((todo >> lane) & 1u) && m == gm;
+            todo &= ~__ballot_sync(FULL_MASK, mine);
+            const MeshDev* __restrict__ GM = A.meshes + gm;
+            const u32 gflags = GM->flags, kb = GM->tgt_begin, ke = GM->tgt_end;
+            for (u32 k1 = kb; k1 <= ke; ++k1) {
+                // k1 = kb: the own tree; then target k1 - 1
+                const bool own = k1 == kb;
+                const u32 t = own ? gm : A.targets[k1 - 1];
+                const MeshDev* __restrict__ T = A.meshes + t;
+                const bool hash = own && A.self_mode == YS_SELF_HASH;
+                bool in = mine;
+                f3 blo = xc - mk(mg, mg, mg), bhi = xc + mk(mg, mg, mg);
+                u32 l0 = T->boxL0, top = T->boxTop;
+                if (hash) {
+                    if (!(gflags & MF_CLOTH) || !(gflags & MF_SELF)) continue;
+                    const float mx = __uint_as_float(A.maxext[gm]);
+                    H1Vertex h;
+                    in = mine && h1_vertex(xc, xpv, 1.f / ((mx > 1e-5f) ? mx : 1e-5f), h);
+                    if (in) {
+                        blo = mk(h.lo[0], h.lo[1], h.lo[2]);
+                        bhi = mk(h.hi[0], h.hi[1], h.hi[2]);
+                    }
+                    l0 = T->keyL0;
+                    top = T->keyTop;
+                } else if (own) {
+                    if (A.self_mode != YS_SELF_BVH || (gflags & MF_ANALYTIC)) continue;
                 } else {
-                    const int w = pop();
-                    if (w >= 0 && (u32)w < nn) {
-                        const bool selfTree = (key & KEY_SELF) != 0;
-                        st |= wide_step_p(wn, w, qmn, qmx, push, [&](int s, u32 f) {
-                            if (!(selfTree && own_face(f))) lf[s] = (int)f;
-                        });
+                    if (ANA && (T->flags & MF_ANALYTIC)) {
+                        // narrowAnalytic for a marked (cloth, collider) pair:
+                        // each vertex against the shape, no descent
+                        const u32 p = A.tpair[k1 - 1];
+                        if (p == NO_PAIR || !mine) continue;
+                        const DShape* S = A.shapes + T->shape;
+                        VContact c;
+                        if (analytic_live(A, *S, root_box(A, GM), p, g == GM->voff) &&
+                            analytic_contact(S, xc, xpv, A.radius, mg, &c))
+                            insert_contact(buf, nc, st, c);
+                        continue;
+                    }
+                    if (ANA && (gflags & MF_ANALYTIC)) continue;  // no queries from an analytic collider
+                    if (T->nF == 0) continue;
+                    // AABB4::intersect (bvh.hpp:64-69) of the two root boxes
+                    const Node a = root_box(A, GM), b = root_box(A, T);
+                    if (a.mxx < b.mnx || a.mnx > b.mxx || a.mxy < b.mny || a.mny > b.mxy || a.mxz < b.mnz || a.mnz > b.mxz)
+                        continue;
+                }
+                if (!__ballot_sync(FULL_MASK, in)) continue;
+                const u32 n = T->nF, n1 = (n + 31u) / 32u, n2 = (n + 1023u) / 1024u,
+                          n3 = (n + GROUP_TOP - 1u) / GROUP_TOP;
+                const float4* __restrict__ L0 = A.grp.l0 + 2 * (size_t)l0;
+                const float4* __restrict__ L1 = A.grp.l1 + 2 * (size_t)(l0 / 32u);
+                const float4* __restrict__ L2 = A.grp.l2 + 2 * (size_t)(l0 / 1024u);
+                const u32 key = (t << 6) | (own ? KEY_SELF : 0u), rec = T->rec;
+                const uint4* __restrict__ vids = A.lvid + T->foff;
+                __syncwarp();
+                Q.vlo[lane] = make_float4(blo.x, blo.y, blo.z, __uint_as_float(g - GM->voff));
+                Q.vhi[lane] = make_float4(bhi.x, bhi.y, bhi.z, 0.f);
+                __syncwarp();
+                const LaneBox LB = lane_box(blo, bhi);
+                f3 ulo, uhi;
+                for (u32 c3 = 0; c3 < n3; ++c3) {
+                    // a run of 32768 leaves: the vertices that meet it
+                    float tl[3], th[3];
+                    group_acc_box(A.grp.top + 8 * (size_t)(top + c3), tl, th);
+                    const bool in3 = in && meets(blo, bhi, make_float4(tl[0], tl[1], tl[2], 0.f),
+                                                 make_float4(th[0], th[1], th[2], 0.f));
+                    if (!__ballot_sync(FULL_MASK, in3)) continue;
+                    lane_union(LB, in3, ulo, uhi);
+                    const u32 k2 = c3 * 32u + lane;
+                    unsigned m2 = __ballot_sync(FULL_MASK, k2 < n2 && meets(ulo, uhi, __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u)),
+                                                                            __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u) + 1)));
+                    while (m2) {
+                        // a run of 1024
+                        const u32 c2 = c3 * 32u + (u32)__ffs(m2) - 1u;
+                        m2 &= m2 - 1u;
+                        const bool in2 = in3 && meets(blo, bhi, __ldg(L2 + 2 * (size_t)c2), __ldg(L2 + 2 * (size_t)c2 + 1));
+                        if (!__ballot_sync(FULL_MASK, in2)) continue;
+                        lane_union(LB, in2, ulo, uhi);
+                        const u32 k1c = c2 * 32u + lane;
+                        unsigned m1 = __ballot_sync(FULL_MASK, k1c < n1 && meets(ulo, uhi, __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u)),
+                                                                                 __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u) + 1)));
+                        while (m1) {
+                            // a run of 32 leaves: the vertices that meet it, each against the leaves
+                            const u32 c1 = c2 * 32u + (u32)__ffs(m1) - 1u;
+                            m1 &= m1 - 1u;
+                            unsigned vm = __ballot_sync(
+                                FULL_MASK, in2 && meets(blo, bhi, __ldg(L1 + 2 * (size_t)c1), __ldg(L1 + 2 * (size_t)c1 + 1)));
+                            if (!vm) continue;
+                            const u32 i = c1 * 32u + lane;
+                            const bool live = i < n;
+                            const u32 li = live ? i : n - 1u;
+                            const float4 lo = __ldg(L0 + 2 * (size_t)li), hi = __ldg(L0 + 2 * (size_t)li + 1);
+                            uint4 id = make_uint4(NO_VERTEX, NO_VERTEX, NO_VERTEX, 0u);
+                            if (own) id = __ldg(vids + li);
+                            do {
+                                const u32 v = (u32)__ffs(vm) - 1u;
+                                vm &= vm - 1u;
+                                const float4 a = Q.vlo[v], b = Q.vhi[v];
+                                const u32 lid = __float_as_uint(a.w);
+                                const bool hit = live & meets(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), lo, hi) &
+                                                 (id.x != lid) & (id.y != lid) & (id.z != lid);
+                                const unsigned hm = __ballot_sync(FULL_MASK, hit);
+                                if (hit) {
+                                    const u32 slot = qn + (u32)__popc(hm & ((1u << lane) - 1u));
+                                    Q.qf[slot] = rec + i;
+                                    Q.qk[slot] = key | v;
+                                }
+                                qn += (u32)__popc(hm);
+                                if (qn >= 32u) {
+                                    qn -= 32u;
+                                    drain(qn, 32);
+                                }
+                            } while (vm);
+                        }
                     }
                 }
             }
-#pragma unroll
-            for (int s = 0; s < 4; ++s) enqueue(lf[s]);
-        } else {
+        }
+    } else {
+        // own faces of this vertex: never a self row, dropped before the queue
+        const uint2 ownw = (query && A.own) ? A.own[g] : make_uint2(0u, 0u);
+        auto own_face = [&](u32 f) -> bool {
+            const u32 da = f - ownw.x, db = da - (ownw.y >> 16);
+            return (da < 8u && ((ownw.y >> da) & 1u)) || (db < 8u && ((ownw.y >> (8u + db)) & 1u));
+        };
+
+        // ---- descent state: the own tree first (set up here), then the targets
+        int stack[STACK_DEPTH];
+        int sp = 0;
+        auto push = [&](int v) -> bool {
+            if (sp >= STACK_DEPTH) return false;
+            stack[sp++] = v;
+            return true;
+        };
+        auto pop = [&]() -> int { return stack[--sp]; };
+        u32 visited = 0, nn = 0, key = 0;
+        const Node* nodes = A.nodes;
+        f3 qmn = xc, qmx = xc;
+        // start a descent of mesh t's tree
+        auto start = [&](u32 t, u32 k) {
+            const MeshDev* T = A.meshes + t;
+            key = k;
+            visited = 0;
+            nodes = A.nodes + T->node_off;
+            nn = 2 * T->nF - 1;
+            sp = 0;
+            push(0);
+        };
+        if (query && Mp->nF) {
+            bool selfOK = false;
+            if (A.self_mode == YS_SELF_HASH && (mflags & MF_CLOTH) && (mflags & MF_SELF)) {
+                float mx = __uint_as_float(A.maxext[m]);
+                float cs = (mx > 1e-5f) ? mx : 1e-5f;
+                inv = 1.f / cs;
+                H1Vertex h;
+                if (h1_vertex(xc, xpv, inv, h)) { selfOK = true; h1_query_box(h, mg, qmn, qmx); }
+            } else if (A.self_mode == YS_SELF_BVH && !(mflags & MF_ANALYTIC)) {
+                selfOK = true;
+                qmn = xc - mk(mg, mg, mg);
+                qmx = xc + mk(mg, mg, mg);
+            }
+            if (selfOK) start(m, (m << 6) | KEY_SELF | lane);
+        }
+        const u32 te = query ? Mp->tgt_end : 0u;
+        u32 tk = query ? Mp->tgt_begin : 0u;  // next target
+        auto next_tree = [&]() -> bool {
+            while (tk < te) {
+                const u32 k = tk++;
+                const u32 t = A.targets[k];
+                if (ANA && (A.meshes[t].flags & MF_ANALYTIC)) {
+                    // narrowAnalytic for a marked (cloth, collider) pair: this
+                    // vertex against the shape, no descent
+                    const u32 p = A.tpair[k];
+                    if (p == NO_PAIR) continue;
+                    const DShape* S = A.shapes + A.meshes[t].shape;
+                    VContact c;
+                    if (analytic_live(A, *S, A.nodes[Mp->node_off], p, g == Mp->voff) &&
+                        analytic_contact(S, xc, xpv, A.radius, mg, &c))
+                        insert_contact(buf, nc, st, c);
+                    continue;
+                }
+                if (ANA && (mflags & MF_ANALYTIC)) continue;  // no queries from an analytic collider
+                const u32 tno = A.meshes[t].node_off, tnf = A.meshes[t].nF;
+                if (tnf == 0 || !root_overlap(A.nodes + Mp->node_off, A.nodes + tno)) continue;
+                qmn = xc - mk(mg, mg, mg);
+                qmx = xc + mk(mg, mg, mg);
+                start(t, (t << 6) | lane);
+                if (sp) return true;
+            }
+            return false;
+        };
+
+        // warp-aggregated append of this lane's leaf (face >= 0) to the queue
+        auto enqueue = [&](int face) {
+            const unsigned lm = __ballot_sync(FULL_MASK, face >= 0);
+            if (lm) {
+                if (face >= 0) {
+                    const u32 slot = qn + (u32)__popc(lm & ((1u << lane) - 1u));
+                    Q.qf[slot] = (u32)face;
+                    Q.qk[slot] = key;
+                }
+                qn += (u32)__popc(lm);
+            }
+        };
+
+        bool active = sp > 0 || next_tree();
+        while (true) {
+            if (active && sp == 0) active = next_tree();
+            if (!__ballot_sync(FULL_MASK, active)) break;
             int leaf = -1;
             if (active) {
                 if (++visited > VISIT_CAP) {
@@ -766,10 +933,10 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
                 }
             }
             enqueue(leaf);
-        }
-        while (qn >= 32) {
-            drain(qn - 32, 32);
-            qn -= 32;
+            while (qn >= 32) {
+                drain(qn - 32, 32);
+                qn -= 32;
+            }
         }
     }
     if (qn) drain(0, qn);
@@ -941,7 +1108,7 @@ __global__ void __launch_bounds__(128) k_narrow_analytic_scene(StepArgs A) {
     const MeshDev& Q = A.meshes[P.x];
     const u32 id = i - P.w, g = Q.voff + id;
     const DShape& S = A.shapes[P.z];
-    if (!analytic_live(A, S, A.nodes + Q.node_off, lo, id == 0)) return;
+    if (!analytic_live(A, S, A.nodes[Q.node_off], lo, id == 0)) return;
     f3 n;
     float d;
     if (!analytic_narrow(S.s, ld(A.x, g), ld(A.xp, g), A.radius, A.margin, S.rot_margin, n, d)) return;
@@ -1159,6 +1326,13 @@ struct DBuf {
     void free() { if (p) cudaFree(p); p = nullptr; n = 0; }
 };
 
+// Part of another allocation.
+template <class T>
+struct DView {
+    T* p = nullptr;
+    size_t n = 0;
+};
+
 // MeshAdjacencyInitializer::initialize (mesh_state.hpp:236-411) restricted to
 // what the path consumes: vertexAdjFacets CSR, unique edges with rest
 // lengths, vertexAdjEdges and vertexOppVertices with rest lengths; merged
@@ -1243,12 +1417,26 @@ struct ys_scene {
     int cur = 0, prev = 1, cv = 0;
     bool snapshot_pending = false;
     DBuf<float> mass, mask;
-    DBuf<u32> vobj, targets, spr_off, spr_split, spr_nbr, vaf_off, vaf, maxext, status, codes, idx, visits, box;
+    DBuf<u32> vobj, targets, spr_off, spr_split, spr_nbr, vaf_off, vaf, status, codes, idx, visits, box;
     DBuf<float> spr_rest, scratch3;
     DBuf<uint4> F4;
     DBuf<u32> F3;  // packed facets (3 per face) for the refit kernel
     DBuf<float4> fpos;  // per face: its three vertex positions (id in w), for the fused kernel's tests
     DBuf<uint4> lvid;   // per sorted leaf: its face's vertex ids and the face id (range refit)
+    // sorted-leaf groups of the fused path (cube layout; GroupJob): boxes,
+    // records, tops and roots.  gzero holds, in this order, what a substep
+    // reduces into (the grid extents, the tops and roots of the meshes refit
+    // every substep, the counters: cleared by one memset), the running totals,
+    // and the tops and roots of the other meshes, written at their build.
+    DBuf<float4> gl0, gl1, gl2, grec;
+    DBuf<u32> gzero;
+    DView<u32> maxext, gacc;                    // grid extents; all tops and roots (8 words each)
+    size_t gclear = 0;                          // words of gzero before the counters
+    DBuf<GroupJob> gjobs;                       // per mesh build jobs, then the substep's jobs
+    DBuf<u32> gblk;                             // job of each block of the substep's refit
+    std::vector<GroupJob> hgbuild;              // per mesh: its build job (flags 0: none)
+    u32 ngjobs = 0, ngblocks = 0;
+    int refit_stale = -1;  // buffer pair (cur * 2 + cv) of a refit that left the 4-wide trees behind, or -1
     DBuf<uint2> own;    // per vertex: its own faces as two 8-face windows (StepArgs::own)
     DBuf<Node> nodes;
     DBuf<i32> parent, claims;        // largest claimant per node; claimant lists (offset node_off)
@@ -1285,7 +1473,7 @@ struct ys_scene {
     std::vector<RefitJob> hjobs;
     u32 njobs = 0;
     u32 refitLeaves = 0;
-    DBuf<unsigned long long> counters;
+    DView<unsigned long long> counters;  // inside gzero
     DBuf<float4> ext;
     bool use_ext = false;
     DBuf<float> gk, gL;              // per-spring grid-cloth parameters
@@ -1351,6 +1539,10 @@ ys_status check_scene(ys_scene* s) {
     return YS_OK;
 }
 
+GroupBufs group_bufs(ys_scene* s) {
+    return GroupBufs{s->gl0.p, s->gl1.p, s->gl2.p, s->grec.p, s->gacc.p, s->gacc.p};
+}
+
 StepArgs make_args(ys_scene* s) {
     StepArgs A;
     memset(&A, 0, sizeof(A));
@@ -1401,6 +1593,8 @@ StepArgs make_args(ys_scene* s) {
     A.vbuf = (u32)s->cv;
     A.tbase = 0;
     A.tend = s->nact;
+    A.grp = group_bufs(s);
+    A.lvid = s->lvid.p;
     A.self_mode = s->P.self_mode;
     A.record = s->record ? 1u : 0u;
     A.cap = s->cap;
@@ -1432,6 +1626,21 @@ u32* claim_off(ys_scene* s, const HostMesh& H) {
     return s->claimOff.p + H.node_off + (size_t)(&H - s->meshes.data());
 }
 
+// Sorted-leaf groups of a mesh that no substep refits, from its just sorted
+// leaves and the current positions (those of the others come from the next
+// substep's refit).
+void build_groups(ys_scene* s, size_t m) {
+    if (m >= s->hgbuild.size() || !s->hgbuild[m].flags) return;
+    const GroupJob& J = s->hgbuild[m];
+    const MeshDev& M = s->hmeshes[m];
+    cudaStream_t st = s->stream;
+    const u32 tops = (J.n + GROUP_TOP - 1) / GROUP_TOP;
+    if (J.flags & GJ_BOX) cudaMemsetAsync(s->gacc.p + 8 * (size_t)J.boxTop, 0, 32 * (size_t)tops, st);
+    if (J.flags & GJ_ROOT) cudaMemsetAsync(s->gacc.p + 8 * (size_t)M.root, 0, 32, st);
+    launch_refit_groups(s->gjobs.p + m, s->gblk.p + s->ngblocks, (J.n + GROUP_BLOCK - 1) / GROUP_BLOCK, s->X[s->cur].p,
+                        s->V[s->cv].p, group_bufs(s), st);
+}
+
 ys_status build_tree(ys_scene* s, HostMesh& H) {
     const u32 n = H.d.num_facets;
     if (n == 0) return YS_OK;
@@ -1458,8 +1667,10 @@ ys_status build_tree(ys_scene* s, HostMesh& H) {
         YS_CK(launch_wide_build(s->nodes.p + H.node_off, s->parent.p + H.node_off, n, s->w4.p + H.w4_off,
                                 s->leafW.p + H.foff, s->leafWf.p + H.foff, s->warrive.p + H.w4_off,
                                 s->wcount.p + (&H - s->meshes.data()), s->wideScratch.p, st));
-    k_face_pos<<<ceil_div(n, 256), 256, 0, st>>>(s->X[s->cur].p, H.voff, s->F3.p + 3 * (size_t)H.foff, n,
-                                                  s->fpos.p + 3 * (size_t)H.foff);
+    if (s->fpos.p)
+        k_face_pos<<<ceil_div(n, 256), 256, 0, st>>>(s->X[s->cur].p, H.voff, s->F3.p + 3 * (size_t)H.foff, n,
+                                                      s->fpos.p + 3 * (size_t)H.foff);
+    build_groups(s, (size_t)(&H - s->meshes.data()));
     RefitJob J;
     memset(&J, 0, sizeof(J));
     J.nodes = s->nodes.p + H.node_off;
@@ -1751,6 +1962,8 @@ ys_status encode_tile_maps(ys_scene* s) {
 
 // One k_fused launch per non-empty size class (classes do not interact:
 // each launch writes only its own vertices' next state).
+ys_status refresh_wide(ys_scene* s);
+
 void launch_fused_classes(ys_scene* s, StepArgs A) {
     for (size_t c = 0; c + 1 < s->cls_off.size(); ++c) {
         A.tbase = s->cls_off[c];
@@ -1768,6 +1981,8 @@ ys_status preamble(ys_scene* s) {
     }
     if (s->P.rebuild_frames && s->frame % s->P.rebuild_frames == 0) {
         bool rebuilt = false;
+        ys_status rw = refresh_wide(s);  // trees not rebuilt below keep the last substep's boxes
+        if (rw) return rw;
         for (auto& H : s->meshes) {
             if (H.built && H.d.behavior == YS_FLOAT) continue;
             if (!H.needs_tree) continue;  // its root box comes from the root-only refit
@@ -1788,6 +2003,7 @@ ys_status preamble(ys_scene* s) {
 // Refit of every live tree (the analytic markers are taken from the new root
 // boxes by the kernels that consume them).
 ys_status refit(ys_scene* s) {
+    s->refit_stale = -1;
     if (s->nrjobs)
         launch_root_boxes(s->rjobs.p + (size_t)(s->cur * 2 + s->cv) * s->nrjobs, s->nrjobs, s->rchunks.p,
                           s->nrchunks, s->stream);
@@ -1804,6 +2020,43 @@ ys_status refit(ys_scene* s) {
         if (s->nRootOnly) launch_refit_roots(table, s->njobs, s->stream);
     }
     return YS_OK;
+}
+
+// What the fused substep reads of the trees at the current positions: the
+// sorted-leaf groups (cube layout; the 4-wide trees then stay as they are
+// until someone asks for them, see refresh_wide) or the binary trees.  Clears
+// the substep's counters as well.
+ys_status refit_fused(ys_scene* s) {
+    const size_t cnt = s->record ? 24 : 16;  // counters [0] [1] ([2]: the record pool); [3] [4] keep running totals
+    if (s->tree_layout != YS_TREE_CUBE) {
+        ys_status r = refit(s);
+        if (r) return r;
+        YS_CK(cudaMemsetAsync(s->counters.p, 0, cnt, s->stream));
+        return YS_OK;
+    }
+    YS_CK(cudaMemsetAsync(s->gzero.p, 0, 4 * s->gclear + cnt, s->stream));
+    launch_refit_groups(s->gjobs.p + s->meshes.size(), s->gblk.p, s->ngblocks, s->X[s->cur].p, s->V[s->cv].p,
+                        group_bufs(s), s->stream);
+    return YS_OK;
+}
+
+void mark_refit(ys_scene* s) {
+    if (s->tree_layout == YS_TREE_CUBE) s->refit_stale = s->cur * 2 + s->cv;
+}
+
+// The 4-wide trees as the last fused substep's refit would have left them
+// (that substep's buffers hold its positions and velocities until the next
+// one).  Called by whoever reads the wide trees or overwrites those buffers.
+ys_status refresh_wide(ys_scene* s) {
+    if (s->refit_stale < 0 || s->njobs == 0) return YS_OK;
+    const int cur = s->cur, cv = s->cv;
+    s->cur = s->refit_stale / 2;
+    s->cv = s->refit_stale % 2;
+    s->refit_stale = -1;
+    const ys_status r = refit(s);
+    s->cur = cur;
+    s->cv = cv;
+    return r;
 }
 
 ys_status ensure_staged(ys_scene* s) {
@@ -1888,9 +2141,8 @@ void drop_graphs(ys_scene* s) {
 
 // Enqueue the device work of one fused substep (no preamble, no rotation).
 ys_status enqueue_fused(ys_scene* s) {
-    ys_status r = refit(s);
+    ys_status r = refit_fused(s);
     if (r) return r;
-    YS_CK(cudaMemsetAsync(s->counters.p, 0, s->record ? 24 : 16, s->stream));
     StepArgs A = make_args(s);
     launch_fused_classes(s, A);
     YS_CK(cudaGetLastError());
@@ -1923,6 +2175,7 @@ ys_status fused_substep(ys_scene* s) {
             if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
         }
         YS_CK(cudaGraphLaunch(s->graphs[key], s->stream));
+        mark_refit(s);
         s->snapshot_pending = true;
         rotate(s);
         return YS_OK;
@@ -1931,18 +2184,15 @@ ys_status fused_substep(ys_scene* s) {
         s->evRefit.push_back(s->evUsed);
         YS_CK(cudaEventRecord(next_event(s), s->stream));
     }
-    r = refit(s);
-    if (r) return r;
-    if (s->timing) {
-        YS_CK(cudaEventRecord(next_event(s), s->stream));
-    }
     if (s->record) {
         r = ensure_record(s);
         if (r) return r;
-        YS_CK(cudaMemsetAsync(s->counters.p, 0, 24, s->stream));
-    } else {
-        // counters [0] [1] only; [3] [4] keep running totals
-        YS_CK(cudaMemsetAsync(s->counters.p, 0, 16, s->stream));
+    }
+    r = refit_fused(s);
+    if (r) return r;
+    mark_refit(s);
+    if (s->timing) {
+        YS_CK(cudaEventRecord(next_event(s), s->stream));
     }
     StepArgs A = make_args(s);
     if (s->timing) {
@@ -1955,6 +2205,116 @@ ys_status fused_substep(ys_scene* s) {
     s->snapshot_pending = true;
     rotate(s);
     if (s->record) s->last_contacts = 2;
+    return YS_OK;
+}
+
+// Sorted-leaf groups of a cube-layout scene: which boxes each mesh needs, where
+// they lie, and the jobs that write them.
+//   key boxes    self rows of the CPU-hash semantics
+//   query boxes  a target of some query mesh, or BVH self rows
+//   root box     the inter-object cull of a query mesh and its targets
+// Meshes refit every substep (all but the static ones; a static self-hash
+// cloth needs the grid extent) are the substep's jobs; the others are written at
+// their build.
+ys_status group_layout(ys_scene* s, std::vector<MeshDev>& md, const std::vector<u32>& targets) {
+    const size_t nm = s->meshes.size();
+    std::vector<u32> need(nm, 0);
+    std::vector<char> live(nm, 0);
+    for (size_t m = 0; m < nm; ++m) {
+        const HostMesh& H = s->meshes[m];
+        if (!(H.flags & MF_QUERY) || !(H.flags & MF_TREE)) continue;
+        if (s->P.self_mode == YS_SELF_HASH && (H.flags & MF_CLOTH) && (H.flags & MF_SELF)) {
+            need[m] |= GJ_KEY | GJ_REC;
+            live[m] = 1;
+        }
+        if (s->P.self_mode == YS_SELF_BVH) need[m] |= GJ_BOX | GJ_REC;
+        for (u32 k = md[m].tgt_begin; k < md[m].tgt_end; ++k) {
+            need[m] |= GJ_ROOT;  // the cull, or an analytic marker
+            const HostMesh& T = s->meshes[targets[k]];
+            if (!(T.flags & MF_ANALYTIC) && !(H.flags & MF_ANALYTIC)) need[targets[k]] |= GJ_BOX | GJ_REC | GJ_ROOT;
+        }
+    }
+    if (s->tree_layout != YS_TREE_CUBE) std::fill(need.begin(), need.end(), 0u);
+    u32 l0 = 0, rec = 0, dyn = 0, fix = 0;
+    std::vector<GroupJob> build(nm), step;
+    for (size_t m = 0; m < nm; ++m) {
+        const HostMesh& H = s->meshes[m];
+        live[m] = (live[m] || !(H.flags & MF_STATIC)) ? 1 : 0;
+        memset(&build[m], 0, sizeof(GroupJob));
+        if (H.d.num_facets == 0) need[m] = 0;
+        const u32 n = H.d.num_facets, tops = (n + GROUP_TOP - 1) / GROUP_TOP, span = (n + GROUP_BLOCK - 1) / GROUP_BLOCK * GROUP_BLOCK;
+        u32& acc = live[m] ? dyn : fix;
+        MeshDev& M = md[m];
+        if (need[m] & GJ_KEY) { M.keyL0 = l0; M.keyTop = acc; l0 += span; acc += tops; }
+        if (need[m] & GJ_BOX) { M.boxL0 = l0; M.boxTop = acc; l0 += span; acc += tops; }
+        if (need[m] & GJ_REC) { M.rec = rec; rec += n; }
+        if (need[m] & GJ_ROOT) M.root = acc++;
+    }
+    // words: grid extents (padded to 16 bytes), dynamic accumulators, counters, static accumulators
+    const size_t ext = (nm + 3) & ~(size_t)3;
+    s->gclear = ext + 8 * (size_t)dyn;
+    YS_CK(s->gzero.alloc(s->gclear + 16 + 8 * (size_t)std::max(fix, 1u)));
+    YS_CK(cudaMemsetAsync(s->gzero.p, 0, 4 * s->gzero.n, s->stream));
+    s->maxext.p = s->gzero.p; s->maxext.n = nm;
+    s->gacc.p = s->gzero.p + ext; s->gacc.n = s->gzero.n - ext;
+    s->counters.p = reinterpret_cast<unsigned long long*>(s->gzero.p + s->gclear); s->counters.n = 8;
+    YS_CK(s->gl0.alloc(2 * (size_t)std::max(l0, 1u)));
+    YS_CK(s->gl1.alloc(2 * (size_t)(l0 / 32 + 1)));
+    YS_CK(s->gl2.alloc(2 * (size_t)(l0 / GROUP_BLOCK + 1)));
+    YS_CK(s->grec.alloc(4 * (size_t)std::max(rec, 1u)));
+    const u32 past = dyn + 2;  // static accumulators follow the counters (16 words)
+    u32 blocks = 0, most = 1;
+    std::vector<u32> blk;
+    for (size_t m = 0; m < nm; ++m) {
+        const HostMesh& H = s->meshes[m];
+        MeshDev& M = md[m];
+        if (!live[m]) { M.keyTop += past; M.boxTop += past; M.root += past; }
+        if (!need[m]) continue;
+        GroupJob J;
+        memset(&J, 0, sizeof(J));
+        J.facets = s->F3.p + 3 * (size_t)H.foff;
+        J.lvid = (need[m] & GJ_REC) ? s->lvid.p + H.foff : nullptr;  // root only: any order of the faces
+        J.maxExt = s->maxext.p + m;
+        J.voff = H.voff; J.n = H.d.num_facets;
+        J.keyL0 = M.keyL0; J.keyTop = M.keyTop; J.boxL0 = M.boxL0; J.boxTop = M.boxTop; J.rec = M.rec; J.root = M.root;
+        J.dt = s->P.subh; J.margin = s->P.margin;
+        J.flags = need[m];
+        if (!live[m]) {
+            build[m] = J;
+            most = std::max(most, (J.n + GROUP_BLOCK - 1) / GROUP_BLOCK);
+            continue;
+        }
+        if (!(H.flags & MF_STATIC)) J.flags |= GJ_SWEPT;
+        auto add = [&](GroupJob q, u32 count) {
+            q.block0 = blocks;
+            const u32 nb = (count + GROUP_BLOCK - 1) / GROUP_BLOCK;
+            blk.insert(blk.end(), nb, (u32)step.size());
+            blocks += nb;
+            step.push_back(q);
+        };
+        std::vector<char> onFace(H.d.num_vertices, 0);
+        for (u32 v : H.F) onFace[v] = 1;
+        if ((J.flags & GJ_ROOT) && !(J.flags & GJ_BOX) &&
+            std::all_of(onFace.begin(), onFace.end(), [](char c) { return c != 0; })) {
+            GroupJob q = J;
+            q.flags = GJ_VERTS | (J.flags & GJ_SWEPT);
+            q.n = H.d.num_vertices;
+            add(q, q.n);
+            J.flags &= ~(u32)GJ_ROOT;
+        }
+        if (J.flags & ~(u32)GJ_SWEPT) add(J, J.n);
+    }
+    s->ngjobs = (u32)step.size();
+    s->ngblocks = blocks;
+    s->hgbuild = build;
+    std::vector<GroupJob> all(build);
+    all.insert(all.end(), step.begin(), step.end());
+    blk.resize(blocks + most, 0u);  // a build launch's blocks: job 0 of its one-job table
+    YS_CK(s->gjobs.alloc(all.size()));
+    YS_CK(s->gblk.alloc(blk.size()));
+    YS_CK(cudaMemcpyAsync(s->gjobs.p, all.data(), sizeof(GroupJob) * all.size(), cudaMemcpyHostToDevice, s->stream));
+    YS_CK(cudaMemcpyAsync(s->gblk.p, blk.data(), 4 * blk.size(), cudaMemcpyHostToDevice, s->stream));
+    YS_CK(cudaStreamSynchronize(s->stream));
     return YS_OK;
 }
 
@@ -1987,10 +2347,11 @@ ys_status ys_scene_destroy(ys_scene* s) {
     for (auto& b : s->X) b.free();
     for (auto& b : s->V) b.free();
     s->Fbuf.free(); s->mass.free(); s->mask.free(); s->vobj.free(); s->targets.free(); s->spr_off.free();
-    s->spr_split.free(); s->spr_nbr.free(); s->vaf_off.free(); s->vaf.free(); s->maxext.free(); s->status.free();
+    s->spr_split.free(); s->spr_nbr.free(); s->vaf_off.free(); s->vaf.free(); s->status.free();
+    s->gl0.free(); s->gl1.free(); s->gl2.free(); s->grec.free(); s->gzero.free(); s->gjobs.free(); s->gblk.free();
     s->codes.free(); s->idx.free(); s->lvid.free(); s->visits.free(); s->box.free(); s->spr_rest.free(); s->scratch3.free(); s->gk.free(); s->gL.free(); s->F4.free(); s->F3.free();
     s->nodes.free(); s->parent.free(); s->claims.free(); s->claimOff.free(); s->karrasScratch.free(); s->aggScratch.free(); s->rootAcc.free();
-    s->rjobs.free(); s->rchunks.free(); s->dmeshes.free(); s->jobs.free(); s->counters.free(); s->sortScratch.free();
+    s->rjobs.free(); s->rchunks.free(); s->dmeshes.free(); s->jobs.free(); s->sortScratch.free();
     s->w4.free(); s->leafW.free(); s->warrive.free(); s->wideScratch.free();
     s->leafWf.free(); s->wcount.free(); s->hacc.free(); s->wlist.free(); s->hcount.free(); s->hoff.free();
     s->hcursor.free();
@@ -2154,11 +2515,13 @@ ys_status ys_scene_pack(ys_scene* s) {
     YS_CK(s->spr_off.alloc(nV + 1)); YS_CK(s->spr_split.alloc(nV));
     YS_CK(s->spr_nbr.alloc(std::max<size_t>(spr_nbr.size(), 1))); YS_CK(s->spr_rest.alloc(std::max<size_t>(spr_rest.size(), 1)));
     YS_CK(s->vaf_off.alloc(nV + 1)); YS_CK(s->vaf.alloc(std::max<size_t>(vaf.size(), 1)));
-    YS_CK(s->maxext.alloc(s->meshes.size())); YS_CK(s->status.alloc(1)); YS_CK(s->box.alloc(8));
+    YS_CK(s->status.alloc(1)); YS_CK(s->box.alloc(8));
     YS_CK(s->codes.alloc(std::max(nF, 1u))); YS_CK(s->idx.alloc(std::max(nF, 1u))); YS_CK(s->lvid.alloc(std::max(nF, 1u))); YS_CK(s->visits.alloc(std::max(nF, 1u)));
     YS_CK(s->F4.alloc(std::max(nF, 1u))); YS_CK(s->F3.alloc(3 * (size_t)std::max(nF, 1u)));
-    YS_CK(s->fpos.alloc(3 * (size_t)std::max(nF, 1u)));
-    YS_CK(s->own.alloc(std::max(nV, 1u)));
+    if (s->tree_layout == YS_TREE_REFERENCE) {  // what the descent of the binary trees reads
+        YS_CK(s->fpos.alloc(3 * (size_t)std::max(nF, 1u)));
+        YS_CK(s->own.alloc(std::max(nV, 1u)));
+    }
     YS_CK(s->nodes.alloc(std::max(nNodes, 1u))); YS_CK(s->parent.alloc(std::max(nNodes, 1u)));
     YS_CK(s->claims.alloc(std::max(nNodes, 1u)));
     YS_CK(s->claimOff.alloc((size_t)nNodes + s->meshes.size() + 1));
@@ -2176,7 +2539,6 @@ ys_status ys_scene_pack(ys_scene* s) {
         YS_CK(s->hcount.alloc(MAX_LEVELS + 2)); YS_CK(s->hoff.alloc(MAX_LEVELS + 2));
         YS_CK(s->hcursor.alloc(MAX_LEVELS + 2));
     }
-    YS_CK(s->counters.alloc(8));
     YS_CK(s->sortScratch.alloc(sort_scratch_bytes(maxF)));
     // uploads
     DBuf<float> tmp3;
@@ -2199,11 +2561,15 @@ ys_status ys_scene_pack(ys_scene* s) {
         YS_CK(cudaMemcpyAsync(s->spr_rest.p, spr_rest.data(), 4 * spr_rest.size(), cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
     }
     YS_CK(cudaMemcpyAsync(s->vaf_off.p, vaf_off.data(), 4 * (size_t)(nV + 1), cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
-    YS_CK(cudaMemcpyAsync(s->own.p, ownw.data(), sizeof(uint2) * (size_t)nV, cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
+    if (s->own.p) YS_CK(cudaMemcpyAsync(s->own.p, ownw.data(), sizeof(uint2) * (size_t)nV, cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
     if (!vaf.empty()) YS_CK(cudaMemcpyAsync(s->vaf.p, vaf.data(), 4 * vaf.size(), cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
     if (nF) {
         YS_CK(cudaMemcpyAsync(s->F4.p, F4.data(), 16 * (size_t)nF, cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
         YS_CK(cudaMemcpyAsync(s->F3.p, F3.data(), 12 * (size_t)nF, cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
+    }
+    {
+        ys_status r = group_layout(s, md, targets);
+        if (r) return r;
     }
     YS_CK(cudaMemcpyAsync(s->dmeshes.p, md.data(), sizeof(MeshDev) * md.size(), cudaMemcpyHostToDevice, s->stream)); YS_CK(cudaStreamSynchronize(s->stream));
     s->hmeshes = md;
@@ -2251,8 +2617,6 @@ ys_status ys_scene_pack(ys_scene* s) {
         }
     }
     YS_CK(cudaMemsetAsync(s->status.p, 0, 4, s->stream));
-    YS_CK(cudaMemsetAsync(s->maxext.p, 0, 4 * s->meshes.size(), s->stream));
-    YS_CK(cudaMemsetAsync(s->counters.p, 0, 8 * s->counters.n, s->stream));
     // Which trees a query descends: the targets of every query mesh, and the
     // self-queried meshes.  A query mesh whose own tree nothing descends
     // still needs that tree's root box (the inter-object cull): a root-only
@@ -2322,7 +2686,7 @@ ys_status ys_scene_pack(ys_scene* s) {
             J.wcount = s->wcount.p + m;
             J.hacc = s->hacc.p + H.w4_off;
         }
-        if (!J.rootOnly) J.fpos = s->fpos.p + 3 * (size_t)H.foff;  // faces the fused kernel tests
+        if (!J.rootOnly && s->fpos.p) J.fpos = s->fpos.p + 3 * (size_t)H.foff;  // faces the fused kernel tests
         if (J.w4) { J.wrange = s->wrange.p + H.w4_off; J.idx = s->idx.p + H.foff; J.lvid = s->lvid.p + H.foff; }
         s->hjobs.push_back(J);
         // every job's leaves start on a 256-leaf boundary (the range refit's
@@ -2532,11 +2896,11 @@ ys_status ys_scene_autotune(ys_scene* s, uint32_t reps, int* chosen, float* ms_o
     cudaStream_t st = s->stream;
     const bool rec = s->record;
     s->record = false;
-    r = refit(s);  // trees of the current positions
-    if (r) { s->record = rec; return r; }
     unsigned long long saved[8];
     YS_CK(cudaMemcpyAsync(saved, s->counters.p, sizeof(saved), cudaMemcpyDeviceToHost, st));
     YS_CK(cudaStreamSynchronize(st));
+    if ((r = refit_fused(s))) { s->record = rec; return r; }
+    mark_refit(s);  // trees of the current positions
     cudaEvent_t e0, e1;
     YS_CK(cudaEventCreate(&e0));
     YS_CK(cudaEventCreate(&e1));
@@ -2584,11 +2948,11 @@ ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* 
     cudaStream_t st = s->stream;
     const bool rec = s->record;
     s->record = false;
-    r = refit(s);
-    if (r) { s->record = rec; return r; }
     unsigned long long saved[8];
     YS_CK(cudaMemcpyAsync(saved, s->counters.p, sizeof(saved), cudaMemcpyDeviceToHost, st));
     YS_CK(cudaStreamSynchronize(st));
+    if ((r = refit_fused(s))) { s->record = rec; return r; }
+    mark_refit(s);
     cudaEvent_t e0, e1;
     YS_CK(cudaEventCreate(&e0));
     YS_CK(cudaEventCreate(&e1));
@@ -2696,6 +3060,7 @@ ys_status ys_scene_set_state(ys_scene* s, int which, const float* in) {
     ys_status r = check_scene(s);
     if (r) return r;
     if (!in) return fail(YS_ERR_BAD_ARG, "null input");
+    if ((r = refresh_wide(s))) return r;
     DBuf<float> tmp;
     YS_CK(tmp.alloc(3 * (size_t)s->nV));
     YS_CK(cudaMemcpyAsync(tmp.p, in, 12 * (size_t)s->nV, cudaMemcpyHostToDevice, s->stream));
@@ -2874,6 +3239,7 @@ ys_status ys_scene_wide_tree(ys_scene* s, int mesh, void* out, uint32_t cap, uin
     *count = 0;
     HostMesh& H = s->meshes[mesh];
     if (s->tree_layout != YS_TREE_CUBE || !H.built || H.d.num_facets == 0) return YS_OK;
+    if ((r = refresh_wide(s))) return r;
     u32 n = 0;
     YS_CK(cudaMemcpyAsync(&n, s->wcount.p + mesh, 4, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
@@ -3107,6 +3473,7 @@ struct ys_adjoint {
 namespace {
 
 void restore_state(ys_scene* s, const float4* x, const float4* xp, const float4* v, uint64_t frame, u32 cursor) {
+    refresh_wide(s);
     const size_t bytes = sizeof(float4) * s->nV;
     cudaMemcpyAsync(s->X[s->cur].p, x, bytes, cudaMemcpyDeviceToDevice, s->stream);
     cudaMemcpyAsync(s->X[s->prev].p, xp, bytes, cudaMemcpyDeviceToDevice, s->stream);
