@@ -83,3 +83,17 @@ def test_box_sets(cuda_lib, oracle, self_mode):
                            thickness=cloth.thickness))
     spec.meshes = [cloth, *tiny[:2], other, loose, below, moving, *tiny[2:]]
     assert _against_oracle(oracle, spec, steps=4) > 0
+
+
+# one vertex past each count of vertices that fits a wave at 2, 4, 8 and 16 per warp, and that count
+@pytest.mark.parametrize("n", [8288, 8289, 16576, 16577, 33152, 33153, 66304, 66305])
+def test_vertices_per_warp(cuda_lib, oracle, n):
+    """The same states whatever the warps' share: a self-colliding cloth filled up with loose vertices to n."""
+    spec = _folded(60, 1)
+    cloth = spec.meshes[0]
+    k = n - cloth.nV
+    loose = np.random.default_rng(n).uniform(-0.3, 0.3, (k, 3)).astype(np.float32) + np.float32([0, 0.3, 0])
+    spec.meshes[0] = dataclasses.replace(
+        cloth, x=np.concatenate([cloth.x, loose]), v=np.concatenate([cloth.v, np.zeros_like(loose)]),
+        mass=np.full(n, 1e-2, np.float32), mask=np.ones(n, np.float32))
+    assert _against_oracle(oracle, spec, steps=2) > 0

@@ -123,6 +123,7 @@ struct StepArgs {
     // one class.
     const u32* vorder;
     u32 tbase, tend;
+    u32 vpw;  // vertices per warp; the lanes past them only help
     // tile thread order (a launch over a class in that order): each CTA of a
     // FastGridCloth is one 16 x 8 tile, whose positions and velocities with a
     // 2-vertex halo come into shared memory by two TMA loads through the
@@ -576,8 +577,8 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
     extern __shared__ unsigned char fused_dyn[];  // TILE_SMEM bytes in tile order, else none
     const u32 lane = threadIdx.x & 31u;
     WarpWork& Q = wq[threadIdx.x >> 5];
-    const u32 t = A.tbase + blockIdx.x * blockDim.x + threadIdx.x;
-    u32 g = t < A.tend ? A.vorder[t] : NO_VERTEX;
+    const u32 t = A.tbase + (blockIdx.x * FUSED_WARPS + (threadIdx.x >> 5)) * A.vpw + lane;
+    u32 g = (lane < A.vpw && t < A.tend) ? A.vorder[t] : NO_VERTEX;
     const bool valid = g != NO_VERTEX;
     if (!valid) g = 0u;
     // tile order: this CTA is one tile of a grid cloth when its first slot
@@ -1039,9 +1040,26 @@ void launch_fused_t(const StepArgs& A, dim3 g, dim3 b, cudaStream_t st, int minB
     }
 }
 
-void launch_fused(const StepArgs& A, cudaStream_t st, int minBlocks) {
+// Vertices per warp of a launch over n: the fewest that still fit one wave
+// (148 SMs x 28 warps).  Descents, candidates and contacts of a warp's vertices
+// follow one another, so a launch that leaves the chip idle is as long as its
+// busiest warp; past one wave the idle lanes of the forces and the descents'
+// shared steps cost more than they give.  Fused kernel with 2 / 4 / 8 / 16 / 32
+// vertices per warp, us: grid cloth landing, 1024 vertices 19 / 22 / 24 / 29 / 31,
+// 16,384 36 / 26 / 29 / 35 / 47, 65,536 96 / 58 / 44 / 43 / 54; folded cloth,
+// 9409 50 / 48 / 55 / 76 / 127, 40,000 195 / 142 / 128 / 113 / 168; drape,
+// 102,400 367 / 255 / 177 / 147 / 148.  The binary descent has one walk per
+// lane and shares nothing: always 32.
+u32 vertices_per_warp(u32 n) {
+    for (u32 v = 2; v < 32; v *= 2)
+        if (ceil_div(n, v) <= 148 * 28) return v;
+    return 32;
+}
+
+void launch_fused(StepArgs A, cudaStream_t st, int minBlocks) {
     if (A.tend <= A.tbase) return;
-    const dim3 g(ceil_div(A.tend - A.tbase, 128)), b(128);
+    A.vpw = (A.tiles || !A.wide) ? 32u : vertices_per_warp(A.tend - A.tbase);
+    const dim3 g(ceil_div(A.tend - A.tbase, FUSED_WARPS * A.vpw)), b(128);
     const size_t smem = A.tiles ? TILE_SMEM : 0;
     if (A.analytic) launch_fused_t<true>(A, g, b, st, minBlocks, smem);
     else launch_fused_t<false>(A, g, b, st, minBlocks, smem);
