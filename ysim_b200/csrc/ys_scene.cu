@@ -1201,6 +1201,20 @@ __global__ void k_pack4(const float* __restrict__ in, float4* __restrict__ out, 
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], 0.f);
 }
+// k_pack4 with the vertices of static meshes written to two more buffers (or
+// null) as well.
+__global__ void k_pack4_static(const float* __restrict__ in, float4* __restrict__ out, float4* __restrict__ o1,
+                               float4* __restrict__ o2, const u32* __restrict__ vobj,
+                               const MeshDev* __restrict__ meshes, u32 n) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 q = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], 0.f);
+    out[i] = q;
+    if (o1 && (meshes[vobj[i]].flags & MF_STATIC)) {
+        o1[i] = q;
+        if (o2) o2[i] = q;
+    }
+}
 __global__ void k_unpack4(const float4* __restrict__ in, float* __restrict__ out, u32 n) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { float4 q = in[i]; out[3 * i] = q.x; out[3 * i + 1] = q.y; out[3 * i + 2] = q.z; }
@@ -3075,12 +3089,12 @@ ys_status ys_scene_get_state(ys_scene* s, int which, float* out) {
     else if (which == 2) src = s->snapshot_pending ? s->X[s->cur].p : s->X[s->prev].p;
     else if (which == 3) { r = ensure_staged(s); if (r) return r; src = s->Fbuf.p; }
     else return fail(YS_ERR_BAD_ARG, "bad state id");
-    DBuf<float> tmp;
-    YS_CK(tmp.alloc(3 * (size_t)s->nV));
-    k_unpack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(src, tmp.p, s->nV);
-    YS_CK(cudaMemcpyAsync(out, tmp.p, 12 * (size_t)s->nV, cudaMemcpyDeviceToHost, s->stream));
+    // the scene's own staging buffer, kept between calls: an allocation and
+    // its release cost a call 0.1 to 20 ms of driver time on a busy host
+    if (!s->scratch3.p) YS_CK(s->scratch3.alloc(3 * (size_t)s->nV));
+    k_unpack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(src, s->scratch3.p, s->nV);
+    YS_CK(cudaMemcpyAsync(out, s->scratch3.p, 12 * (size_t)s->nV, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
-    tmp.free();
     return YS_OK;
 }
 
@@ -3088,32 +3102,24 @@ ys_status ys_scene_set_state(ys_scene* s, int which, const float* in) {
     ys_status r = check_scene(s);
     if (r) return r;
     if (!in) return fail(YS_ERR_BAD_ARG, "null input");
+    if (which < 0 || which > 2) return fail(YS_ERR_BAD_ARG, "bad state id");
     if ((r = refresh_wide(s))) return r;
-    DBuf<float> tmp;
-    YS_CK(tmp.alloc(3 * (size_t)s->nV));
-    YS_CK(cudaMemcpyAsync(tmp.p, in, 12 * (size_t)s->nV, cudaMemcpyHostToDevice, s->stream));
-    if (which == 0) k_pack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(tmp.p, s->X[s->cur].p, s->nV);
-    else if (which == 1) k_pack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(tmp.p, s->V[s->cv].p, s->nV);
-    else if (which == 2) k_pack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(tmp.p, s->X[s->prev].p, s->nV);
-    else { tmp.free(); return fail(YS_ERR_BAD_ARG, "bad state id"); }
+    if (!s->scratch3.p) YS_CK(s->scratch3.alloc(3 * (size_t)s->nV));
+    YS_CK(cudaMemcpyAsync(s->scratch3.p, in, 12 * (size_t)s->nV, cudaMemcpyHostToDevice, s->stream));
     // vertices of static meshes are never rewritten by a substep, so every
     // rotating buffer must hold the same values for them
-    if (which == 0 || which == 1)
-        for (auto& H : s->meshes) {
-            if (!(H.flags & MF_STATIC)) continue;
-            const size_t bytes = sizeof(float4) * H.d.num_vertices;
-            if (which == 0) {
-                for (int b = 0; b < 3; ++b)
-                    if (b != s->cur)
-                        YS_CK(cudaMemcpyAsync(s->X[b].p + H.voff, s->X[s->cur].p + H.voff, bytes,
-                                              cudaMemcpyDeviceToDevice, s->stream));
-            } else {
-                YS_CK(cudaMemcpyAsync(s->V[1 - s->cv].p + H.voff, s->V[s->cv].p + H.voff, bytes,
-                                      cudaMemcpyDeviceToDevice, s->stream));
-            }
-        }
+    float4 *dst = s->X[s->prev].p, *o1 = nullptr, *o2 = nullptr;
+    if (which == 0) {
+        dst = s->X[s->cur].p;
+        o1 = s->X[s->prev].p;
+        o2 = s->X[3 - s->cur - s->prev].p;
+    } else if (which == 1) {
+        dst = s->V[s->cv].p;
+        o1 = s->V[1 - s->cv].p;
+    }
+    k_pack4_static<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(s->scratch3.p, dst, o1, o2, s->vobj.p, s->dmeshes.p, s->nV);
+    YS_CK(cudaGetLastError());
     YS_CK(cudaStreamSynchronize(s->stream));
-    tmp.free();
     return YS_OK;
 }
 
@@ -3146,10 +3152,8 @@ ys_status ys_scene_set_external_forces(ys_scene* s, const float* host_ext) {
         return YS_OK;
     }
     if (!s->use_ext) drop_graphs(s);  // captured graphs read g * m, not the buffer
-    if (!s->ext.p) {
-        YS_CK(s->ext.alloc(s->nV));
-        YS_CK(s->scratch3.alloc(3 * (size_t)s->nV));
-    }
+    if (!s->ext.p) YS_CK(s->ext.alloc(s->nV));
+    if (!s->scratch3.p) YS_CK(s->scratch3.alloc(3 * (size_t)s->nV));
     YS_CK(cudaMemcpyAsync(s->scratch3.p, host_ext, 12 * (size_t)s->nV, cudaMemcpyHostToDevice, s->stream));
     k_pack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(s->scratch3.p, s->ext.p, s->nV);
     YS_CK(cudaGetLastError());
