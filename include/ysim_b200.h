@@ -195,11 +195,8 @@ ys_status ys_scene_set_fused_variant(ys_scene* s, int min_blocks);
  *     from the positions at every tree rebuild, so a warp's 32 vertices are a
  *     compact patch whose descents and candidate faces overlap;
  *   YS_ORDER_VERTEX: thread i takes vertex i;
- *   YS_ORDER_TILE: each CTA takes one 16 x 8 tile of a FastGridCloth (other
- *     meshes in vertex order, each from a CTA boundary); the tile's positions
- *     and velocities with a 2-vertex halo come into shared memory by TMA, and
- *     each stencil spring with an end in the tile is evaluated once for both
- *     of its ends (890 spring evaluations per tile instead of 1536).
+ *   YS_ORDER_TILE: a FastGridCloth's vertices in 16 x 8 tiles (other meshes in
+ *     vertex order, each from a multiple of 128 slots).
  * The results are the same, bit for bit, in every order.  No counterpart in
  * the reference (one Metal thread per vertex id). */
 #define YS_ORDER_VERTEX 0

@@ -85,8 +85,8 @@ def test_box_sets(cuda_lib, oracle, self_mode):
     assert _against_oracle(oracle, spec, steps=4) > 0
 
 
-# one vertex past each count of vertices that fits a wave at 2, 4, 8 and 16 per warp, and that count
-@pytest.mark.parametrize("n", [8288, 8289, 16576, 16577, 33152, 33153, 66304, 66305])
+# the last count of vertices with 2, 4, 8 and 16 per warp, and one more
+@pytest.mark.parametrize("n", [9472, 9473, 18944, 18945, 75776, 75777, 151552, 151553])
 def test_vertices_per_warp(cuda_lib, oracle, n):
     """The same states whatever the warps' share: a self-colliding cloth filled up with loose vertices to n."""
     spec = _folded(60, 1)

@@ -124,11 +124,12 @@ struct StepArgs {
     const u32* vorder;
     u32 tbase, tend;
     u32 vpw;  // vertices per warp; the lanes past them only help
-    // tile thread order (a launch over a class in that order): each CTA of a
-    // FastGridCloth is one 16 x 8 tile, whose positions and velocities with a
-    // 2-vertex halo come into shared memory by two TMA loads through the
-    // mesh's tensor maps (tmaps[tmap + xbuf], tmaps[tmap + 3 + vbuf])
-    u32 tiles, xbuf, vbuf;
+    // force kernels: the tiles of the grid cloths (mesh, row << 16 | column of
+    // the tile's first vertex); a tile's positions and velocities with a
+    // 2-vertex halo come into shared memory by two TMA loads through the mesh's
+    // tensor maps (tmaps[tmap + xbuf], tmaps[tmap + 3 + vbuf])
+    const uint2* ftiles;
+    u32 xbuf, vbuf;
     const CUtensorMap* tmaps;
     u32* status;
     unsigned long long* counters;  // [0] broad rows, [1] contacts, [2] pool fill, [3] [4] running totals of 0, 1
@@ -276,8 +277,8 @@ __device__ __forceinline__ f3 vertex_force(const StepArgs& A, const MeshDev& M, 
 }
 
 // ---------------------------------------------------------- grid-cloth tiles
-// In tile thread order a CTA's 128 threads are one 16 x 8 tile of a
-// FastGridCloth (tile-row-major, 16 vertices per tile row).  Each spring with
+// A CTA of k_force_tiles is one 16 x 8 tile of a FastGridCloth
+// (16 vertices per tile row).  Each spring with
 // an end in the tile is evaluated once, as the force on its first end a from
 // its second end b.  Seen from b the force is its negation, bit for bit (dx,
 // dv and the unit vector change sign exactly, the length and the scalar
@@ -301,8 +302,8 @@ static constexpr int TILE_W = 16, TILE_H = 8;
 static constexpr int HALO_W = TILE_W + 4, HALO_H = TILE_H + 4;  // the stencil reaches 2 vertices out
 static constexpr u32 TILE_BOX_BYTES = HALO_W * HALO_H * 16;      // one float4 buffer's tile
 static constexpr u32 TILE_FLAG_BYTES = 896;                      // one flag byte per tile spring
-// x and v tiles, then the spring flags; 128-byte aligned
-static constexpr size_t TILE_SMEM = 2 * TILE_BOX_BYTES + TILE_FLAG_BYTES + 128;
+// x and v tiles, then the spring flags
+static constexpr size_t TILE_SMEM = 2 * TILE_BOX_BYTES + TILE_FLAG_BYTES;
 // first spring of each family in the tile's table
 static constexpr u32 TS_SX = 0, TS_SY = 136, TS_HA = 280, TS_HB = 433, TS_BX = 586, TS_BY = 730;
 static constexpr u32 TILE_SPRINGS = 890;
@@ -449,6 +450,50 @@ __device__ __forceinline__ void warp_count(unsigned long long* ctr, u32 v) {
     }
 }
 
+// ------------------------------------------------------------------ forces
+// Velocity after the forces, v + (f subh / m) mask, of every cloth vertex into
+// the next state's velocities; k_fused applies the contacts to it.  The forces
+// need no tree, so these kernels run beside the refit, and the query's warps
+// neither carry the springs' code nor idle lanes through them.
+__device__ __forceinline__ void put_velocity(const StepArgs& A, u32 g, f3 vel, f3 force, float mass) {
+    vel = vel + ((force * A.subh) / mass) * A.mask[g];
+    A.vn[g] = make_float4(vel.x, vel.y, vel.z, 0.f);
+}
+
+// Every cloth vertex that no tile covers, one thread each, in vertex order.
+__global__ void __launch_bounds__(128) k_force_vertices(StepArgs A) {
+    const u32 g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= A.nV) return;
+    const MeshDev& M = A.meshes[A.vobj[g]];
+    if (!(M.flags & MF_CLOTH) || ((M.flags & MF_GRID) && M.tmap != NO_PAIR)) return;
+    const f3 vel = ld(A.v, g);
+    const float mass = A.mass[g];
+    put_velocity(A, g, vel, vertex_force(A, M, g, ld(A.x, g), vel, mass), mass);
+}
+
+// The grid cloths, one 16 x 8 tile per CTA (see "grid-cloth tiles" above).
+__global__ void __launch_bounds__(TILE_W * TILE_H) k_force_tiles(StepArgs A) {
+    __shared__ float sf[3 * TILE_SPRINGS];
+    __shared__ unsigned long long bar;
+    __shared__ __align__(128) float4 xs[TILE_SMEM / sizeof(float4)];
+    const uint2 t = A.ftiles[blockIdx.x];
+    const MeshDev& M = A.meshes[t.x];
+    const int r0 = (int)(t.y >> 16), c0 = (int)(t.y & 0xFFFFu), N = (int)M.grid_n;
+    if (threadIdx.x == 0) tile_load(xs, A.tmaps + M.tmap + A.xbuf, A.tmaps + M.tmap + 3 + A.vbuf, r0, c0, &bar);
+    __syncthreads();  // the barrier is initialised
+    if (!tile_wait(&bar) && threadIdx.x == 0) atomicOr(A.status, ST_ITER_CAP);
+    unsigned char* flags = reinterpret_cast<unsigned char*>(xs + 2 * HALO_W * HALO_H);
+    tile_springs(A, M, r0, c0, xs, xs + HALO_W * HALO_H, sf, flags);
+    __syncthreads();
+    const int ty = (int)threadIdx.x / TILE_W, tx = (int)threadIdx.x % TILE_W, row = r0 + ty, col = c0 + tx;
+    if (row >= N || col >= N) return;
+    const u32 g = M.voff + (u32)(row * N + col);
+    const float4 v4 = xs[HALO_W * HALO_H + (ty + 2) * HALO_W + tx + 2];
+    const f3 vel = mk(v4.x, v4.y, v4.z);
+    const float mass = A.mass[g];
+    put_velocity(A, g, vel, tile_force(base_force(A, g, vel, mass), N, row, col, ty, tx, sf, flags), mass);
+}
+
 // ------------------------------------------------------------------ fused
 // One lane per vertex, but neither the tree descents nor the per-candidate
 // work run in a lane's own control flow.
@@ -485,7 +530,6 @@ struct WarpWork {
     VContact cb[WC_CAP];
     unsigned char co[WC_CAP];
     float4 vlo[32], vhi[32];  // groups: per lane the box its candidates must meet; w of vlo = mesh-local vertex id
-    float tile[90];           // the rest of the warp's share of the tile's spring table
 };
 
 // The lanes' boxes as order-preserving integers, for unions over subsets.
@@ -567,41 +611,16 @@ __device__ __noinline__ bool analytic_contact(const DShape* S, f3 pcur, f3 pprev
 // ANA: the scene has analytic colliders (without them the kernel carries no
 // analytic branch).
 static constexpr u32 NO_VERTEX = 0xFFFFFFFFu;  // a padding slot of the thread order
-static_assert(sizeof(WarpWork) * FUSED_WARPS >= 3 * TILE_SPRINGS * sizeof(float),
-              "the tile's spring table reuses the warps' queues");
 
 template <bool GROUPS, int MINB, bool ANA>
 __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
     __shared__ WarpWork wq[FUSED_WARPS];
-    __shared__ unsigned long long tile_bar;
-    extern __shared__ unsigned char fused_dyn[];  // TILE_SMEM bytes in tile order, else none
     const u32 lane = threadIdx.x & 31u;
     WarpWork& Q = wq[threadIdx.x >> 5];
     const u32 t = A.tbase + (blockIdx.x * FUSED_WARPS + (threadIdx.x >> 5)) * A.vpw + lane;
     u32 g = (lane < A.vpw && t < A.tend) ? A.vorder[t] : NO_VERTEX;
     const bool valid = g != NO_VERTEX;
     if (!valid) g = 0u;
-    // tile order: this CTA is one tile of a grid cloth when its first slot
-    // (a tile's origin, never padding) is a vertex of one (block-uniform)
-    bool tile = false;
-    int tr0 = 0, tc0 = 0;
-    const MeshDev* TM = A.meshes;
-    // 128-byte aligned, kept a shared-memory pointer (an offset into fused_dyn)
-    float4* xs = reinterpret_cast<float4*>(fused_dyn + ((128u - (smem_u32(fused_dyn) & 127u)) & 127u));
-    if (A.tiles) {
-        const u32 g0 = A.vorder[A.tbase + blockIdx.x * blockDim.x];
-        if (g0 != NO_VERTEX) {
-            TM = A.meshes + A.vobj[g0];
-            if ((TM->flags & MF_GRID) && (TM->flags & MF_CLOTH) && TM->tmap != NO_PAIR) {
-                const u32 N = TM->grid_n, l0 = g0 - TM->voff;
-                tile = true;
-                tr0 = (int)(l0 / N);
-                tc0 = (int)(l0 % N);
-                if (threadIdx.x == 0)
-                    tile_load(xs, A.tmaps + TM->tmap + A.xbuf, A.tmaps + TM->tmap + 3 + A.vbuf, tr0, tc0, &tile_bar);
-            }
-        }
-    }
     const u32 m = valid ? A.vobj[g] : 0u;
     const MeshDev* __restrict__ Mp = A.meshes + m;
     const u32 mflags = Mp->flags;
@@ -943,34 +962,10 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
     if (qn) drain(0, qn);
     if (cn) flush();
 
-    // The tile's springs, once every warp is done with its queue (the table
-    // takes the queues' memory); the TMA loads ran during the descents.
-    float* sf = reinterpret_cast<float*>(wq);
-    if (tile) {
-        __syncthreads();  // also orders the barrier's initialisation before the waits
-        if (!tile_wait(&tile_bar)) st |= ST_ITER_CAP;
-        tile_springs(A, *TM, tr0, tc0, xs, xs + HALO_W * HALO_H, sf,
-                     reinterpret_cast<unsigned char*>(xs + 2 * HALO_W * HALO_H));
-        __syncthreads();
-    }
     if (valid && (mflags & MF_CLOTH)) {
-        f3 vel = ld(A.v, g);
-        const float mass = A.mass[g], mask = A.mask[g];
-        f3 force;
-        // by the tile layout every vertex of a tile CTA is in its tile; the
-        // test keeps any other vertex on the per-vertex stencil
-        const u32 N = TM->grid_n, lid = g - TM->voff;
-        const bool in = tile && Mp == TM;
-        const int row = in ? (int)(lid / N) : 0, col = in ? (int)(lid % N) : 0;
-        if (in && row >= tr0 && row < tr0 + TILE_H && col >= tc0 && col < tc0 + TILE_W)
-            force = tile_force(base_force(A, g, vel, mass), (int)N, row, col, row - tr0, col - tc0, sf,
-                               reinterpret_cast<const unsigned char*>(xs + 2 * HALO_W * HALO_H));
-        else
-            force = vertex_force(A, *Mp, g, xc, vel, mass);
-        f3 pos = xc;
-        vel = vel + ((force * A.subh) / mass) * mask;
+        f3 pos = xc, vel = ld(A.vn, g);  // the velocity after the forces
         contact_response(pos, vel, nc, Mp->thickness, [&](int i) { return buf[i]; });
-        pos = pos + (vel * A.subh) * mask;
+        pos = pos + (vel * A.subh) * A.mask[g];
         if (sanitize(pos, vel, xc)) st |= ST_NONFINITE;
         A.xn[g] = make_float4(pos.x, pos.y, pos.z, 0.f);
         A.vn[g] = make_float4(vel.x, vel.y, vel.z, 0.f);
@@ -1029,40 +1024,38 @@ enum : int { ORDER_VERTEX = 0, ORDER_MORTON = 1, ORDER_TILE = 2 };  // a class's
 static constexpr u32 CLASS_MAX[NCLASS] = {4096u, 16384u, 65536u, 0xFFFFFFFFu};
 
 template <bool ANA>
-void launch_fused_t(const StepArgs& A, dim3 g, dim3 b, cudaStream_t st, int minBlocks, size_t smem) {
+void launch_fused_t(const StepArgs& A, int g, cudaStream_t st, int minBlocks) {
     switch ((A.wide ? 0 : 10) + minBlocks) {
-        case 8: k_fused<true, 8, ANA><<<g, b, smem, st>>>(A); break;
-        case 7: k_fused<true, 7, ANA><<<g, b, smem, st>>>(A); break;
-        case 4: k_fused<true, 4, ANA><<<g, b, smem, st>>>(A); break;
-        case 18: k_fused<false, 8, ANA><<<g, b, smem, st>>>(A); break;
-        case 17: k_fused<false, 7, ANA><<<g, b, smem, st>>>(A); break;
-        default: k_fused<false, 4, ANA><<<g, b, smem, st>>>(A); break;
+        case 8: k_fused<true, 8, ANA><<<g, 128, 0, st>>>(A); break;
+        case 7: k_fused<true, 7, ANA><<<g, 128, 0, st>>>(A); break;
+        case 4: k_fused<true, 4, ANA><<<g, 128, 0, st>>>(A); break;
+        case 18: k_fused<false, 8, ANA><<<g, 128, 0, st>>>(A); break;
+        case 17: k_fused<false, 7, ANA><<<g, 128, 0, st>>>(A); break;
+        default: k_fused<false, 4, ANA><<<g, 128, 0, st>>>(A); break;
     }
 }
 
-// Vertices per warp of a launch over n: the fewest that still fit one wave
-// (148 SMs x 28 warps).  Descents, candidates and contacts of a warp's vertices
-// follow one another, so a launch that leaves the chip idle is as long as its
-// busiest warp; past one wave the idle lanes of the forces and the descents'
-// shared steps cost more than they give.  Fused kernel with 2 / 4 / 8 / 16 / 32
-// vertices per warp, us: grid cloth landing, 1024 vertices 19 / 22 / 24 / 29 / 31,
-// 16,384 36 / 26 / 29 / 35 / 47, 65,536 96 / 58 / 44 / 43 / 54; folded cloth,
-// 9409 50 / 48 / 55 / 76 / 127, 40,000 195 / 142 / 128 / 113 / 168; drape,
-// 102,400 367 / 255 / 177 / 147 / 148.  The binary descent has one walk per
-// lane and shares nothing: always 32.
+// Vertices per warp of a launch over n.  Descents, candidates and contacts of
+// a warp's vertices follow one another, so a launch that leaves the chip idle
+// is as long as its busiest warp; with fewer vertices per warp the steps that
+// they share are taken more often.  Fused kernel with 2 / 4 / 8 / 16 / 32, us:
+// grid cloth landing, 4096 vertices 17 / 19 / 21 / 27 / 38, 16,384 22 / 20 / 23 /
+// 30 / 43, 65,536 43 / 31 / 29 / 34 / 47; folded cloth, 9409 38 / 40 / 48 / 71 /
+// 121, 22,500 66 / 55 / 46 / 56 / 80, 40,000 131 / 107 / 101 / 96 / 158; drape,
+// 102,400 227 / 164 / 121 / 121 / 133, 160,000 - / 225 / 154 / 132 / 134, 262,144
+// - / 447 / 302 / 230 / 229; grid batch, 137,189 - / 59 / 42 / 40 / 47, 1.1M - /
+// 379 / 223 / 149 / 119.  The binary descent has one walk per lane and shares
+// nothing: always 32.
 u32 vertices_per_warp(u32 n) {
-    for (u32 v = 2; v < 32; v *= 2)
-        if (ceil_div(n, v) <= 148 * 28) return v;
-    return 32;
+    return n <= 9472u ? 2u : n <= 18944u ? 4u : n <= 75776u ? 8u : n <= 151552u ? 16u : 32u;
 }
 
 void launch_fused(StepArgs A, cudaStream_t st, int minBlocks) {
     if (A.tend <= A.tbase) return;
-    A.vpw = (A.tiles || !A.wide) ? 32u : vertices_per_warp(A.tend - A.tbase);
-    const dim3 g(ceil_div(A.tend - A.tbase, FUSED_WARPS * A.vpw)), b(128);
-    const size_t smem = A.tiles ? TILE_SMEM : 0;
-    if (A.analytic) launch_fused_t<true>(A, g, b, st, minBlocks, smem);
-    else launch_fused_t<false>(A, g, b, st, minBlocks, smem);
+    A.vpw = A.wide ? vertices_per_warp(A.tend - A.tbase) : 32u;
+    const int g = ceil_div(A.tend - A.tbase, FUSED_WARPS * A.vpw);
+    if (A.analytic) launch_fused_t<true>(A, g, st, minBlocks);
+    else launch_fused_t<false>(A, g, st, minBlocks);
 }
 
 // ------------------------------------------------------------------ staged
@@ -1542,7 +1535,12 @@ struct ys_scene {
     std::vector<int> cls_variant;    // CTAs per SM of each class's launch
     std::vector<int> cls_order;      // per class: ORDER_VERTEX, ORDER_MORTON or ORDER_TILE
     std::vector<u32> act_aoff;       // per mesh: first slot in vorder, or NO_PAIR (not working)
-    DBuf<CUtensorMap> tmaps;         // 5 per grid cloth: X[0..2], V[0..1] (tile order)
+    DBuf<CUtensorMap> tmaps;         // 5 per grid cloth: X[0..2], V[0..1]
+    DBuf<uint2> ftiles;              // tiles of the grid cloths with maps (StepArgs::ftiles)
+    u32 nftiles = 0;
+    bool force_vertices = false;     // some cloth has no tiles
+    cudaStream_t side = nullptr;     // the force kernels run here, beside the refit
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::vector<int> mesh_class;     // per mesh, or -1 (not working)
     DBuf<char> oscratch;
     int tree_layout = YS_TREE_CUBE;  // Morton normalisation of the scene trees
@@ -1621,6 +1619,7 @@ StepArgs make_args(ys_scene* s) {
     A.nV = s->nV;
     A.vorder = s->vorder.p;
     A.tmaps = s->tmaps.p;
+    A.ftiles = s->ftiles.p;
     A.xbuf = (u32)s->cur;
     A.vbuf = (u32)s->cv;
     A.tbase = 0;
@@ -1944,10 +1943,10 @@ ys_status compute_order(ys_scene* s) {
     return YS_OK;
 }
 
-// Tensor maps of the tile order: per grid cloth, each of X[0..2] and V[0..1]
-// as a 3-D float array {4 components, N columns, N rows} with a box of
-// {4, HALO_W, HALO_H}.  Without the driver's encoder the grid cloths keep no
-// maps, and their tile-order CTAs gather the stencil per vertex instead.
+// Tiles and tensor maps of the grid cloths' force kernel: per grid cloth, each
+// of X[0..2] and V[0..1] as a 3-D float array {4 components, N columns, N rows}
+// with a box of {4, HALO_W, HALO_H}.  Without the driver's encoder the grid
+// cloths keep no maps, and k_force_vertices gathers their stencils.
 ys_status encode_tile_maps(ys_scene* s) {
     using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1959,11 +1958,16 @@ ys_status encode_tile_maps(ys_scene* s) {
         encode = nullptr;
     std::vector<MeshDev> md = s->hmeshes;
     std::vector<CUtensorMap> maps;
+    std::vector<uint2> tiles;
     for (size_t m = 0; m < md.size(); ++m) {
         md[m].tmap = NO_PAIR;
         const HostMesh& H = s->meshes[m];
-        if (!encode || !(H.flags & MF_GRID) || !(H.flags & MF_CLOTH)) continue;
+        if (!(H.flags & MF_CLOTH)) continue;
         const u32 n = H.d.grid_n;
+        if (!encode || !(H.flags & MF_GRID) || n >= 65536u || (u64)n * n != H.d.num_vertices) {
+            s->force_vertices = true;
+            continue;
+        }
         const cuuint64_t dims[3] = {4, n, n};
         const cuuint64_t strides[2] = {16, 16 * (cuuint64_t)n};  // bytes, dims 1 and 2
         const cuuint32_t box[3] = {4, (cuuint32_t)HALO_W, (cuuint32_t)HALO_H};
@@ -1978,8 +1982,19 @@ ys_status encode_tile_maps(ys_scene* s) {
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
             if (ok) maps.push_back(tm);
         }
-        if (!ok) { maps.resize(first); continue; }
+        if (!ok) {
+            maps.resize(first);
+            s->force_vertices = true;
+            continue;
+        }
         md[m].tmap = first;
+        for (u32 r = 0; r < n; r += TILE_H)
+            for (u32 c = 0; c < n; c += TILE_W) tiles.push_back(make_uint2((u32)m, (r << 16) | c));
+    }
+    s->nftiles = (u32)tiles.size();
+    if (!tiles.empty()) {
+        YS_CK(s->ftiles.alloc(tiles.size()));
+        YS_CK(cudaMemcpyAsync(s->ftiles.p, tiles.data(), sizeof(uint2) * tiles.size(), cudaMemcpyHostToDevice, s->stream));
     }
     if (!maps.empty()) {
         YS_CK(s->tmaps.alloc(maps.size()));
@@ -1987,7 +2002,7 @@ ys_status encode_tile_maps(ys_scene* s) {
                               s->stream));
     }
     YS_CK(cudaMemcpyAsync(s->dmeshes.p, md.data(), sizeof(MeshDev) * md.size(), cudaMemcpyHostToDevice, s->stream));
-    YS_CK(cudaStreamSynchronize(s->stream));  // md and maps live on the host stack
+    YS_CK(cudaStreamSynchronize(s->stream));  // md, maps and tiles live on the host stack
     s->hmeshes = md;
     return YS_OK;
 }
@@ -1996,23 +2011,25 @@ ys_status refresh_wide(ys_scene* s);
 
 // The size classes' k_fused launches (classes do not interact: a launch
 // writes only its own vertices' next state).  Neighbouring classes of the same
-// register cap share one launch (in tile order or not), smallest meshes
+// register cap share one launch, smallest meshes
 // first: the few long warps of a small class then run beside the large
 // class's instead of before them (48 FastGrid instances of 16^2 to 256^2
 // vertices: 27 + 58 + 231 us one after another).
 void launch_fused_classes(ys_scene* s, StepArgs A) {
     const size_t n = s->cls_off.size() ? s->cls_off.size() - 1 : 0;
     for (size_t c = 0, e = 0; c < n; c = e) {
-        const bool tiles = s->cls_order[c] == ORDER_TILE;
         for (e = c + 1; e < n; ++e)
-            if (s->cls_off[e + 1] > s->cls_off[e] &&
-                (s->cls_variant[e] != s->cls_variant[c] || (s->cls_order[e] == ORDER_TILE) != tiles))
-                break;
+            if (s->cls_off[e + 1] > s->cls_off[e] && s->cls_variant[e] != s->cls_variant[c]) break;
         A.tbase = s->cls_off[c];
         A.tend = s->cls_off[e];
-        A.tiles = tiles ? 1u : 0u;
         launch_fused(A, s->stream, s->cls_variant[c]);
     }
+}
+
+// The force kernels of every cloth.
+void launch_forces(ys_scene* s, const StepArgs& A, cudaStream_t st) {
+    if (s->nftiles) k_force_tiles<<<s->nftiles, TILE_W * TILE_H, 0, st>>>(A);
+    if (s->force_vertices) k_force_vertices<<<ceil_div(s->nV, 128), 128, 0, st>>>(A);
 }
 
 ys_status preamble(ys_scene* s) {
@@ -2183,9 +2200,15 @@ void drop_graphs(ys_scene* s) {
 
 // Enqueue the device work of one fused substep (no preamble, no rotation).
 ys_status enqueue_fused(ys_scene* s) {
+    const StepArgs A = make_args(s);
+    // the forces beside the refit, on the scene's second stream
+    YS_CK(cudaEventRecord(s->fork, s->stream));
+    YS_CK(cudaStreamWaitEvent(s->side, s->fork, 0));
+    launch_forces(s, A, s->side);
+    YS_CK(cudaEventRecord(s->join, s->side));
     ys_status r = refit_fused(s);
+    YS_CK(cudaStreamWaitEvent(s->stream, s->join, 0));
     if (r) return r;
-    StepArgs A = make_args(s);
     launch_fused_classes(s, A);
     YS_CK(cudaGetLastError());
     return YS_OK;
@@ -2222,28 +2245,28 @@ ys_status fused_substep(ys_scene* s) {
         rotate(s);
         return YS_OK;
     }
-    if (s->timing) {
-        s->evRefit.push_back(s->evUsed);
-        YS_CK(cudaEventRecord(next_event(s), s->stream));
-    }
     if (s->record) {
         r = ensure_record(s);
         if (r) return r;
     }
-    r = refit_fused(s);
-    if (r) return r;
-    mark_refit(s);
-    if (s->timing) {
+    if (!s->timing) {
+        if ((r = enqueue_fused(s))) return r;
+    } else {
+        // one after another, with events around the refit and around the
+        // forces and the fused kernel
+        s->evRefit.push_back(s->evUsed);
         YS_CK(cudaEventRecord(next_event(s), s->stream));
-    }
-    StepArgs A = make_args(s);
-    if (s->timing) {
+        if ((r = refit_fused(s))) return r;
+        YS_CK(cudaEventRecord(next_event(s), s->stream));
+        const StepArgs A = make_args(s);
         s->evFused.push_back(s->evUsed);
         YS_CK(cudaEventRecord(next_event(s), s->stream));
+        launch_forces(s, A, s->stream);
+        launch_fused_classes(s, A);
+        YS_CK(cudaGetLastError());
+        YS_CK(cudaEventRecord(next_event(s), s->stream));
     }
-    launch_fused_classes(s, A);
-    YS_CK(cudaGetLastError());
-    if (s->timing) YS_CK(cudaEventRecord(next_event(s), s->stream));
+    mark_refit(s);
     s->snapshot_pending = true;
     rotate(s);
     if (s->record) s->last_contacts = 2;
@@ -2377,7 +2400,10 @@ ys_status ys_scene_create(ys_scene** out, const ys_sim_params* p, int device) {
     s->P = *p;
     if (s->P.cols_per_point == 0) s->P.cols_per_point = 15;
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) { delete s; return fail(YS_ERR_CUDA, cudaGetErrorString(e)); }
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming);
+    if (e != cudaSuccess) { ys_scene_destroy(s); return fail(YS_ERR_CUDA, cudaGetErrorString(e)); }
     *out = s;
     return YS_OK;
 }
@@ -2404,7 +2430,11 @@ ys_status ys_scene_destroy(ys_scene* s) {
     s->fpos.free(); s->own.free(); s->bb16.free(); s->bb256.free(); s->wrange.free(); s->blkEnt.free(); s->bigEnt.free();
     s->blkCnt.free(); s->blkOff.free(); s->bigCnt.free(); s->rangeScratch.free(); s->vorder.free(); s->okeys.free(); s->oaoff.free(); s->orank.free(); s->obox.free(); s->oscratch.free(); s->omorton.free();
     for (auto e : s->evPool) cudaEventDestroy(e);
-    cudaStreamDestroy(s->stream);
+    s->tmaps.free(); s->ftiles.free();
+    if (s->fork) cudaEventDestroy(s->fork);
+    if (s->join) cudaEventDestroy(s->join);
+    if (s->side) cudaStreamDestroy(s->side);
+    if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return YS_OK;
 }
@@ -2947,6 +2977,7 @@ ys_status ys_scene_autotune(ys_scene* s, uint32_t reps, int* chosen, float* ms_o
     YS_CK(cudaEventCreate(&e0));
     YS_CK(cudaEventCreate(&e1));
     const StepArgs A = make_args(s);
+    launch_forces(s, A, st);
     float best = 1e30f;
     int bestV = s->fused_min_blocks;
     for (int i = 0; i < 3; ++i) {
@@ -3003,7 +3034,7 @@ ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* 
         for (auto& o : s->cls_order) o = order;
         if ((r = order_layout(s)) || (r = compute_order(s))) break;
         StepArgs A = make_args(s);
-        A.tiles = order == ORDER_TILE ? 1u : 0u;
+        launch_forces(s, A, st);
         for (int c = 0; c < NCLASS; ++c) {
             A.tbase = s->cls_off[c];
             A.tend = s->cls_off[c + 1];

@@ -154,8 +154,8 @@ class Scene:
     def set_thread_order(self, order):
         """Fused-kernel threads over the working vertices in per-mesh Morton
         order ("morton" or True, default), vertex order ("vertex" or False),
-        or 16 x 8 tiles of each grid cloth with TMA-staged spring tables
-        ("tile"); the results are the same in every order."""
+        or 16 x 8 tiles of each grid cloth ("tile"); the results are the same
+        in every order."""
         if isinstance(order, str):
             code = _lib.ORDER_NAMES.index(order)
         else:
