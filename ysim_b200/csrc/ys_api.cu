@@ -62,15 +62,18 @@ struct ys_lbvh {
     QueryOrder qorder;        // Morton order of large query sets
     int builder = YS_BUILD_KARRAS;  // ys_lbvh_set_builder
     void* aggScratch = nullptr;     // Apetrei range ends and root slot
-    // range refit of a consistent Karras tree: per internal node its
-    // sorted-leaf range, the nodes whose range leaves their block, block boxes
+    // range refit of a Karras tree (BinRanges): per internal node its
+    // sorted-leaf range, the nodes whose range leaves their block, the nodes
+    // inside runs of equal codes and the leaves reached there, block boxes
     uint2* range = nullptr;
-    u32 *big = nullptr, *huge = nullptr, *bcount = nullptr;
+    u32 *big = nullptr, *huge = nullptr, *runs = nullptr, *reach = nullptr, *bcount = nullptr;
     Node *bb16 = nullptr, *bb256 = nullptr;
     u32* rank = nullptr;      // sorted-leaf position of each face
     float4* lbox = nullptr;   // leaf boxes in sorted order (face-order pass of the refit)
-    u32 nbig = 0, nhuge = 0;
-    bool ranged = false;            // the last build recorded ranges (consistent Karras split)
+    u32 nbig = 0, nhuge = 0, nruns = 0;
+    bool split = false;             // the last build's Karras split (consistent)
+    bool claimed = false;           // the claimant lists are the last build's
+    bool ranged = false;            // the last build's tree is refit by ranges (no long run of equal codes)
 };
 
 #define YS_CK2(call)                                                                                   \
@@ -106,7 +109,9 @@ ys_status ys_lbvh_create(ys_lbvh** out, uint32_t maxPrims, int device, void* str
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->range, (size_t)maxPrims * sizeof(uint2));
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->big, (size_t)maxPrims * 4);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->huge, (size_t)maxPrims * 4);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t->bcount, 8);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&t->runs, (size_t)maxPrims * 4);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&t->reach, ((size_t)maxPrims / 32 + 1) * 4);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&t->bcount, 20);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->bb16, ((size_t)maxPrims / 16 + 1) * sizeof(Node));
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->bb256, ((size_t)maxPrims / 256 + 1) * sizeof(Node));
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->rank, (size_t)maxPrims * 4);
@@ -129,7 +134,7 @@ ys_status ys_lbvh_destroy(ys_lbvh* t) {
     cudaStreamSynchronize(t->stream);
     cudaFree(t->nodes); cudaFree(t->parent); cudaFree(t->claimOff); cudaFree(t->claims); cudaFree(t->karrasScratch); cudaFree(t->aggScratch); cudaFree(t->codes); cudaFree(t->idx); cudaFree(t->visits);
     cudaFree(t->box); cudaFree(t->status); cudaFree(t->scratch); cudaFree(t->job);
-    cudaFree(t->range); cudaFree(t->big); cudaFree(t->huge); cudaFree(t->bcount); cudaFree(t->bb16); cudaFree(t->bb256);
+    cudaFree(t->range); cudaFree(t->big); cudaFree(t->huge); cudaFree(t->runs); cudaFree(t->reach); cudaFree(t->bcount); cudaFree(t->bb16); cudaFree(t->bb256);
     cudaFree(t->rank); cudaFree(t->lbox);
     query_order_free(t->qorder);
     delete t;
@@ -143,14 +148,24 @@ static ys_status run_refit(ys_lbvh* t, const float* x, const float* v, float dt,
     J.x3 = x; J.v3 = v; J.voff = 0; J.n = t->n; J.leafBase = 0; J.dt = dt; J.swept = swept ? 1u : 0u;
     J.selfMargin = 0.f; J.maxExt = t->box;
     if (t->ranged) {
-        // consistent tree: every internal box is the union of its sorted-leaf
-        // range, from the leaf pass's block boxes (no climb)
+        // every internal box is the union of its sorted-leaf range, from the
+        // leaf pass's block boxes (no climb)
         J.bb16 = t->bb16;
         J.bb256 = t->bb256;
-        launch_refit_bin(J, t->range, t->big, t->nbig, t->huge, t->nhuge, t->rank, t->lbox, t->stream);
+        u32* nan = t->bcount + 4;
+        if (!t->split) YS_CK2(cudaMemsetAsync(nan, 0, 4, t->stream));
+        launch_refit_bin(J, t->range, t->big, t->nbig, t->huge, t->nhuge, t->rank, t->lbox, t->stream,
+                         t->runs, t->nruns, t->reach, t->split ? nullptr : nan);
         YS_CK2(cudaGetLastError());
+        u32 found = 0;
+        if (!t->split) YS_CK2(cudaMemcpyAsync(&found, nan, 4, cudaMemcpyDeviceToHost, t->stream));
         YS_CK2(cudaStreamSynchronize(t->stream));
-        return YS_OK;
+        if (!found) return YS_OK;
+        // a NaN among the reference tree's boxes: the boxes its climb gives
+        if (!t->claimed) {
+            YS_CK2(launch_claims(t->nodes, t->n, t->claimOff, t->claims, t->karrasScratch, t->stream));
+            t->claimed = true;
+        }
     }
     YS_CK2(cudaMemcpyAsync(t->job, &J, sizeof(J), cudaMemcpyHostToDevice, t->stream));
     launch_refit(t->job, 1, t->n, t->status, t->stream);
@@ -189,21 +204,28 @@ ys_status ys_lbvh_build(ys_lbvh* t, const float* x, uint32_t nV, const uint32_t*
         YS_CK2(cudaStreamSynchronize(t->stream));
         return YS_OK;
     }
+    t->split = t->consistent;
+    t->claimed = false;
     BinRanges R;
-    if (t->consistent) {  // one parent per node: boxes are unions of contiguous sorted-leaf ranges
-        R.range = t->range; R.big = t->big; R.huge = t->huge; R.count = t->bcount;
-    }
+    R.range = t->range; R.big = t->big; R.huge = t->huge; R.runs = t->runs; R.count = t->bcount;
     YS_CK2(launch_karras(t->codes, t->idx, nF, t->nodes, t->parent, t->claimOff, t->claims, t->visits,
                          t->karrasScratch, t->stream, t->consistent, R));
-    YS_CK2(cudaGetLastError());
-    if (t->consistent) {
-        u32 cnt[2] = {0, 0};
-        YS_CK2(cudaMemcpyAsync(cnt, t->bcount, 8, cudaMemcpyDeviceToHost, t->stream));
-        YS_CK2(cudaStreamSynchronize(t->stream));
-        t->nbig = cnt[0];
-        t->nhuge = cnt[1];
-        t->ranged = true;
+    u32 cnt[4] = {0, 0, 0, 0};
+    YS_CK2(cudaMemcpyAsync(cnt, t->bcount, 16, cudaMemcpyDeviceToHost, t->stream));
+    YS_CK2(cudaStreamSynchronize(t->stream));
+    t->nbig = cnt[0];
+    t->nhuge = cnt[1];
+    t->nruns = cnt[2];
+    t->ranged = cnt[3] <= BIN_RUN_MAX;
+    if (t->ranged) {
+        if (t->nruns) {
+            YS_CK2(cudaMemsetAsync(t->reach, 0xFF, ((size_t)nF / 32 + 1) * 4, t->stream));
+            launch_run_reach(t->nodes, nF, t->range, t->codes, t->runs, t->nruns, t->reach, t->stream);
+        }
         launch_leaf_rank(t->idx, nF, t->rank, t->stream);
+    } else {
+        YS_CK2(launch_claims(t->nodes, nF, t->claimOff, t->claims, t->karrasScratch, t->stream));
+        t->claimed = true;
     }
     return run_refit(t, x, nullptr, 0.f, 0);
 }

@@ -161,7 +161,7 @@ struct KarrasView {
 __global__ void k_parent_init(i32* __restrict__ parent, u32* __restrict__ claimOff, u32 numNodes) {
     u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < numNodes) parent[i] = -1;
-    if (i <= numNodes) claimOff[i] = 0;
+    if (claimOff && i <= numNodes) claimOff[i] = 0;
 }
 // After the exclusive scan of the claim counts: every internal node enters
 // itself in its two children's claimant lists.  The cursor is the list start
@@ -228,42 +228,91 @@ __global__ void __launch_bounds__(256) k_karras(const u32* __restrict__ codes, c
     nodes[i].a = ca;
     nodes[i].b = cb;
     atomicMax(&parent[ca], i);
-    atomicAdd(&claimCount[ca], 1u);
     atomicMax(&parent[cb], i);
-    atomicAdd(&claimCount[cb], 1u);
-    if (R.range) {
+    if (!R.range) {
+        atomicAdd(&claimCount[ca], 1u);
+        atomicAdd(&claimCount[cb], 1u);
+    } else {
         // sorted-leaf range of node i (one end is leaf i); nodes whose range
         // leaves i's 256-leaf block go to the big / huge lists
         R.range[i] = make_uint2((u32)first, (u32)last);
-        const bool out = ((u32)first >> 8) != ((u32)last >> 8);
+        const bool run = !consistent && c0 == c1 && last - first >= 2;
+        const bool out = !run && ((u32)first >> 8) != ((u32)last >> 8);
         const bool huge = out && (u32)(last - first) >= BIN_RANGE_HUGE;
         const unsigned act = __activemask();
-        const unsigned mb = __ballot_sync(act, out && !huge), mh = __ballot_sync(act, huge);
+        const unsigned mb = __ballot_sync(act, out && !huge), mh = __ballot_sync(act, huge), mr = __ballot_sync(act, run);
         const u32 lane = threadIdx.x & 31u, lead = (u32)__ffs(act) - 1u;
-        u32 bb = 0, bh = 0;
+        u32 bb = 0, bh = 0, br = 0;
         if (lane == lead) {
             if (mb) bb = atomicAdd(&R.count[0], (u32)__popc(mb));
             if (mh) bh = atomicAdd(&R.count[1], (u32)__popc(mh));
+            if (mr) br = atomicAdd(&R.count[2], (u32)__popc(mr));
         }
         bb = __shfl_sync(act, bb, (int)lead);
         bh = __shfl_sync(act, bh, (int)lead);
+        br = __shfl_sync(act, br, (int)lead);
         const unsigned below = (1u << lane) - 1u;
         if (out && !huge) R.big[bb + (u32)__popc(mb & below)] = (u32)i;
         if (huge) R.huge[bh + (u32)__popc(mh & below)] = (u32)i;
+        if (run) {
+            R.runs[br + (u32)__popc(mr & below)] = (u32)i;
+            atomicMax(&R.count[3], (u32)(last - first) + 1u);
+        }
     }
 }
 
 size_t karras_scratch_bytes(u32 n) { return scan_scratch_bytes(n ? 2 * n : 1); }
 
+// Leaves (sorted position) and how a node of a run reaches them: a bounded
+// walk over its children, all of them inside its own range, so the walk is
+// over at most the run's nodes.  fn(leaf) for every visit.
+template <class Fn>
+__device__ __forceinline__ void run_walk(const Node* __restrict__ nodes, u32 n, u32 node, Fn&& fn) {
+    u32 stack[BIN_RUN_MAX];
+    int sp = 0;
+    stack[sp++] = node;
+    for (u32 step = 0; sp > 0 && step < 4096u; ++step) {
+        const u32 i = stack[--sp];
+        const i32 c[2] = {__ldcg(&nodes[i].a), __ldcg(&nodes[i].b)};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (c[k] < 0 || (u32)c[k] > 2u * n - 2u) continue;
+            if ((u32)c[k] >= n - 1u) fn((u32)c[k] - (n - 1u));
+            else if (sp < (int)BIN_RUN_MAX) stack[sp++] = (u32)c[k];
+        }
+    }
+}
+
+__global__ void k_run_reach(const Node* __restrict__ nodes, u32 n, const uint2* __restrict__ range,
+                            const u32* __restrict__ codes, const u32* __restrict__ runs, u32 nruns,
+                            u32* __restrict__ reach) {
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nruns) return;
+    const uint2 r = range[runs[t]];
+    const u32 c = codes[r.x];
+    if ((r.x > 0 && codes[r.x - 1] == c) || (r.y + 1 < n && codes[r.y + 1] == c)) return;  // not the run's top
+    if (r.y - r.x >= BIN_RUN_MAX) return;
+    unsigned long long seen = 0;
+    run_walk(nodes, n, runs[t], [&](u32 leaf) { if (leaf >= r.x && leaf <= r.y) seen |= 1ull << (leaf - r.x); });
+    for (u32 l = r.x; l <= r.y; ++l)
+        if (!((seen >> (l - r.x)) & 1ull)) atomicAnd(&reach[l >> 5], ~(1u << (l & 31u)));
+}
+
+void launch_run_reach(const Node* nodes, u32 n, const uint2* range, const u32* codes, const u32* runs, u32 nruns,
+                      u32* reach, cudaStream_t s) {
+    if (nruns) k_run_reach<<<ceil_div(nruns, 128), 128, 0, s>>>(nodes, n, range, codes, runs, nruns, reach);
+}
+
 cudaError_t launch_karras(const u32* codes, const u32* idx, u32 n, Node* nodes, i32* parent, u32* claimOff,
                           i32* claims, u32* visits, void* scratch, cudaStream_t s, bool consistent, BinRanges R) {
     if (n == 0) return cudaSuccess;
-    k_parent_init<<<ceil_div(2 * n, 256), 256, 0, s>>>(parent, claimOff, 2 * n - 1);
+    k_parent_init<<<ceil_div(2 * n, 256), 256, 0, s>>>(parent, R.range ? nullptr : claimOff, 2 * n - 1);
     if (R.range) {
-        cudaError_t e0 = cudaMemsetAsync(R.count, 0, 8, s);
+        cudaError_t e0 = cudaMemsetAsync(R.count, 0, 16, s);
         if (e0 != cudaSuccess) return e0;
     }
     k_karras<<<ceil_div(n, 256), 256, 0, s>>>(codes, idx, n, nodes, parent, claimOff, visits, consistent ? 1 : 0, R);
+    if (R.range) return cudaGetLastError();
     cudaError_t e = exclusive_scan(claimOff, 2 * n, scratch, s);
     if (e != cudaSuccess) return e;
     if (n > 1) k_claim_fill<<<ceil_div(n - 1, 256), 256, 0, s>>>(nodes, n - 1, claimOff, claims);
@@ -583,8 +632,10 @@ __device__ __forceinline__ void box_union(f3& lo, f3& hi, const Node* nd) {
 // 256-leaf boundary, 256-leaf blocks, then 16-leaf blocks and single leaves
 // again; the lanes take those pieces in turn (four loads in flight per lane)
 // and the group reduces.  Every lane of the group gets the union.
+// Leaves whose bit in reach is clear (null: none) are left out.
 template <int G, int RED = G>
-__device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 R, u32 g, f3& lo, f3& hi) {
+__device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 R, u32 g, f3& lo, f3& hi,
+                                                  const u32* reach = nullptr) {
     const float inf = __int_as_float(0x7F800000);
     const Node* leaves = J.nodes + (J.n - 1);
     const u32 b = J.leafBase;  // a multiple of 256
@@ -595,12 +646,13 @@ __device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 
     if (s256 >= e256) { s256 = e16; e256 = e16; }
     const u32 n0 = s16 - L, n1 = (s256 - s16) >> 4, n2 = (e256 - s256) >> 8, n3 = (e16 - e256) >> 4;
     const u32 total = n0 + n1 + n2 + n3 + (e - e16);
+    auto on = [&](u32 l) { return !reach || ((reach[l >> 5] >> (l & 31u)) & 1u); };
     auto piece = [&](u32 r) -> const Node* {
-        if (r < n0) return leaves + L + r;
+        if (r < n0) return on(L + r) ? leaves + L + r : nullptr;
         if ((r -= n0) < n1) return J.bb16 + ((b + s16) >> 4) + r;
         if ((r -= n1) < n2) return J.bb256 + ((b + s256) >> 8) + r;
         if ((r -= n2) < n3) return J.bb16 + ((b + e256) >> 4) + r;
-        return leaves + e16 + (r - n3);
+        return on(e16 + (r - n3)) ? leaves + e16 + (r - n3) : nullptr;
     };
     float v[6] = {inf, inf, inf, -inf, -inf, -inf};
     u32 q = g;
@@ -609,8 +661,8 @@ __device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float4* p = reinterpret_cast<const float4*>(piece(q + u * G));
-            a[u] = __ldcg(p);
-            c[u] = __ldcg(p + 1);
+            a[u] = p ? __ldcg(p) : make_float4(inf, inf, inf, 0.f);
+            c[u] = p ? __ldcg(p + 1) : make_float4(-inf, -inf, -inf, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -620,6 +672,7 @@ __device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 
     }
     for (; q < total; q += G) {
         const float4* p = reinterpret_cast<const float4*>(piece(q));
+        if (!p) continue;
         const float4 a = __ldcg(p), c = __ldcg(p + 1);
         v[0] = fminf(v[0], a.x); v[1] = fminf(v[1], a.y); v[2] = fminf(v[2], a.z);
         v[3] = fmaxf(v[3], c.x); v[4] = fmaxf(v[4], c.y); v[5] = fmaxf(v[5], c.z);
@@ -638,9 +691,10 @@ __device__ __forceinline__ void range_union_group(const RefitJob& J, u32 L, u32 
 
 // Union of the leaf boxes of sorted leaves [L, R] of job J by a whole block
 // (every thread calls this; each gets the union).
-__device__ __forceinline__ void range_union_block(const RefitJob& J, u32 L, u32 R, f3& lo, f3& hi) {
+__device__ __forceinline__ void range_union_block(const RefitJob& J, u32 L, u32 R, f3& lo, f3& hi,
+                                                  const u32* reach = nullptr) {
     __shared__ float sh_red[8][6];
-    range_union_group<256, 32>(J, L, R, threadIdx.x, lo, hi);  // pieces over the block, reduced per warp
+    range_union_group<256, 32>(J, L, R, threadIdx.x, lo, hi, reach);  // pieces over the block, reduced per warp
     // then across the warps
     if ((threadIdx.x & 31u) == 0) {
         sh_red[threadIdx.x >> 5][0] = lo.x; sh_red[threadIdx.x >> 5][1] = lo.y; sh_red[threadIdx.x >> 5][2] = lo.z;
@@ -779,11 +833,12 @@ __device__ __forceinline__ void face_box(const RefitJob& J, u32 f, f3& lo, f3& h
 // 32-byte sector).  In sorted-leaf order these reads were random gathers,
 // several sectors per leaf.
 __global__ void __launch_bounds__(256) k_refit_bin_faces(RefitJob J, const u32* __restrict__ rank,
-                                                         float4* __restrict__ lbox) {
+                                                         float4* __restrict__ lbox, u32* __restrict__ nan) {
     const u32 f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= J.n) return;
     f3 lo, hi;
     face_box(J, f, lo, hi);
+    if (nan && (lo.x != lo.x || lo.y != lo.y || lo.z != lo.z || hi.x != hi.x || hi.y != hi.y || hi.z != hi.z)) *nan = 1u;
     const u32 r = rank[f];
     __stcg(lbox + 2 * (size_t)r, make_float4(lo.x, lo.y, lo.z, __int_as_float(-1)));  // the leaf node's a
     __stcg(lbox + 2 * (size_t)r + 1, make_float4(hi.x, hi.y, hi.z, __uint_as_float(f)));  // and b (its face)
@@ -793,9 +848,12 @@ __global__ void __launch_bounds__(256) k_refit_bin_faces(RefitJob J, const u32* 
 // its box (from lbox when the face pass ran, else gathered here) goes to the
 // leaf node, the block's 16- and 256-leaf boxes to bb16 / bb256, and
 // internal node i (whose range has leaf i at one end) gets its box here when
-// its range stays in the block.
+// its range stays in the block.  Leaves whose bit in reach is clear take no
+// part in the unions (midpoint split; nodes inside runs are written by
+// k_refit_bin_runs afterwards).
 __global__ void __launch_bounds__(256) k_refit_bin_leaves(RefitJob J, const uint2* __restrict__ range,
-                                                          const float4* __restrict__ lbox) {
+                                                          const float4* __restrict__ lbox,
+                                                          const u32* __restrict__ reach) {
     __shared__ float sh_leaf[6][256];
     __shared__ float sh_g16[6][16];
     __shared__ float sh_box[8][6];
@@ -821,8 +879,9 @@ __global__ void __launch_bounds__(256) k_refit_bin_leaves(RefitJob J, const uint
         if (has) store_box(&nodes[n - 1 + i], lo, hi);
     }
     const float inf = __int_as_float(0x7F800000);
-    float v[6] = {has ? lo.x : inf, has ? lo.y : inf, has ? lo.z : inf,
-                  has ? hi.x : -inf, has ? hi.y : -inf, has ? hi.z : -inf};
+    const bool on = has && (!reach || ((reach[i >> 5] >> (i & 31u)) & 1u));
+    float v[6] = {on ? lo.x : inf, on ? lo.y : inf, on ? lo.z : inf,
+                  on ? hi.x : -inf, on ? hi.y : -inf, on ? hi.z : -inf};
 #pragma unroll
     for (int k = 0; k < 6; ++k) sh_leaf[k][threadIdx.x] = v[k];
     const u32 lane = threadIdx.x & 31u;
@@ -878,7 +937,8 @@ __global__ void __launch_bounds__(256) k_refit_bin_leaves(RefitJob J, const uint
 // per node of huge (ranges of BIN_RANGE_HUGE leaves or more).
 __global__ void __launch_bounds__(256) k_refit_bin_ranges(RefitJob J, const uint2* __restrict__ range,
                                                           const u32* __restrict__ big, u32 nbig,
-                                                          const u32* __restrict__ huge, u32 nhuge) {
+                                                          const u32* __restrict__ huge, u32 nhuge,
+                                                          const u32* __restrict__ reach) {
     const u32 medBlocks = (nbig + 31) / 32;
     if (blockIdx.x < medBlocks) {
         const u32 grp = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -889,7 +949,7 @@ __global__ void __launch_bounds__(256) k_refit_bin_ranges(RefitJob J, const uint
             r = range[node];
         }
         f3 lo, hi;
-        range_union_group<8>(J, r.x, r.y, threadIdx.x & 7u, lo, hi);
+        range_union_group<8>(J, r.x, r.y, threadIdx.x & 7u, lo, hi, reach);
         if ((threadIdx.x & 7u) == 0 && r.x <= r.y) store_box(&J.nodes[node], lo, hi);
         return;
     }
@@ -899,8 +959,19 @@ __global__ void __launch_bounds__(256) k_refit_bin_ranges(RefitJob J, const uint
     const uint2 r = range[node];
     if (r.x > r.y || r.y >= J.n) return;  // uniform over the block
     f3 lo, hi;
-    range_union_block(J, r.x, r.y, lo, hi);
+    range_union_block(J, r.x, r.y, lo, hi, reach);
     if (threadIdx.x == 0) store_box(&J.nodes[node], lo, hi);
+}
+
+// Nodes inside runs of equal codes: the union of the leaves each reaches
+// through its children.  One thread per node; runs are a few leaves long.
+__global__ void __launch_bounds__(128) k_refit_bin_runs(RefitJob J, const u32* __restrict__ runs, u32 nruns) {
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nruns) return;
+    const float inf = __int_as_float(0x7F800000);
+    f3 lo = mk(inf, inf, inf), hi = mk(-inf, -inf, -inf);
+    run_walk(J.nodes, J.n, runs[t], [&](u32 leaf) { box_union(lo, hi, J.nodes + (J.n - 1) + leaf); });
+    store_box(&J.nodes[runs[t]], lo, hi);
 }
 
 __global__ void k_leaf_vids(const u32* __restrict__ idx, const u32* __restrict__ facets, u32 n,
@@ -926,12 +997,15 @@ void launch_leaf_rank(const u32* idx, u32 n, u32* rank, cudaStream_t s) {
 }
 
 void launch_refit_bin(const RefitJob& J, const uint2* range, const u32* big, u32 nbig, const u32* huge, u32 nhuge,
-                      const u32* rank, float4* lbox, cudaStream_t s) {
+                      const u32* rank, float4* lbox, cudaStream_t s, const u32* runs, u32 nruns, const u32* reach,
+                      u32* nan) {
     if (J.n == 0) return;
-    if (rank && lbox) k_refit_bin_faces<<<ceil_div(J.n, 256), 256, 0, s>>>(J, rank, lbox);
-    k_refit_bin_leaves<<<ceil_div(J.n, 256), 256, 0, s>>>(J, range, rank && lbox ? lbox : nullptr);
+    if (!nruns) reach = nullptr;
+    if (rank && lbox) k_refit_bin_faces<<<ceil_div(J.n, 256), 256, 0, s>>>(J, rank, lbox, nan);
+    k_refit_bin_leaves<<<ceil_div(J.n, 256), 256, 0, s>>>(J, range, rank && lbox ? lbox : nullptr, reach);
     const u32 blocks = (nbig + 31) / 32 + nhuge;
-    if (blocks) k_refit_bin_ranges<<<blocks, 256, 0, s>>>(J, range, big, nbig, huge, nhuge);
+    if (blocks) k_refit_bin_ranges<<<blocks, 256, 0, s>>>(J, range, big, nbig, huge, nhuge, reach);
+    if (nruns) k_refit_bin_runs<<<ceil_div(nruns, 128), 128, 0, s>>>(J, runs, nruns);
 }
 
 void launch_refit_ranges(const RefitJob* jobsDev, u32 numJobs, const uint4* big, u32 bigCap, u32 nmed, u32 nhuge,
@@ -1688,6 +1762,15 @@ __global__ void k_claim_count(const Node* __restrict__ nodes, u32 nInner, u32* _
     const i32 a = nodes[i].a, b = nodes[i].b, nn = 2 * (i32)nInner + 1;
     if (a >= 0 && a < nn) atomicAdd(&claimCount[a], 1u);
     if (b >= 0 && b < nn) atomicAdd(&claimCount[b], 1u);
+}
+
+cudaError_t launch_claims(const Node* nodes, u32 n, u32* claimOff, i32* claims, void* scratch, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(claimOff, 0, 8 * (size_t)n, s);
+    if (e != cudaSuccess || n <= 1) return e;
+    k_claim_count<<<ceil_div(n - 1, 256), 256, 0, s>>>(nodes, n - 1, claimOff);
+    if ((e = exclusive_scan(claimOff, 2 * n, scratch, s)) != cudaSuccess) return e;
+    k_claim_fill<<<ceil_div(n - 1, 256), 256, 0, s>>>(nodes, n - 1, claimOff, claims);
+    return cudaGetLastError();
 }
 
 size_t apetrei_scratch_bytes(u32 n) { return 8 * (size_t)(n ? n : 1) + 256; }

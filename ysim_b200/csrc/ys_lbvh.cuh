@@ -124,29 +124,49 @@ void launch_morton(const float4* x4, const float* x3, u32 voff, const u32* facet
 // determineRange already orders them by, so every node has one parent (the
 // cube layout); false keeps the reference's midpoint split.
 size_t karras_scratch_bytes(u32 n);
-// Optional outputs of a Karras build for the range refit of a consistent
-// tree: per internal node its sorted-leaf range, and the nodes whose range
-// leaves the 256-leaf block of their own index, in big (ranges under
-// BIN_RANGE_HUGE leaves, count[0]) or huge (count[1]); both lists need n
-// entries.  range = null: none.
+// Optional outputs of a Karras build for the range refit: per internal node
+// its sorted-leaf range, and the nodes whose range leaves the 256-leaf block of
+// their own index, in big (ranges under BIN_RANGE_HUGE leaves, count[0]) or
+// huge (count[1]); both lists need n entries.  range = null: none, and the
+// claimant lists are built instead (with ranges they are not: nothing climbs).
+//
+// With the midpoint split, a node over one run of three or more equal codes
+// reaches only some leaves of its range, some of them twice.  Every other
+// node splits as in the consistent tree, so its box is the union of its range
+// over the leaves that the topmost node of each run reaches.  runs gets the nodes
+// inside such runs (n entries, count[2]); their boxes are followed through
+// their children.  count[3] is the longest run; count has 4 words.
+// launch_run_reach then clears the bits of the other leaves in reach (all
+// ones before, n bits; null: no run).
 static constexpr u32 BIN_RANGE_HUGE = 16384;
+// Runs up to this length are followed node by node; with a longer one the
+// tree is climbed (a node's thread visits its part of the run).
+static constexpr u32 BIN_RUN_MAX = 64;
 struct BinRanges {
     uint2* range = nullptr;
     u32* big = nullptr;
     u32* huge = nullptr;
+    u32* runs = nullptr;
     u32* count = nullptr;
 };
+void launch_run_reach(const Node* nodes, u32 n, const uint2* range, const u32* codes, const u32* runs, u32 nruns,
+                      u32* reach, cudaStream_t s);
+// Claimant lists of a built tree (for the climb).
+cudaError_t launch_claims(const Node* nodes, u32 n, u32* claimOff, i32* claims, void* scratch, cudaStream_t s);
 cudaError_t launch_karras(const u32* codes, const u32* idx, u32 n, Node* nodes, i32* parent, u32* claimOff,
                           i32* claims, u32* visits, void* scratch, cudaStream_t s, bool consistent = false,
                           BinRanges R = BinRanges());
-// Range refit of a consistent binary tree built with BinRanges (J: nodes,
+// Range refit of a binary tree built with BinRanges (J: nodes,
 // facets, positions (and velocities when swept), n; bb16 / bb256 with
 // n / 16 + 1 and n / 256 + 1 boxes): leaf pass, then the big and huge nodes.
 // With rank (each face's sorted-leaf position) and lbox (2 float4 per leaf) a
 // face-order pass computes the leaf boxes first, so the leaf pass reads them
-// in order instead of gathering facets and vertices.
+// in order instead of gathering facets and vertices; *nan becomes nonzero when
+// a leaf box has a NaN (the unions leave NaN out, a climb's tinym::min keeps
+// it or not by operand order).
 void launch_refit_bin(const RefitJob& J, const uint2* range, const u32* big, u32 nbig, const u32* huge, u32 nhuge,
-                      const u32* rank, float4* lbox, cudaStream_t s);
+                      const u32* rank, float4* lbox, cudaStream_t s, const u32* runs = nullptr, u32 nruns = 0,
+                      const u32* reach = nullptr, u32* nan = nullptr);
 // lvid[i] = (facet of idx[i], idx[i]) for the sorted faces of a build.
 void launch_leaf_vids(const u32* idx, const u32* facets, u32 n, uint4* lvid, cudaStream_t s);
 // rank[idx[i]] = i for the sorted face indices of a build.
