@@ -654,8 +654,8 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
                           __shfl_sync(FULL_MASK, xc.z, owner));
         const f3 oxp = mk(__shfl_sync(FULL_MASK, xpv.x, owner), __shfl_sync(FULL_MASK, xpv.y, owner),
                           __shfl_sync(FULL_MASK, xpv.z, owner));
-        const u32 og = __shfl_sync(FULL_MASK, g, owner);
-        const float oinv = __shfl_sync(FULL_MASK, inv, owner);
+        const u32 og = GROUPS ? 0u : __shfl_sync(FULL_MASK, g, owner);
+        const float oinv = GROUPS ? 0.f : __shfl_sync(FULL_MASK, inv, owner);
         bool hit = false;
         VContact c;
         if (has) {
@@ -778,60 +778,81 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
                 Q.vhi[lane] = make_float4(bhi.x, bhi.y, bhi.z, 0.f);
                 __syncwarp();
                 const LaneBox LB = lane_box(blo, bhi);
-                f3 ulo, uhi;
-                for (u32 c3 = 0; c3 < n3; ++c3) {
-                    // a run of 32768 leaves: the vertices that meet it
+                f3 alo, ahi;  // the union of all, of those that meet a run of 32768, of 1024
+                lane_union(LB, in, alo, ahi);
+                const unsigned inm = __ballot_sync(FULL_MASK, in);
+                for (u32 q3 = 0; q3 < n3; q3 += 32u) {
                     float tl[3], th[3];
-                    group_acc_box(A.grp.top + 8 * (size_t)(top + c3), tl, th);
-                    const bool in3 = in && meets(blo, bhi, make_float4(tl[0], tl[1], tl[2], 0.f),
-                                                 make_float4(th[0], th[1], th[2], 0.f));
-                    if (!__ballot_sync(FULL_MASK, in3)) continue;
-                    lane_union(LB, in3, ulo, uhi);
-                    const u32 k2 = c3 * 32u + lane;
-                    unsigned m2 = __ballot_sync(FULL_MASK, k2 < n2 && meets(ulo, uhi, __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u)),
-                                                                            __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u) + 1)));
-                    while (m2) {
-                        // a run of 1024
-                        const u32 c2 = c3 * 32u + (u32)__ffs(m2) - 1u;
-                        m2 &= m2 - 1u;
-                        const bool in2 = in3 && meets(blo, bhi, __ldg(L2 + 2 * (size_t)c2), __ldg(L2 + 2 * (size_t)c2 + 1));
-                        if (!__ballot_sync(FULL_MASK, in2)) continue;
-                        lane_union(LB, in2, ulo, uhi);
-                        const u32 k1c = c2 * 32u + lane;
-                        unsigned m1 = __ballot_sync(FULL_MASK, k1c < n1 && meets(ulo, uhi, __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u)),
-                                                                                 __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u) + 1)));
-                        while (m1) {
-                            // a run of 32 leaves: the vertices that meet it, each against the leaves
-                            const u32 c1 = c2 * 32u + (u32)__ffs(m1) - 1u;
-                            m1 &= m1 - 1u;
-                            unsigned vm = __ballot_sync(
-                                FULL_MASK, in2 && meets(blo, bhi, __ldg(L1 + 2 * (size_t)c1), __ldg(L1 + 2 * (size_t)c1 + 1)));
-                            if (!vm) continue;
-                            const u32 i = c1 * 32u + lane;
-                            const bool live = i < n;
-                            const u32 li = live ? i : n - 1u;
-                            const float4 lo = __ldg(L0 + 2 * (size_t)li), hi = __ldg(L0 + 2 * (size_t)li + 1);
-                            uint4 id = make_uint4(NO_VERTEX, NO_VERTEX, NO_VERTEX, 0u);
-                            if (own) id = __ldg(vids + li);
-                            do {
-                                const u32 v = (u32)__ffs(vm) - 1u;
-                                vm &= vm - 1u;
-                                const float4 a = Q.vlo[v], b = Q.vhi[v];
-                                const u32 lid = __float_as_uint(a.w);
-                                const bool hit = live & meets(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), lo, hi) &
-                                                 (id.x != lid) & (id.y != lid) & (id.z != lid);
-                                const unsigned hm = __ballot_sync(FULL_MASK, hit);
-                                if (hit) {
-                                    const u32 slot = qn + (u32)__popc(hm & ((1u << lane) - 1u));
-                                    Q.qf[slot] = rec + i;
-                                    Q.qk[slot] = key | v;
+                    group_acc_box(A.grp.top + 8 * (size_t)(top + min(q3 + lane, n3 - 1u)), tl, th);
+                    unsigned m3 = __ballot_sync(FULL_MASK, q3 + lane < n3 && meets(alo, ahi, make_float4(tl[0], tl[1], tl[2], 0.f),
+                                                                                   make_float4(th[0], th[1], th[2], 0.f)));
+                    while (m3) {
+                        // a run of 32768 leaves: the vertices that meet it
+                        const u32 s3 = (u32)__ffs(m3) - 1u, c3 = q3 + s3;
+                        m3 &= m3 - 1u;
+                        const float4 b0 = make_float4(__shfl_sync(FULL_MASK, tl[0], (int)s3), __shfl_sync(FULL_MASK, tl[1], (int)s3),
+                                                      __shfl_sync(FULL_MASK, tl[2], (int)s3), 0.f);
+                        const float4 b1 = make_float4(__shfl_sync(FULL_MASK, th[0], (int)s3), __shfl_sync(FULL_MASK, th[1], (int)s3),
+                                                      __shfl_sync(FULL_MASK, th[2], (int)s3), 0.f);
+                        const bool in3 = in && meets(blo, bhi, b0, b1);
+                        const unsigned in3m = __ballot_sync(FULL_MASK, in3);
+                        if (!in3m) continue;
+                        f3 ulo = alo, uhi = ahi;
+                        if (in3m != inm) lane_union(LB, in3, ulo, uhi);
+                        const u32 k2 = c3 * 32u + lane;
+                        unsigned m2 = __ballot_sync(FULL_MASK, k2 < n2 && meets(ulo, uhi, __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u)),
+                                                                                __ldg(L2 + 2 * (size_t)min(k2, n2 - 1u) + 1)));
+                        while (m2) {
+                            // a run of 1024
+                            const u32 c2 = c3 * 32u + (u32)__ffs(m2) - 1u;
+                            m2 &= m2 - 1u;
+                            const bool in2 = in3 && meets(blo, bhi, __ldg(L2 + 2 * (size_t)c2), __ldg(L2 + 2 * (size_t)c2 + 1));
+                            const unsigned in2m = __ballot_sync(FULL_MASK, in2);
+                            if (!in2m) continue;
+                            f3 wlo = ulo, whi = uhi;
+                            if (in2m != in3m) lane_union(LB, in2, wlo, whi);
+                            const u32 k1c = c2 * 32u + lane;
+                            unsigned m1 = __ballot_sync(FULL_MASK, k1c < n1 && meets(wlo, whi, __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u)),
+                                                                                     __ldg(L1 + 2 * (size_t)min(k1c, n1 - 1u) + 1)));
+                            while (m1) {
+                                // a run of 32 leaves: the vertices that meet it, each against the leaves
+                                const u32 c1 = c2 * 32u + (u32)__ffs(m1) - 1u;
+                                m1 &= m1 - 1u;
+                                unsigned vm = __ballot_sync(
+                                    FULL_MASK, in2 && meets(blo, bhi, __ldg(L1 + 2 * (size_t)c1), __ldg(L1 + 2 * (size_t)c1 + 1)));
+                                if (!vm) continue;
+                                const u32 i = c1 * 32u + lane;
+                                const bool live = i < n;
+                                const u32 li = live ? i : n - 1u;
+                                const float4 lo = __ldg(L0 + 2 * (size_t)li), hi = __ldg(L0 + 2 * (size_t)li + 1);
+                                uint4 id = make_uint4(NO_VERTEX, NO_VERTEX, NO_VERTEX, 0u);
+                                if (own) id = __ldg(vids + li);
+                                u32 hits = 0;  // vertices whose box meets this lane's leaf
+                                do {
+                                    const u32 v = (u32)__ffs(vm) - 1u;
+                                    vm &= vm - 1u;
+                                    const float4 a = Q.vlo[v], b = Q.vhi[v];
+                                    const u32 lid = __float_as_uint(a.w);
+                                    const bool hit = meets(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), lo, hi) &
+                                                     (id.x != lid) & (id.y != lid) & (id.z != lid);
+                                    hits |= hit ? 1u << v : 0u;
+                                } while (vm);
+                                if (!live) hits = 0;
+                                // into the queue, one per lane at a time
+                                for (unsigned hm; (hm = __ballot_sync(FULL_MASK, hits != 0)) != 0;) {
+                                    if (hits) {
+                                        const u32 slot = qn + (u32)__popc(hm & ((1u << lane) - 1u));
+                                        Q.qf[slot] = rec + i;
+                                        Q.qk[slot] = key | ((u32)__ffs(hits) - 1u);
+                                        hits &= hits - 1u;
+                                    }
+                                    qn += (u32)__popc(hm);
+                                    if (qn >= 32u) {
+                                        qn -= 32u;
+                                        drain(qn, 32);
+                                    }
                                 }
-                                qn += (u32)__popc(hm);
-                                if (qn >= 32u) {
-                                    qn -= 32u;
-                                    drain(qn, 32);
-                                }
-                            } while (vm);
+                            }
                         }
                     }
                 }
