@@ -20,11 +20,11 @@
 // each obstacle by its root box; the point query box x +- margin selects
 // every face whose exact AABB it overlaps (queryPoints, bvh.metal:1322-1412),
 // and narrow_pt_tri (bruteforce.metal:41-178) runs in double on each.  The
-// candidates come from the scene's float tree of the obstacle, queried with
-// the double box rounded outward to float: a float box that contains the
+// candidates come from the obstacle's sorted-leaf groups (float boxes), queried
+// with the double box rounded outward to float: a float box that contains the
 // double one overlaps every leaf whose face AABB the double box overlaps, so
 // the exact double test then sees the same faces as a search over all faces.
-// The contacts of a vertex are kept sorted by face, so the order of the tree
+// The contacts of a vertex are kept sorted by face, so the order of the
 // descent does not reach the result.
 //
 // Every operation is a single IEEE binary64 add, multiply, divide or square
@@ -58,11 +58,6 @@ __device__ __forceinline__ dd3 ldf(const float4* p, u32 i) {
 struct __align__(32) DContact { double nx, ny, nz, d; };
 
 static constexpr u32 D64_CAP = 16;    // contacts kept per vertex and step
-static constexpr int D64_SPLIT = 4;   // the contact search splits a vertex's descent at this depth
-static constexpr u32 D64_LANES = 1u << D64_SPLIT;  // into this many threads, one per subtree
-static constexpr u32 D64_LCAP = 8;    // contacts one of those threads may find
-static constexpr int D64_STACK = 64;  // tree descent stack
-static constexpr u32 D64_VISIT_CAP = 1u << 20;
 // Block size of the per-vertex kernels (32 measured the same on the
 // 128x128 rollout: the step kernel is bound by its divergent descents).
 static constexpr u32 D64_BLOCK = 128;
@@ -83,7 +78,8 @@ struct A64 {
     // static), faces, trees, meshes, the cloth's target list
     const float4* sx;
     const uint4* F;
-    const Node* nodes;
+    GroupBufs grp;
+    const uint4* lvid;
     const MeshDev* meshes;
     const u32* targets;
     const float4* ext;  // external forces or null (then g m)
@@ -102,12 +98,13 @@ struct A64 {
     DContact* cs;  // D64_CAP slots per vertex, sorted by (object, face)
     u32* cf;       // their face ids
     u32* cn;       // contacts per vertex
-    // the contact search's output, per (vertex, subtree): D64_LCAP contacts
-    // in search order, their face ids and target ordinals, the count
+    // the contact search's output, per vertex: up to D64_CAP contacts in
+    // search order, their face ids and target ordinals, the count
     DContact* ls;
     u32* lf;
     u32* lk;
     u32* ln;
+    u32 vpw;  // vertices per warp of the contact search
     unsigned long long* box;  // cloth swept box: ~dord(min) x3 then dord(max) x3, all by atomicMax
     u32* status;
 };
@@ -198,98 +195,126 @@ __global__ void __launch_bounds__(256) k_d64_box(A64 A) {
     }
 }
 
-// Contact search of one step, D64_LANES threads per vertex: thread j of a
-// vertex descends the subtree reached from the root by the bits of j (high
-// bit first) over D64_SPLIT levels; a leaf met above that depth belongs to
-// the thread whose remaining bits are zero.  Together the threads visit
-// every root-to-leaf path the one-thread descent visits, with D64_LANES
-// times the threads in flight (a 128x128 cloth is otherwise 512 warps, and
-// the descents' dependent loads are the step's time).
+// Contact search of one step: a warp descends each obstacle's groups once for
+// its vpw vertices, as the fused substep does (one lane per child, then one
+// per leaf), and tests the candidates 32 at a time in double.  (Sixteen
+// one-thread subtree descents per vertex: 41 us on the 65 x 65 cloth.)
+struct D64Work {
+    u32 qf[64], qk[64];       // candidates: sorted leaf, target ordinal << 5 | owner lane
+    float4 vlo[32], vhi[32];  // the vertices' query boxes, rounded outward
+    u32 n[32];                // contacts found per vertex
+};
 __global__ void __launch_bounds__(D64_BLOCK) k_d64_cand(A64 A) {
-    const u32 tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= A.nV * D64_LANES) return;
-    const u32 i = tid / D64_LANES, j = tid % D64_LANES;
-    const dd3 p = ldd(A.x, i), pp = ldd(A.xp, i);
-    DContact* ls = A.ls + (size_t)tid * D64_LCAP;
-    u32* lf = A.lf + (size_t)tid * D64_LCAP;
-    u32* lk = A.lk + (size_t)tid * D64_LCAP;
-    u32 n = 0, st = 0;
-    const dd3 blo = dm(dunord(~A.box[0]), dunord(~A.box[1]), dunord(~A.box[2]));
-    const dd3 bhi = dm(dunord(A.box[3]), dunord(A.box[4]), dunord(A.box[5]));
-    const dd3 qmn = p - dm(A.margin, A.margin, A.margin), qmx = p + dm(A.margin, A.margin, A.margin);
-    const float4 flo = make_float4(__double2float_rd(qmn.x), __double2float_rd(qmn.y), __double2float_rd(qmn.z), 0.f);
-    const float4 fhi = make_float4(__double2float_ru(qmx.x), __double2float_ru(qmx.y), __double2float_ru(qmx.z), 0.f);
+    __shared__ D64Work work[D64_BLOCK / 32];
+    D64Work& Q = work[threadIdx.x >> 5];
+    const u32 lane = threadIdx.x & 31u;
+    const u32 first = (blockIdx.x * (D64_BLOCK / 32) + (threadIdx.x >> 5)) * A.vpw;
+    const bool in = lane < A.vpw && first + lane < A.nV;
+    const u32 i = in ? first + lane : 0u;
+    const dd3 p = ldd(A.x, i);
+    u32 st = 0, qn = 0;
+    const f3 blo = mk(__double2float_rd(p.x - A.margin), __double2float_rd(p.y - A.margin), __double2float_rd(p.z - A.margin));
+    const f3 bhi = mk(__double2float_ru(p.x + A.margin), __double2float_ru(p.y + A.margin), __double2float_ru(p.z + A.margin));
+    Q.vlo[lane] = make_float4(blo.x, blo.y, blo.z, 0.f);
+    Q.vhi[lane] = make_float4(bhi.x, bhi.y, bhi.z, 0.f);
+    Q.n[lane] = 0;
+    __syncwarp();
+    const LaneBox LB = lane_box(blo, bhi);
+    f3 alo, ahi;
+    lane_union(LB, in, alo, ahi);
+    const dd3 slo = dm(dunord(~A.box[0]), dunord(~A.box[1]), dunord(~A.box[2]));
+    const dd3 shi = dm(dunord(A.box[3]), dunord(A.box[4]), dunord(A.box[5]));
+    auto drain = [&](u32 base, u32 cnt) {
+        __syncwarp();
+        if (lane < cnt) {
+            const u32 key = Q.qk[base + lane], v = key & 31u, k = key >> 5;
+            const MeshDev& T = A.meshes[A.targets[A.tgt_begin + k]];
+            const u32 f = A.lvid[T.foff + Q.qf[base + lane]].w;
+            const uint4 tri = A.F[T.foff + f];
+            const dd3 t0 = ldf(A.sx, T.voff + tri.x), t1 = ldf(A.sx, T.voff + tri.y), t2 = ldf(A.sx, T.voff + tri.z);
+            const dd3 x = ldd(A.x, first + v);
+            const dd3 qmn = x - dm(A.margin, A.margin, A.margin), qmx = x + dm(A.margin, A.margin, A.margin);
+            const double mnx = fmin(t0.x, fmin(t1.x, t2.x)), mxx = fmax(t0.x, fmax(t1.x, t2.x));
+            const double mny = fmin(t0.y, fmin(t1.y, t2.y)), mxy = fmax(t0.y, fmax(t1.y, t2.y));
+            const double mnz = fmin(t0.z, fmin(t1.z, t2.z)), mxz = fmax(t0.z, fmax(t1.z, t2.z));
+            dd3 cn;
+            double cd;
+            if (!(qmx.x < mnx || qmn.x > mxx || qmx.y < mny || qmn.y > mxy || qmx.z < mnz || qmn.z > mxz) &&
+                narrow64(x, ldd(A.xp, first + v), t0, t1, t2, A.radius, A.margin, cn, cd)) {
+                const u32 slot = atomicAdd(&Q.n[v], 1u);
+                const size_t o = (size_t)(first + v) * D64_CAP + slot;
+                if (slot >= D64_CAP) st |= YS_FLAG_CONTACT_OVF;
+                else {
+                    A.ls[o] = DContact{cn.x, cn.y, cn.z, cd};
+                    A.lf[o] = f;
+                    A.lk[o] = k;
+                }
+            }
+        }
+        __syncwarp();
+    };
     for (u32 k = A.tgt_begin; k < A.tgt_end; ++k) {
         const u32 t = A.targets[k];
         const MeshDev& T = A.meshes[t];
         if (t == A.cloth || T.nF == 0 || (T.flags & MF_ANALYTIC)) continue;
-        const Node* nodes = A.nodes + T.node_off;
-        const Node root = nodes[0];
-        if (bhi.x < (double)root.mnx || blo.x > (double)root.mxx || bhi.y < (double)root.mny ||
-            blo.y > (double)root.mxy || bhi.z < (double)root.mnz || blo.z > (double)root.mxz)
+        float rl[3], rh[3];
+        group_acc_box(A.grp.root + 8 * (size_t)T.root, rl, rh);
+        if (shi.x < (double)rl[0] || slo.x > (double)rh[0] || shi.y < (double)rl[1] || slo.y > (double)rh[1] ||
+            shi.z < (double)rl[2] || slo.z > (double)rh[2])
             continue;
-        const u32 nn = 2 * T.nF - 1;
-        // this thread's subtree
-        int id = 0;
-        bool mine = true;
-        for (int L = 0; L < D64_SPLIT; ++L) {
-            const Node q = nodes[id];
-            if (fhi.x < q.mnx || flo.x > q.mxx || fhi.y < q.mny || flo.y > q.mxy || fhi.z < q.mnz || flo.z > q.mxz) {
-                mine = false;
-                break;
+        const u32 n = T.nF, n1 = (n + 31u) / 32u, n2 = (n + 1023u) / 1024u;
+        const float4* __restrict__ L0 = A.grp.l0 + 2 * (size_t)T.boxL0;
+        const float4* __restrict__ L1 = A.grp.l1 + 2 * (size_t)(T.boxL0 / 32u);
+        const float4* __restrict__ L2 = A.grp.l2 + 2 * (size_t)(T.boxL0 / 1024u);
+        for (u32 q2 = 0; q2 < n2; q2 += 32u) {
+            // the children of a run of 32768 at once
+            const u32 k2 = min(q2 + lane, n2 - 1u);
+            unsigned m2 = __ballot_sync(FULL_MASK, q2 + lane < n2 && meets(alo, ahi, __ldg(L2 + 2 * (size_t)k2), __ldg(L2 + 2 * (size_t)k2 + 1)));
+            while (m2) {
+                const u32 c2 = q2 + (u32)__ffs(m2) - 1u;
+                m2 &= m2 - 1u;
+                const bool in2 = in && meets(blo, bhi, __ldg(L2 + 2 * (size_t)c2), __ldg(L2 + 2 * (size_t)c2 + 1));
+                if (!__ballot_sync(FULL_MASK, in2)) continue;
+                f3 ulo, uhi;
+                lane_union(LB, in2, ulo, uhi);
+                const u32 k1 = min(c2 * 32u + lane, n1 - 1u);
+                unsigned m1 = __ballot_sync(FULL_MASK, c2 * 32u + lane < n1 && meets(ulo, uhi, __ldg(L1 + 2 * (size_t)k1), __ldg(L1 + 2 * (size_t)k1 + 1)));
+                while (m1) {
+                    const u32 c1 = c2 * 32u + (u32)__ffs(m1) - 1u;
+                    m1 &= m1 - 1u;
+                    unsigned vm = __ballot_sync(FULL_MASK, in2 && meets(blo, bhi, __ldg(L1 + 2 * (size_t)c1), __ldg(L1 + 2 * (size_t)c1 + 1)));
+                    if (!vm) continue;
+                    const u32 leaf = c1 * 32u + lane, li = min(leaf, n - 1u);
+                    const float4 lo = __ldg(L0 + 2 * (size_t)li), hi = __ldg(L0 + 2 * (size_t)li + 1);
+                    do {
+                        const u32 v = (u32)__ffs(vm) - 1u;
+                        vm &= vm - 1u;
+                        const float4 a = Q.vlo[v], b = Q.vhi[v];
+                        const bool hit = leaf < n && meets(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), lo, hi);
+                        const unsigned hm = __ballot_sync(FULL_MASK, hit);
+                        if (hit) {
+                            const u32 slot = qn + (u32)__popc(hm & ((1u << lane) - 1u));
+                            Q.qf[slot] = leaf;
+                            Q.qk[slot] = ((k - A.tgt_begin) << 5) | v;
+                        }
+                        qn += (u32)__popc(hm);
+                        if (qn >= 32u) {
+                            qn -= 32u;
+                            drain(qn, 32);
+                        }
+                    } while (vm);
+                }
             }
-            if (q.a < 0) {  // a leaf above the split depth
-                mine = (j & ((1u << (D64_SPLIT - L)) - 1u)) == 0u;
-                break;
-            }
-            id = ((j >> (D64_SPLIT - 1 - L)) & 1u) ? q.b : q.a;
-            if (id < 0 || (u32)id >= nn) { mine = false; break; }
-        }
-        if (!mine) continue;
-        int stack[D64_STACK];
-        int sp = 1;
-        stack[0] = id;
-        u32 visited = 0;
-        while (sp > 0) {
-            if (++visited > D64_VISIT_CAP) { st |= YS_FLAG_STACK_OVF; break; }
-            const int nid = stack[--sp];
-            if (nid < 0 || (u32)nid >= nn) continue;
-            const Node q = nodes[nid];
-            if (fhi.x < q.mnx || flo.x > q.mxx || fhi.y < q.mny || flo.y > q.mxy || fhi.z < q.mnz || flo.z > q.mxz)
-                continue;
-            if (q.a >= 0) {
-                if (sp + 2 > D64_STACK) { st |= YS_FLAG_STACK_OVF; continue; }
-                stack[sp++] = q.a;
-                stack[sp++] = q.b;
-                continue;
-            }
-            const u32 f = (u32)q.b;
-            if (f >= T.nF) continue;
-            const uint4 tri = A.F[T.foff + f];
-            const dd3 t0 = ldf(A.sx, T.voff + tri.x), t1 = ldf(A.sx, T.voff + tri.y), t2 = ldf(A.sx, T.voff + tri.z);
-            const double mnx = fmin(t0.x, fmin(t1.x, t2.x)), mxx = fmax(t0.x, fmax(t1.x, t2.x));
-            const double mny = fmin(t0.y, fmin(t1.y, t2.y)), mxy = fmax(t0.y, fmax(t1.y, t2.y));
-            const double mnz = fmin(t0.z, fmin(t1.z, t2.z)), mxz = fmax(t0.z, fmax(t1.z, t2.z));
-            if (qmx.x < mnx || qmn.x > mxx || qmx.y < mny || qmn.y > mxy || qmx.z < mnz || qmn.z > mxz) continue;
-            dd3 cn;
-            double cd;
-            if (!narrow64(p, pp, t0, t1, t2, A.radius, A.margin, cn, cd)) continue;
-            if (n >= D64_LCAP) { st |= YS_FLAG_CONTACT_OVF; continue; }
-            ls[n] = DContact{cn.x, cn.y, cn.z, cd};
-            lf[n] = f;
-            lk[n] = k - A.tgt_begin;
-            ++n;
         }
     }
-    A.ln[tid] = n;
+    if (qn) drain(0, qn);
+    if (in) A.ln[i] = Q.n[lane];
     if (st) atomicOr(A.status, st);
 }
 
-// One step of the FP64 rollout for each vertex: its contacts from the
-// search threads merged into one list sorted by (object, face) (a face
-// reported twice -- the reference tree layout over runs of equal codes -- is
-// one candidate, as in a search over all faces; recorded in cs / cf / cn),
-// then forces, integration and the contact response.
+// One step of the FP64 rollout for each vertex: its contacts sorted by
+// (object, face) (recorded in cs / cf / cn), then forces, integration and the
+// contact response.
 __global__ void __launch_bounds__(D64_BLOCK) k_d64_step(A64 A) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.nV) return;
@@ -299,27 +324,20 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_step(A64 A) {
     u32* cf = A.cf + (size_t)i * D64_CAP;
     unsigned long long key[D64_CAP];
     u32 n = 0, st = 0;
-    for (u32 j = 0; j < D64_LANES; ++j) {
-        const u32 tid = i * D64_LANES + j;
-        const u32 m = min(A.ln[tid], D64_LCAP);
-        for (u32 c = 0; c < m; ++c) {
-            const size_t o = (size_t)tid * D64_LCAP + c;
-            const unsigned long long kc = ((unsigned long long)A.lk[o] << 32) | A.lf[o];
-            bool seen = false;
-            for (u32 e = 0; e < n && !seen; ++e) seen = key[e] == kc;
-            if (seen) continue;
-            if (n >= D64_CAP) { st |= YS_FLAG_CONTACT_OVF; continue; }
-            u32 s2 = n++;
-            while (s2 > 0 && key[s2 - 1] > kc) {
-                key[s2] = key[s2 - 1];
-                cs[s2] = cs[s2 - 1];
-                cf[s2] = cf[s2 - 1];
-                --s2;
-            }
-            key[s2] = kc;
-            cs[s2] = A.ls[o];
-            cf[s2] = A.lf[o];
+    const u32 m0 = min(A.ln[i], D64_CAP);
+    for (u32 c = 0; c < m0; ++c) {
+        const size_t o = (size_t)i * D64_CAP + c;
+        const unsigned long long kc = ((unsigned long long)A.lk[o] << 32) | A.lf[o];
+        u32 s2 = n++;
+        while (s2 > 0 && key[s2 - 1] > kc) {
+            key[s2] = key[s2 - 1];
+            cs[s2] = cs[s2 - 1];
+            cf[s2] = cf[s2 - 1];
+            --s2;
         }
+        key[s2] = kc;
+        cs[s2] = A.ls[o];
+        cf[s2] = A.lf[o];
     }
     A.cn[i] = n;
     const dd3 f = force64(A, A.x, A.v, i);

@@ -2294,7 +2294,7 @@ ys_status fused_substep(ys_scene* s) {
     return YS_OK;
 }
 
-// Sorted-leaf groups of a cube-layout scene: which boxes each mesh needs, where
+// Sorted-leaf groups: which boxes each mesh needs, where
 // they lie, and the jobs that write them.
 //   key boxes    self rows of the CPU-hash semantics
 //   query boxes  a target of some query mesh, or BVH self rows
@@ -2320,7 +2320,10 @@ ys_status group_layout(ys_scene* s, std::vector<MeshDev>& md, const std::vector<
             if (!(T.flags & MF_ANALYTIC) && !(H.flags & MF_ANALYTIC)) need[targets[k]] |= GJ_BOX | GJ_REC | GJ_ROOT;
         }
     }
-    if (s->tree_layout != YS_TREE_CUBE) std::fill(need.begin(), need.end(), 0u);
+    // under the reference layout the fused path descends the binary trees; the
+    // binary64 rollout still queries the static obstacles' groups
+    for (size_t m = 0; m < nm; ++m)
+        if (s->tree_layout != YS_TREE_CUBE && (live[m] || !(s->meshes[m].flags & MF_STATIC))) need[m] = 0;
     u32 l0 = 0, rec = 0, dyn = 0, fix = 0;
     std::vector<GroupJob> build(nm), step;
     for (size_t m = 0; m < nm; ++m) {
@@ -3541,7 +3544,7 @@ struct ys_adjoint {
     std::vector<DBuf<u32>> dst_f, dst_n;
     DBuf<D4> dX[3], dV[2];
     DBuf<DContact> dsc_c;  // contacts of steps that are not recorded
-    DBuf<DContact> dls;    // contact search output per (vertex, search thread)
+    DBuf<DContact> dls;    // contact search output per vertex
     DBuf<u32> dlf, dlk, dln;
     DBuf<u32> dsc_f, dsc_n;
     DBuf<D4> dax, dav, dax2, dav2, dxbar, dvbar, dfbar;
@@ -3600,8 +3603,7 @@ cudaError_t d64_alloc(ys_adjoint* a) {
         if ((e = b->alloc(n))) return e;
     if ((e = a->d_k.alloc(a->S)) || (e = a->d_L.alloc(a->S)) || (e = a->dgk.alloc(a->S)) || (e = a->dgL.alloc(a->S)))
         return e;
-    const size_t nl = n * D64_LANES, cl = nl * D64_LCAP;
-    if ((e = a->dls.alloc(cl)) || (e = a->dlf.alloc(cl)) || (e = a->dlk.alloc(cl)) || (e = a->dln.alloc(nl))) return e;
+    if ((e = a->dls.alloc(c)) || (e = a->dlf.alloc(c)) || (e = a->dlk.alloc(c)) || (e = a->dln.alloc(n))) return e;
     if ((e = a->dsc_c.alloc(c)) || (e = a->dsc_f.alloc(c)) || (e = a->dsc_n.alloc(n)) || (e = a->dbox.alloc(6)) ||
         (e = a->dstatus.alloc(1)))
         return e;
@@ -3666,7 +3668,9 @@ A64 d64_args(ys_adjoint* a) {
     memset(&A, 0, sizeof(A));
     A.sx = s->X[s->cur].p;
     A.F = s->F4.p;
-    A.nodes = s->nodes.p;
+    A.grp = group_bufs(s);
+    A.lvid = s->lvid.p;
+    A.vpw = vertices_per_warp(a->nV);
     A.meshes = s->dmeshes.p;
     A.targets = s->targets.p;
     A.ext = s->use_ext ? s->ext.p : nullptr;
@@ -3698,7 +3702,7 @@ void d64_step(ys_adjoint* a, A64 A, cudaStream_t st) {
     cudaMemsetAsync(a->dbox.p, 0, 6 * sizeof(unsigned long long), st);
     const u32 gb = std::min<u32>(ceil_div(a->nV, 256), 148 * 4);
     k_d64_box<<<gb, 256, 0, st>>>(A);
-    k_d64_cand<<<ceil_div(a->nV * D64_LANES, D64_BLOCK), D64_BLOCK, 0, st>>>(A);
+    k_d64_cand<<<ceil_div(a->nV, A.vpw * (D64_BLOCK / 32)), D64_BLOCK, 0, st>>>(A);
     k_d64_step<<<ceil_div(a->nV, D64_BLOCK), D64_BLOCK, 0, st>>>(A);
 }
 
@@ -3707,7 +3711,6 @@ ys_status d64_status(ys_adjoint* a) {
     YS_CK(cudaMemcpyAsync(&f, a->dstatus.p, 4, cudaMemcpyDeviceToHost, a->s->stream));
     YS_CK(cudaStreamSynchronize(a->s->stream));
     if (f & YS_FLAG_CONTACT_OVF) return fail(YS_ERR_CAPACITY, "FP64 rollout: more than 16 contacts at a vertex");
-    if (f & YS_FLAG_STACK_OVF) return fail(YS_ERR_CAPACITY, "FP64 rollout: tree descent stack exceeded");
     return YS_OK;
 }
 
