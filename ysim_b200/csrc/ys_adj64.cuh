@@ -145,22 +145,73 @@ __device__ __forceinline__ bool narrow64(dd3 qc, dd3 qp, dd3 t0, dd3 t1, dd3 t2,
     return true;
 }
 
-// Force on cloth vertex i (local) from the state (x, v).
-__device__ __forceinline__ dd3 force64(const A64& A, const D4* x, const D4* v, u32 i) {
+// Spring q (0 .. 11, in grid_stencil's order) of grid vertex (row, col): its
+// other end and id; false when the cloth ends before it.
+__device__ __forceinline__ bool grid_spring(int N, int row, int col, int q, u32& j, u32& sid) {
+    // per spring: row and column offset, family, and the first end's offset
+    // from the vertex (the id counts first ends, row-major in the family)
+    static constexpr signed char DR[12] = {0, 0, -1, 1, -1, -1, 1, 1, 0, 0, -2, 2};
+    static constexpr signed char DC[12] = {-1, 1, 0, 0, -1, 1, -1, 1, -2, 2, 0, 0};
+    if (q >= 12) return false;
+    int dr = 0, dc = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+        if (q == k) { dr = DR[k]; dc = DC[k]; }
+    const int r = row + dr, c = col + dc;
+    if (r < 0 || r >= N || c < 0 || c >= N) return false;
+    j = (u32)(r * N + c);
+    const u32 n = (u32)N, top = (u32)min(row, r), left = (u32)min(col, c);
+    const u32 bSY = n * (n - 1), bHA = bSY + (n - 1) * n, bHB = bHA + (n - 1) * (n - 1), bBX = bHB + (n - 1) * (n - 1),
+              bBY = bBX + n * (n - 2);
+    if (dr == 0) sid = dc * dc == 1 ? top * (n - 1) + left : bBX + top * (n - 2) + left;
+    else if (dc == 0) sid = dr * dr == 1 ? bSY + top * n + left : bBY + top * n + left;
+    else sid = (dr == dc ? bHA : bHB) + top * (n - 1) + left;
+    return true;
+}
+
+// LPV lanes per vertex: 1 (a thread runs its vertex's 12 springs) or 16 (a
+// lane per spring, then every lane adds the forces in the stencil's order).
+// With a thread per vertex a small cloth is a hundred warps of twelve
+// dependent square roots and divisions each; a lane per spring issues three
+// times the instructions (a step, a vertex and a springs pass of the 65 x 65
+// cloth: 8.1 / 7.8 / 12.0 us by thread, 4.2 / 4.3 / 5.0 us by lane).
+static constexpr u32 D64_SPREAD = 65536;  // vertices up to which a lane per spring is used
+__device__ __forceinline__ double d64_from(double v, int q) { return __shfl_sync(0xFFFFFFFFu, v, q, 16); }
+
+// Force on cloth vertex i (local) from the state (x, v); q: this lane's
+// spring (LPV 16; every lane of the warp calls).
+template <int LPV>
+__device__ __forceinline__ dd3 force64(const A64& A, const D4* x, const D4* v, u32 i, int q) {
     const u32 g = A.voff + i;
     const dd3 p = ldd(x, i), w = ldd(v, i);
     const double m = (double)A.mass[g];
     const dd3 f0 = A.ext ? ldf(A.ext, g) : dm(A.gx * m, A.gy * m, A.gz * m);
     dd3 f = f0 + w * A.kair;
     const int N = (int)A.N, row = (int)(i / A.N), col = (int)(i % A.N);
-    grid_stencil(N, row, col, [&](int r, int c, int, u32 sid) {
-        const u32 j = (u32)(r * N + c);
+    auto one = [&](u32 j, u32 sid, dd3& s) {
         const dd3 dx = ldd(x, j) - p, dv = ldd(v, j) - w;
         const double l = sqrt(ddot(dx, dx));
-        if (l < 1e-7) return;
+        if (l < 1e-7) return false;
         const dd3 nd = dx * (1.0 / l);
-        f = f + nd * (A.k[sid] * (l - A.L[sid]) + A.kd * ddot(dv, nd));
-    });
+        s = nd * (A.k[sid] * (l - A.L[sid]) + A.kd * ddot(dv, nd));
+        return true;
+    };
+    if constexpr (LPV == 1) {
+        grid_stencil(N, row, col, [&](int r, int c, int, u32 sid) {
+            dd3 s;
+            if (one((u32)(r * N + c), sid, s)) f = f + s;
+        });
+    } else {
+        u32 j = 0, sid = 0;
+        dd3 s = dm(0.0, 0.0, 0.0);
+        const bool on = grid_spring(N, row, col, q, j, sid) && one(j, sid, s);
+        const unsigned have = __ballot_sync(0xFFFFFFFFu, on) >> (threadIdx.x & 16u);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const dd3 t = dm(d64_from(s.x, k), d64_from(s.y, k), d64_from(s.z, k));
+            if ((have >> k) & 1u) f = f + t;
+        }
+    }
     return f;
 }
 
@@ -315,9 +366,13 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_cand(A64 A) {
 // One step of the FP64 rollout for each vertex: its contacts sorted by
 // (object, face) (recorded in cs / cf / cn), then forces, integration and the
 // contact response.
+template <int LPV>
 __global__ void __launch_bounds__(D64_BLOCK) k_d64_step(A64 A) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.nV) return;
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % LPV;
+    const bool in = t / LPV < A.nV;
+    const u32 i = in ? t / LPV : A.nV - 1;  // threads past the end help with the last vertex's sums and drop them
+    const dd3 f = force64<LPV>(A, A.x, A.v, i, (int)lane);
+    if (!in || lane != 0) return;
     const u32 g = A.voff + i;
     const dd3 p = ldd(A.x, i);
     DContact* cs = A.cs + (size_t)i * D64_CAP;
@@ -340,7 +395,6 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_step(A64 A) {
         cf[s2] = A.lf[o];
     }
     A.cn[i] = n;
-    const dd3 f = force64(A, A.x, A.v, i);
     const double m = (double)A.mass[g], mk_ = (double)A.mask[g];
     dd3 vel = ldd(A.v, i) + f * (A.subh / m * mk_);
     dd3 pos = p;
@@ -376,13 +430,16 @@ struct J64 {
 
 // Reverse of the integration and the contact response of step t (the
 // forward's active set replayed from the recorded contacts).
+template <int LPV>
 __global__ void __launch_bounds__(D64_BLOCK) k_d64_adj_vertex(A64 A, J64 J) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.nV) return;
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % LPV;
+    const bool in = t / LPV < A.nV;
+    const u32 i = in ? t / LPV : A.nV - 1;
+    const dd3 f = force64<LPV>(A, A.x, A.v, i, (int)lane);
+    if (!in || lane != 0) return;
     const u32 g = A.voff + i;
     const DContact* cs = A.cs + (size_t)i * D64_CAP;
     const u32 n = A.cn[i] < D64_CAP ? A.cn[i] : D64_CAP;
-    const dd3 f = force64(A, A.x, A.v, i);
     const double m = (double)A.mass[g], mk_ = (double)A.mask[g];
     const double s = A.subh / m * mk_;
     dd3 vel = ldd(A.v, i) + f * s;
@@ -421,35 +478,74 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_adj_vertex(A64 A, J64 J) {
 
 // Reverse of the spring and drag forces of step t: gathered per vertex, the
 // spring parameters' gradients accumulated by the lower-index end.
+template <int LPV>
 __global__ void __launch_bounds__(D64_BLOCK) k_d64_adj_springs(A64 A, J64 J) {
-    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.nV) return;
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, lane = t % LPV;
+    const bool in = t / LPV < A.nV;
+    const u32 i = in ? t / LPV : A.nV - 1;
     const int N = (int)A.N, row = (int)(i / A.N), col = (int)(i % A.N);
     const dd3 p = ldd(A.x, i), w = ldd(A.v, i), fi = ldd(J.fbar, i);
     const double kd = A.kd;
     dd3 dxb = dm(0.0, 0.0, 0.0), dvb = dm(0.0, 0.0, 0.0);
-    grid_stencil(N, row, col, [&](int r, int c, int, u32 sid) {
-        const u32 j = (u32)(r * N + c);
+    auto one = [&](u32 j, u32 sid, dd3& ddx, dd3& ddv) {
         const dd3 dx = ldd(A.x, j) - p, dv = ldd(A.v, j) - w;
         const double l = sqrt(ddot(dx, dx));
-        if (l < 1e-7) return;
+        if (l < 1e-7) return false;
         const double k = A.k[sid], rest = A.L[sid];
         const dd3 nd = dx * (1.0 / l);
         const double a = k * (l - rest) + kd * ddot(dv, nd);
         const dd3 gdir = fi - ldd(J.fbar, j);
         const double ng = ddot(nd, gdir);
         const dd3 dvp = dv - nd * ddot(nd, dv), gp = gdir - nd * ng;
-        const dd3 ddx = nd * (k * ng) + dvp * (kd * ng / l) + gp * (a / l);
-        const dd3 ddv = nd * (kd * ng);
-        dxb = dxb - ddx;
-        dvb = dvb - ddv;
-        if (i < j) {  // one owner per spring: no race on the accumulators
+        ddx = nd * (k * ng) + dvp * (kd * ng / l) + gp * (a / l);
+        ddv = nd * (kd * ng);
+        if (in && i < j) {  // one owner per spring: no race on the accumulators
             J.gk[sid] += (l - rest) * ng;
             J.gL[sid] += -k * ng;
         }
-    });
+        return true;
+    };
+    dd3 ddx = dm(0.0, 0.0, 0.0), ddv = dm(0.0, 0.0, 0.0);
+    if constexpr (LPV == 1) {
+        grid_stencil(N, row, col, [&](int r, int c, int, u32 sid) {
+            if (!one((u32)(r * N + c), sid, ddx, ddv)) return;
+            dxb = dxb - ddx;
+            dvb = dvb - ddv;
+        });
+    } else {
+        u32 j = 0, sid = 0;
+        const bool on = grid_spring(N, row, col, (int)lane, j, sid) && one(j, sid, ddx, ddv);
+        const unsigned have = __ballot_sync(0xFFFFFFFFu, on) >> (threadIdx.x & 16u);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const dd3 a = dm(d64_from(ddx.x, k), d64_from(ddx.y, k), d64_from(ddx.z, k));
+            const dd3 c = dm(d64_from(ddv.x, k), d64_from(ddv.y, k), d64_from(ddv.z, k));
+            if ((have >> k) & 1u) {
+                dxb = dxb - a;
+                dvb = dvb - c;
+            }
+        }
+    }
+    if (!in || lane != 0) return;
     std4(J.ax_out, i, ldd(J.xbar, i) + dxb);
     std4(J.av_out, i, ldd(J.vbar, i) + (dvb + fi * A.kair));
+}
+
+// The per-vertex kernels with a lane per spring or a thread per vertex.
+inline void launch_d64_step(const A64& A, cudaStream_t st) {
+    if (A.nV <= D64_SPREAD) k_d64_step<16><<<ceil_div((long long)A.nV * 16, D64_BLOCK), D64_BLOCK, 0, st>>>(A);
+    else k_d64_step<1><<<ceil_div(A.nV, D64_BLOCK), D64_BLOCK, 0, st>>>(A);
+}
+inline void launch_d64_adjoint(const A64& A, const J64& J, cudaStream_t st) {
+    if (A.nV <= D64_SPREAD) {
+        const int g = ceil_div((long long)A.nV * 16, D64_BLOCK);
+        k_d64_adj_vertex<16><<<g, D64_BLOCK, 0, st>>>(A, J);
+        k_d64_adj_springs<16><<<g, D64_BLOCK, 0, st>>>(A, J);
+    } else {
+        const int g = ceil_div(A.nV, D64_BLOCK);
+        k_d64_adj_vertex<1><<<g, D64_BLOCK, 0, st>>>(A, J);
+        k_d64_adj_springs<1><<<g, D64_BLOCK, 0, st>>>(A, J);
+    }
 }
 
 __global__ void k_d64_from_f4(const float4* __restrict__ in, D4* __restrict__ out, u32 voff, u32 n) {

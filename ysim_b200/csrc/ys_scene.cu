@@ -3703,7 +3703,7 @@ void d64_step(ys_adjoint* a, A64 A, cudaStream_t st) {
     const u32 gb = std::min<u32>(ceil_div(a->nV, 256), 148 * 4);
     k_d64_box<<<gb, 256, 0, st>>>(A);
     k_d64_cand<<<ceil_div(a->nV, A.vpw * (D64_BLOCK / 32)), D64_BLOCK, 0, st>>>(A);
-    k_d64_step<<<ceil_div(a->nV, D64_BLOCK), D64_BLOCK, 0, st>>>(A);
+    launch_d64_step(A, st);
 }
 
 ys_status d64_status(ys_adjoint* a) {
@@ -3782,8 +3782,7 @@ ys_status d64_enqueue_backward(ys_adjoint* a) {
             J64 J;
             J.ax = ax; J.av = av; J.xbar = a->dxbar.p; J.vbar = a->dvbar.p; J.fbar = a->dfbar.p;
             J.ax_out = ax2; J.av_out = av2; J.gk = a->dgk.p; J.gL = a->dgL.p;
-            k_d64_adj_vertex<<<ceil_div(a->nV, D64_BLOCK), D64_BLOCK, 0, st>>>(A, J);
-            k_d64_adj_springs<<<ceil_div(a->nV, D64_BLOCK), D64_BLOCK, 0, st>>>(A, J);
+            launch_d64_adjoint(A, J, st);
             std::swap(ax, ax2);
             std::swap(av, av2);
         }
