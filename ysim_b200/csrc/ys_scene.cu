@@ -1543,6 +1543,7 @@ struct ys_scene {
     // refit + fused substep replayed without host launch overhead
     bool use_graphs = true;
     cudaGraphExec_t graphs[18] = {};
+    uint64_t graph_epoch = 0;        // counts what made captured substeps stale (drop_graphs)
     int fused_min_blocks = 8;        // k_fused register cap (ys_scene_set_fused_variant / ys_scene_autotune)
     // fused-kernel thread order (ys_scene_set_thread_order): working vertices
     // in Morton order per mesh, recomputed at every tree rebuild
@@ -2215,6 +2216,7 @@ ys_status system_update(ys_scene* s) {
 }
 
 void drop_graphs(ys_scene* s) {
+    ++s->graph_epoch;
     for (auto& g : s->graphs)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
@@ -3518,6 +3520,19 @@ __global__ void k_mesh_unpack4(const float4* __restrict__ in, float* __restrict_
 
 #include "ys_adj64.cuh"
 
+// A whole pass of the binary32 rollout as a graph, from the second pass on (a
+// capture costs about one pass: 100 steps 12 ms, against 3 ms that it saves
+// each later one).  It starts from the first
+// buffers (cur 0, prev 1, velocity 0), so the buffers of every step are fixed;
+// epoch: the scene's captured-substep epoch it belongs to; the rest: the
+// scene's host state after the pass.
+struct AdjGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t runs = 0, epoch = 0, frame = 0;
+    u32 cursor = 0;
+    int cur = 0, prev = 0, cv = 0, stale = -1;
+};
+
 struct ys_adjoint {
     ys_scene* s = nullptr;
     int mesh = 0;
@@ -3533,6 +3548,9 @@ struct ys_adjoint {
     std::vector<DBuf<VContact>> st_pool;
     DBuf<float4> ax, av, ax2, av2, xbar, vbar, fbar;
     bool forward_done = false;
+    // the two passes as one graph each (AdjGraph)
+    AdjGraph c_fwd, c_bwd;
+    DBuf<float> gk, gL;  // the backward graph's spring gradients
     // 64-bit mode (ys_adjoint_set_precision): the cloth's state in binary64
     // (local vertex index), the parameters, checkpoints, one segment of
     // recorded steps (states and sorted contacts), the reverse-pass buffers
@@ -3572,6 +3590,62 @@ void restore_state(ys_scene* s, const float4* x, const float4* xp, const float4*
     s->frame = frame;
     s->cursor = cursor;
     s->snapshot_pending = false;
+}
+
+// No substep of the rollout rebuilds a tree or reads a collider's pose, so a
+// pass is the same sequence of launches every time; up to ADJ_GRAPH_STEPS of
+// them go into one graph (a substep is four nodes; longer passes launch a graph
+// per substep).
+static constexpr u32 ADJ_GRAPH_STEPS = 1024;
+bool adj_capturable(const ys_adjoint* a) {
+    const ys_scene* s = a->s;
+    if (!s->use_graphs || s->timing || a->T > ADJ_GRAPH_STEPS || !s->shape_mesh.empty()) return false;
+    for (auto& H : s->meshes)
+        if (H.needs_tree && !(H.built && H.d.behavior == YS_FLOAT)) return false;
+    return true;
+}
+
+// Run a pass through its graph; enqueue() issues the pass from the first
+// buffers and rotates the scene's host state along.
+template <class Fn>
+ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
+    ys_scene* s = a->s;
+    cudaStream_t st = s->stream;
+    if (G.exec && G.epoch != s->graph_epoch) {
+        YS_CK(cudaStreamSynchronize(st));
+        cudaGraphExecDestroy(G.exec);
+        G.exec = nullptr;
+    }
+    const uint64_t run0 = s->substeps_run;
+    if (!G.exec) {
+        cudaGraph_t g = nullptr;
+        YS_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        const ys_status er = enqueue();
+        cudaError_t ce = cudaStreamEndCapture(st, &g);
+        if (er) { if (g) cudaGraphDestroy(g); return er; }
+        if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+        ce = cudaGraphInstantiate(&G.exec, g, 0);
+        cudaGraphDestroy(g);
+        if (ce != cudaSuccess) { G.exec = nullptr; return fail(YS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)); }
+        G.epoch = s->graph_epoch;
+        G.frame = s->frame; G.cursor = s->cursor; G.cur = s->cur; G.prev = s->prev; G.cv = s->cv; G.stale = s->refit_stale;
+    }
+    YS_CK(cudaGraphLaunch(G.exec, st));
+    s->frame = G.frame; s->cursor = G.cursor; s->cur = G.cur; s->prev = G.prev; s->cv = G.cv; s->refit_stale = G.stale;
+    s->snapshot_pending = false;
+    s->substeps_run = run0 + substeps;
+    return YS_OK;
+}
+
+// One substep of a pass under capture.
+ys_status adj_substep(ys_scene* s) {
+    const ys_status r = enqueue_fused(s);
+    if (r) return r;
+    mark_refit(s);
+    s->snapshot_pending = true;
+    rotate(s);
+    if (s->record) s->last_contacts = 2;
+    return YS_OK;
 }
 
 // ---- 64-bit mode
@@ -3879,6 +3953,10 @@ ys_status ys_scene_set_grid_springs(ys_scene* s, int mesh, const float* d_k, con
     const u32 base = s->hmeshes[mesh].gspr;
     if (d_k) YS_CK(cudaMemcpyAsync(s->gk.p + base, d_k, 4 * S, cudaMemcpyDeviceToDevice, s->stream));
     if (d_L) YS_CK(cudaMemcpyAsync(s->gL.p + base, d_L, 4 * S, cudaMemcpyDeviceToDevice, s->stream));
+    if (H.grid_springs_on) {  // new values in the arrays that the kernels read already
+        YS_CK(cudaStreamSynchronize(s->stream));
+        return YS_OK;
+    }
     std::vector<MeshDev> md = s->hmeshes;
     for (size_t m = 0; m < md.size(); ++m)
         if ((int)m != mesh && md[m].gspr != NO_SPRINGS && !s->meshes[m].grid_springs_on) md[m].gspr = NO_SPRINGS;
@@ -3942,6 +4020,9 @@ ys_status ys_adjoint_destroy(ys_adjoint* a) {
     for (auto& b : a->st_pool) b.free();
     a->x0.free(); a->v0.free(); a->ax.free(); a->av.free(); a->ax2.free(); a->av2.free();
     a->xbar.free(); a->vbar.free(); a->fbar.free();
+    a->gk.free(); a->gL.free();
+    for (auto* G : {&a->c_fwd, &a->c_bwd})
+        if (G->exec) cudaGraphExecDestroy(G->exec);
     d64_free(a);
     delete a;
     return YS_OK;
@@ -4063,23 +4144,30 @@ ys_status ys_adjoint_forward(ys_adjoint* a, float* d_xT) {
         YS_CK(cudaGetLastError());
         return YS_OK;
     }
+    ys_status r = refresh_wide(s);
+    if (r) return r;
+    s->cur = 0; s->prev = 1; s->cv = 0;
     restore_state(s, a->x0.p, a->x0.p, a->v0.p, 0, 0);
     const bool rec = s->record;
     s->record = false;
-    ys_status r = YS_OK;
-    for (u32 t = 0; t < a->T && !r; ++t) {
-        if (t % a->K == 0) {
-            const u32 i = t / a->K;
-            const size_t bytes = sizeof(float4) * s->nV;
-            const float4* xp = s->snapshot_pending ? s->X[s->cur].p : s->X[s->prev].p;
-            YS_CK(cudaMemcpyAsync(a->ck_x[i].p, s->X[s->cur].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
-            YS_CK(cudaMemcpyAsync(a->ck_xp[i].p, xp, bytes, cudaMemcpyDeviceToDevice, s->stream));
-            YS_CK(cudaMemcpyAsync(a->ck_v[i].p, s->V[s->cv].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
-            a->ck_frame[i] = s->frame;
-            a->ck_cursor[i] = s->cursor;
+    auto pass = [&](auto&& substep) -> ys_status {
+        for (u32 t = 0; t < a->T; ++t) {
+            if (t % a->K == 0) {
+                const u32 i = t / a->K;
+                const size_t bytes = sizeof(float4) * s->nV;
+                const float4* xp = s->snapshot_pending ? s->X[s->cur].p : s->X[s->prev].p;
+                YS_CK(cudaMemcpyAsync(a->ck_x[i].p, s->X[s->cur].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+                YS_CK(cudaMemcpyAsync(a->ck_xp[i].p, xp, bytes, cudaMemcpyDeviceToDevice, s->stream));
+                YS_CK(cudaMemcpyAsync(a->ck_v[i].p, s->V[s->cv].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+                a->ck_frame[i] = s->frame;
+                a->ck_cursor[i] = s->cursor;
+            }
+            const ys_status q = substep(s);
+            if (q) return q;
         }
-        r = fused_substep(s);
-    }
+        return YS_OK;
+    };
+    r = (a->c_fwd.runs++ && adj_capturable(a)) ? adj_graph(a, a->c_fwd, a->T, [&] { return pass(adj_substep); }) : pass(fused_substep);
     s->record = rec;
     if (r) return r;
     if (d_xT) k_mesh_unpack4<<<ceil_div(a->nV, 256), 256, 0, s->stream>>>(s->X[s->cur].p, d_xT, a->voff, a->nV);
@@ -4108,55 +4196,83 @@ ys_status ys_adjoint_backward(ys_adjoint* a, const float* d_dLdx, float* d_gk, f
         return YS_OK;
     }
     const size_t bytes = sizeof(float4) * s->nV;
-    YS_CK(cudaMemsetAsync(a->ax.p, 0, bytes, st));
-    YS_CK(cudaMemsetAsync(a->av.p, 0, bytes, st));
-    k_mesh_pack4<<<ceil_div(a->nV, 256), 256, 0, st>>>(d_dLdx, a->ax.p, a->voff, a->nV);
-    YS_CK(cudaMemsetAsync(d_gk, 0, 4 * (size_t)a->S, st));
-    YS_CK(cudaMemsetAsync(d_gL, 0, 4 * (size_t)a->S, st));
-    ys_status r = YS_OK;
-    const bool rec = s->record;
-    VContact* keep_pool = s->pool.p;
-    u32* keep_vs = s->vstart.p;
-    u32* keep_vc = s->vcount.p;
-    if ((r = ensure_record(s))) return r;
-    keep_pool = s->pool.p; keep_vs = s->vstart.p; keep_vc = s->vcount.p;
-    for (int seg = (int)a->nseg - 1; seg >= 0 && !r; --seg) {
-        const u32 t0 = (u32)seg * a->K, t1 = std::min(a->T, t0 + a->K);
-        restore_state(s, a->ck_x[seg].p, a->ck_xp[seg].p, a->ck_v[seg].p, a->ck_frame[seg], a->ck_cursor[seg]);
-        s->record = true;
-        for (u32 t = t0; t < t1 && !r; ++t) {
-            const u32 k = t - t0;
-            YS_CK(cudaMemcpyAsync(a->st_x[k].p, s->X[s->cur].p, bytes, cudaMemcpyDeviceToDevice, st));
-            YS_CK(cudaMemcpyAsync(a->st_v[k].p, s->V[s->cv].p, bytes, cudaMemcpyDeviceToDevice, st));
-            s->pool.p = a->st_pool[k].p;
-            s->vstart.p = a->st_vstart[k].p;
-            s->vcount.p = a->st_vcount[k].p;
-            r = fused_substep(s);
-        }
-        s->pool.p = keep_pool; s->vstart.p = keep_vs; s->vcount.p = keep_vc;
-        s->record = rec;
-        if (r) break;
-        for (int t = (int)t1 - 1; t >= (int)t0; --t) {
-            const u32 k = (u32)t - t0;
-            StepArgs A = make_args(s);
-            AdjArgs J;
-            J.x = a->st_x[k].p; J.v = a->st_v[k].p;
-            J.vstart = a->st_vstart[k].p; J.vcount = a->st_vcount[k].p; J.pool = a->st_pool[k].p;
-            J.ax = a->ax.p; J.av = a->av.p; J.xbar = a->xbar.p; J.vbar = a->vbar.p; J.fbar = a->fbar.p;
-            J.ax_out = a->ax2.p; J.av_out = a->av2.p;
-            J.gk = d_gk; J.gL = d_gL;
-            J.voff = a->voff; J.nV = a->nV; J.N = a->N;
-            // forces at step t read the step's own state
-            A.x = J.x; A.v = J.v;
-            k_adj_vertex<<<ceil_div(a->nV, 128), 128, 0, st>>>(A, J, (u32)a->mesh);
-            k_adj_springs<<<ceil_div(a->nV, 128), 128, 0, st>>>(A, J, (u32)a->mesh);
-            YS_CK(cudaGetLastError());
-            std::swap(a->ax.p, a->ax2.p);
-            std::swap(a->av.p, a->av2.p);
-        }
+    const bool whole = a->c_bwd.runs++ && adj_capturable(a);
+    if (whole && !a->gk.p) {
+        YS_CK(a->gk.alloc(a->S));
+        YS_CK(a->gL.alloc(a->S));
     }
+    float *gk = whole ? a->gk.p : d_gk, *gL = whole ? a->gL.p : d_gL;
+    YS_CK(cudaMemsetAsync(a->ax.p, 0, bytes, st));
+    k_mesh_pack4<<<ceil_div(a->nV, 256), 256, 0, st>>>(d_dLdx, a->ax.p, a->voff, a->nV);
+    ys_status r = refresh_wide(s);
     if (r) return r;
-    k_mesh_unpack4<<<ceil_div(a->nV, 256), 256, 0, st>>>(a->av.p, d_gv0, a->voff, a->nV);
+    const bool rec = s->record;
+    if ((r = ensure_record(s))) return r;
+    VContact* keep_pool = s->pool.p;
+    u32 *keep_vs = s->vstart.p, *keep_vc = s->vcount.p;
+    s->cur = 0; s->prev = 1; s->cv = 0;
+    // the adjoints ping-pong between two buffers each, from these
+    float4 *ax0 = a->ax.p, *ax20 = a->ax2.p, *av0 = a->av.p, *av20 = a->av2.p;
+    auto pass = [&](auto&& substep) -> ys_status {
+        YS_CK(cudaMemsetAsync(a->av.p, 0, bytes, st));
+        YS_CK(cudaMemsetAsync(gk, 0, 4 * (size_t)a->S, st));
+        YS_CK(cudaMemsetAsync(gL, 0, 4 * (size_t)a->S, st));
+        ys_status q = YS_OK;
+        for (int seg = (int)a->nseg - 1; seg >= 0 && !q; --seg) {
+            const u32 t0 = (u32)seg * a->K, t1 = std::min(a->T, t0 + a->K);
+            restore_state(s, a->ck_x[seg].p, a->ck_xp[seg].p, a->ck_v[seg].p, a->ck_frame[seg], a->ck_cursor[seg]);
+            s->record = true;
+            for (u32 t = t0; t < t1 && !q; ++t) {
+                const u32 k = t - t0;
+                YS_CK(cudaMemcpyAsync(a->st_x[k].p, s->X[s->cur].p, bytes, cudaMemcpyDeviceToDevice, st));
+                YS_CK(cudaMemcpyAsync(a->st_v[k].p, s->V[s->cv].p, bytes, cudaMemcpyDeviceToDevice, st));
+                s->pool.p = a->st_pool[k].p;
+                s->vstart.p = a->st_vstart[k].p;
+                s->vcount.p = a->st_vcount[k].p;
+                q = substep(s);
+            }
+            s->pool.p = keep_pool; s->vstart.p = keep_vs; s->vcount.p = keep_vc;
+            s->record = rec;
+            for (int t = (int)t1 - 1; t >= (int)t0 && !q; --t) {
+                const u32 k = (u32)t - t0;
+                StepArgs A = make_args(s);
+                AdjArgs J;
+                J.x = a->st_x[k].p; J.v = a->st_v[k].p;
+                J.vstart = a->st_vstart[k].p; J.vcount = a->st_vcount[k].p; J.pool = a->st_pool[k].p;
+                J.ax = a->ax.p; J.av = a->av.p; J.xbar = a->xbar.p; J.vbar = a->vbar.p; J.fbar = a->fbar.p;
+                J.ax_out = a->ax2.p; J.av_out = a->av2.p;
+                J.gk = gk; J.gL = gL;
+                J.voff = a->voff; J.nV = a->nV; J.N = a->N;
+                // forces at step t read the step's own state
+                A.x = J.x; A.v = J.v;
+                k_adj_vertex<<<ceil_div(a->nV, 128), 128, 0, st>>>(A, J, (u32)a->mesh);
+                k_adj_springs<<<ceil_div(a->nV, 128), 128, 0, st>>>(A, J, (u32)a->mesh);
+                YS_CK(cudaGetLastError());
+                std::swap(a->ax.p, a->ax2.p);
+                std::swap(a->av.p, a->av2.p);
+            }
+        }
+        return q;
+    };
+    if (whole) {
+        r = adj_graph(a, a->c_bwd, a->T, [&] { return pass(adj_substep); });
+        s->last_contacts = 2;
+        if (!r) {
+            YS_CK(cudaMemcpyAsync(d_gk, gk, 4 * (size_t)a->S, cudaMemcpyDeviceToDevice, st));
+            YS_CK(cudaMemcpyAsync(d_gL, gL, 4 * (size_t)a->S, cudaMemcpyDeviceToDevice, st));
+        }
+    } else {
+        r = pass(fused_substep);
+    }
+    s->pool.p = keep_pool; s->vstart.p = keep_vs; s->vcount.p = keep_vc;  // also after a failed substep
+    // dL/dv0 lies where T swaps put it; the buffers' names go back for the next pass
+    a->ax.p = ax0; a->ax2.p = ax20;
+    a->av.p = (a->T & 1) ? av20 : av0;
+    a->av2.p = (a->T & 1) ? av0 : av20;
+    s->record = rec;
+    if (!r) k_mesh_unpack4<<<ceil_div(a->nV, 256), 256, 0, st>>>(a->av.p, d_gv0, a->voff, a->nV);
+    a->av.p = av0; a->av2.p = av20;
+    if (r) return r;
     YS_CK(cudaGetLastError());
     YS_CK(cudaStreamSynchronize(st));
     return YS_OK;
