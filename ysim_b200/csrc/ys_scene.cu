@@ -277,21 +277,22 @@ __device__ __forceinline__ f3 vertex_force(const StepArgs& A, const MeshDev& M, 
 }
 
 // ---------------------------------------------------------- grid-cloth tiles
-// A CTA of k_force_tiles is one 16 x 8 tile of a FastGridCloth
-// (16 vertices per tile row).  Each spring with
-// an end in the tile is evaluated once, as the force on its first end a from
-// its second end b.  Seen from b the force is its negation, bit for bit (dx,
-// dv and the unit vector change sign exactly, the length and the scalar
-// factor do not change), except where both ends compute the same value: a
-// component whose dx is exactly zero (+0 in the unit vector from either end)
-// and a degenerate spring (+0 from both ends).  The table keeps those cases
-// in a flag byte per spring, so each vertex sums its 12 stencil springs in
-// the reference's order from the table and gets the per-vertex loop's result
-// exactly, signed zeros included.  890 evaluations per full tile instead of
-// 1536.
+// A CTA of k_force_tiles is one 16 x 8 tile of a FastGridCloth, a thread per
+// vertex.  Each spring with an end in the tile is evaluated once, as the
+// force on its first end a from its second end b: a thread takes the six whose
+// first end is its vertex, all at fixed distances in the loaded tile, and the
+// 118 whose first end lies outside are one more for each thread (TILE_HALO).
+// Seen from b the force is its negation (dx, dv and the unit vector change
+// sign exactly, the length and the scalar factor do not change) but for the
+// sign of a zero, and a zero's sign cannot be told in a sum that is not -0
+// before it; nor does such a sum become -0.  So a vertex adds its 12 stencil
+// springs in the reference's order, subtracting those it is the second end
+// of, and gets the per-vertex loop's bits; a vertex whose force before the
+// springs has a component -0 runs that loop.  886 evaluations per full tile
+// instead of 1536.
 //
-// Springs of the tile, by family (first end a, second end b = a + (dr, dc)),
-// a's rows and columns relative to the tile origin:
+// The forces' table, by family (first end a, second end b = a + (dr, dc)), a's
+// rows and columns relative to the tile origin:
 //   0 stretch x  rows 0..7,  cols -1..15  b = a + (0, 1)
 //   1 stretch y  rows -1..7, cols 0..15   b = a + (1, 0)
 //   2 shear "\\" rows -1..7, cols -1..15  b = a + (1, 1)
@@ -300,22 +301,49 @@ __device__ __forceinline__ f3 vertex_force(const StepArgs& A, const MeshDev& M, 
 //   5 bend y     rows -2..7, cols 0..15   b = a + (2, 0)
 static constexpr int TILE_W = 16, TILE_H = 8;
 static constexpr int HALO_W = TILE_W + 4, HALO_H = TILE_H + 4;  // the stencil reaches 2 vertices out
+static constexpr int TILE_CTAS = 8;  // resident per SM
 static constexpr u32 TILE_BOX_BYTES = HALO_W * HALO_H * 16;      // one float4 buffer's tile
-static constexpr u32 TILE_FLAG_BYTES = 896;                      // one flag byte per tile spring
-// x and v tiles, then the spring flags
-static constexpr size_t TILE_SMEM = 2 * TILE_BOX_BYTES + TILE_FLAG_BYTES;
-// first spring of each family in the tile's table
+// the tile's table: first spring, row length, first row and column of each
+// family, and the step from a to b
 static constexpr u32 TS_SX = 0, TS_SY = 136, TS_HA = 280, TS_HB = 433, TS_BX = 586, TS_BY = 730;
 static constexpr u32 TILE_SPRINGS = 890;
+__host__ __device__ constexpr u32 ts_base(int f) {
+    return f == 0 ? TS_SX : f == 1 ? TS_SY : f == 2 ? TS_HA : f == 3 ? TS_HB : f == 4 ? TS_BX : TS_BY;
+}
+__host__ __device__ constexpr int ts_width(int f) { return f == 4 ? 18 : (f == 1 || f == 5) ? 16 : 17; }
+__host__ __device__ constexpr int ts_row0(int f) { return f == 5 ? -2 : (f >= 1 && f <= 3) ? -1 : 0; }
+__host__ __device__ constexpr int ts_col0(int f) { return f == 4 ? -2 : (f == 0 || f == 2) ? -1 : 0; }
+__host__ __device__ constexpr int ts_dr(int f) { return f == 5 ? 2 : (f >= 1 && f <= 3) ? 1 : 0; }
+__host__ __device__ constexpr int ts_dc(int f) { return f == 4 ? 2 : (f == 0 || f == 2) ? 1 : f == 3 ? -1 : 0; }
+
+// The springs into the tile from a first end outside it, one word each: family
+// | (a's row + 2) << 3 | (a's column + 2) << 7 | table slot << 12 | step in the
+// loaded tile << 22 | dr << 28 | (dc + 1) << 30.
+static constexpr u32 TILE_HALO_N = 118;
+struct TileHalo { u32 e[TILE_HALO_N]; };
+constexpr TileHalo tile_halo() {
+    TileHalo h{};
+    u32 n = 0;
+    for (int f = 0; f < 6; ++f)
+        for (int r = -2; r < TILE_H; ++r)
+            for (int c = -2; c < TILE_W + 2; ++c) {
+                const int br = r + ts_dr(f), bc = c + ts_dc(f);
+                const bool a_in = r >= 0 && c >= 0 && c < TILE_W;
+                const bool b_in = br >= 0 && br < TILE_H && bc >= 0 && bc < TILE_W;
+                if (a_in || !b_in) continue;
+                h.e[n++] = (u32)f | (u32)(r + 2) << 3 | (u32)(c + 2) << 7 |
+                           (ts_base(f) + (u32)((r - ts_row0(f)) * ts_width(f) + c - ts_col0(f))) << 12 |
+                           (u32)(ts_dr(f) * HALO_W + ts_dc(f)) << 22 | (u32)ts_dr(f) << 28 | (u32)(ts_dc(f) + 1) << 30;
+            }
+    return h;
+}
+static __device__ const TileHalo TILE_HALO = tile_halo();
 
 __device__ __forceinline__ u32 smem_u32(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void tile_load(float4* xs, const CUtensorMap* mx, const CUtensorMap* mv, int r0, int c0,
                                           unsigned long long* bar) {
     const u32 b = smem_u32(bar);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     // the maps were written by a host copy: acquire them for the tensor-map proxy
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mx) : "memory");
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mv) : "memory");
@@ -331,113 +359,80 @@ __device__ __forceinline__ void tile_load(float4* xs, const CUtensorMap* mx, con
         ::"r"(smem_u32(xs + HALO_W * HALO_H)), "l"(mv), "r"(0), "r"(c0 - 2), "r"(r0 - 2), "r"(b) : "memory");
 }
 
-// Bounded wait for the tile's two loads (phase 0 of the barrier).
-__device__ __forceinline__ bool tile_wait(unsigned long long* bar) {
+// Bounded wait for the tile's two loads.
+__device__ __forceinline__ bool tile_wait(unsigned long long* bar, u32 phase) {
     const u32 b = smem_u32(bar);
     for (u32 i = 0; i < (1u << 22); ++i) {
         u32 done;
         asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done) : "r"(b) : "memory");
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done) : "r"(b), "r"(phase) : "memory");
         if (done) return true;
     }
     return false;
 }
 
-// The springs of one family of the tile at origin (r0, c0) of a grid mesh of
-// side N: force on a from b into sf[0..2][base + i] (zeros for springs off
-// the mesh).  Thread t starts at (t + 32 * FAM) mod 128, so that each
-// family's remainder past 128 springs falls to another warp.  k and rest are
-// the family's values, or per spring from gk / gL at gspr (not NO_SPRINGS).
-template <int FAM>
-__device__ __forceinline__ void tile_family(const StepArgs& A, u32 gspr, u32 n, int r0, int c0, float kf, float restf,
-                                            const float4* xs, const float4* vs, float* sf, unsigned char* flags) {
-    constexpr u32 W = FAM == 4 ? 18u : ((FAM == 1 || FAM == 5) ? 16u : 17u);
-    constexpr u32 H = FAM == 5 ? 10u : ((FAM >= 1 && FAM <= 3) ? 9u : 8u);
-    constexpr u32 BASE = FAM == 0 ? TS_SX : FAM == 1 ? TS_SY : FAM == 2 ? TS_HA : FAM == 3 ? TS_HB : FAM == 4 ? TS_BX : TS_BY;
-    constexpr int AR = FAM == 5 ? -2 : ((FAM >= 1 && FAM <= 3) ? -1 : 0);
-    constexpr int AC = FAM == 4 ? -2 : ((FAM == 0 || FAM == 2) ? -1 : 0);
-    constexpr int DR = FAM == 5 ? 2 : ((FAM >= 1 && FAM <= 3) ? 1 : 0);
-    constexpr int DC = FAM == 4 ? 2 : ((FAM == 0 || FAM == 2) ? 1 : (FAM == 3 ? -1 : 0));
-    static_assert(BASE + W * H <= TILE_SPRINGS, "tile table");
-    for (u32 i = (threadIdx.x + 32u * FAM) & 127u; i < W * H; i += 128u) {
-        const int rr = (int)(i / W), cc = (int)(i % W);
-        const int ar = r0 + AR + rr, ac = c0 + AC + cc, br = ar + DR, bc = ac + DC;
-        f3 F = mk(0.f, 0.f, 0.f);
-        u32 fl = 0;
-        if ((u32)ar < n && (u32)ac < n && (u32)br < n && (u32)bc < n) {
-            const int ia = (AR + 2 + rr) * HALO_W + (AC + 2 + cc), ib = ia + DR * HALO_W + DC;
-            float k = kf, rest = restf;
-            if (gspr != NO_SPRINGS) {
-                const u32 R = (u32)ar, C = (u32)ac;
-                const u32 bSY = n * (n - 1), bHA = bSY + (n - 1) * n, bHB = bHA + (n - 1) * (n - 1),
-                          bBX = bHB + (n - 1) * (n - 1), bBY = bBX + n * (n - 2);
-                const u32 sid = FAM == 0 ? R * (n - 1) + C
-                              : FAM == 1 ? bSY + R * n + C
-                              : FAM == 2 ? bHA + R * (n - 1) + C
-                              : FAM == 3 ? bHB + R * (n - 1) + C - 1
-                              : FAM == 4 ? bBX + R * (n - 2) + C
-                                         : bBY + R * n + C;
-                k = A.gk[gspr + sid];
-                rest = A.gL[gspr + sid];
-            }
-            const float4 pa = xs[ia], va = vs[ia], pb = xs[ib], vb = vs[ib];
-            const f3 P0 = mk(pa.x, pa.y, pa.z), P1 = mk(pb.x, pb.y, pb.z);
-            F = spring(P0, mk(va.x, va.y, va.z), P1, mk(vb.x, vb.y, vb.z), rest, k, A.kd);
-            // the cases where b computes the same value as a (see above)
-            const f3 dx = P1 - P0;
-            fl = (dx.x == 0.f ? 1u : 0u) | (dx.y == 0.f ? 2u : 0u) | (dx.z == 0.f ? 4u : 0u) |
-                 (sqrtf(dot(dx, dx)) < 1e-7f ? 7u : 0u);
-        }
-        flags[BASE + i] = (unsigned char)fl;
-        sf[BASE + i] = F.x;
-        sf[TILE_SPRINGS + BASE + i] = F.y;
-        sf[2 * TILE_SPRINGS + BASE + i] = F.z;
+// A mesh's spring parameters in shared memory: read through global memory
+// they would be fetched again after every store to the table.
+struct TileMesh { float k[6], rest[6]; };
+
+// k and rest of the spring of family fam whose first end is (R, C).
+__device__ __forceinline__ void tile_spring_kL(const StepArgs& A, const TileMesh& T, u32 gspr, int fam, u32 n, u32 R, u32 C,
+                                               float& k, float& rest) {
+    k = T.k[fam];
+    rest = T.rest[fam];
+    if (gspr != NO_SPRINGS) {
+        const u32 bSY = n * (n - 1), bHA = bSY + (n - 1) * n, bHB = bHA + (n - 1) * (n - 1), bBX = bHB + (n - 1) * (n - 1),
+                  bBY = bBX + n * (n - 2);
+        const u32 sid = gspr + (fam == 0 ? R * (n - 1) + C
+                              : fam == 1 ? bSY + R * n + C
+                              : fam == 2 ? bHA + R * (n - 1) + C
+                              : fam == 3 ? bHB + R * (n - 1) + C - 1
+                              : fam == 4 ? bBX + R * (n - 2) + C
+                                         : bBY + R * n + C);
+        k = __ldg(A.gk + sid);
+        rest = __ldg(A.gL + sid);
     }
 }
 
-// Every spring of the tile at origin (r0, c0) of grid mesh M.
-__device__ __forceinline__ void tile_springs(const StepArgs& A, const MeshDev& M, int r0, int c0, const float4* xs,
-                                             const float4* vs, float* sf, unsigned char* flags) {
-    const u32 n = M.grid_n, gspr = M.gspr;
-    const float ks = M.kstretch, kh = M.kshear, kb = M.kbend;
-    const float r[6] = {M.rest[0], M.rest[1], M.rest[2], M.rest[3], M.rest[4], M.rest[5]};
-    tile_family<0>(A, gspr, n, r0, c0, ks, r[0], xs, vs, sf, flags);
-    tile_family<1>(A, gspr, n, r0, c0, ks, r[1], xs, vs, sf, flags);
-    tile_family<2>(A, gspr, n, r0, c0, kh, r[2], xs, vs, sf, flags);
-    tile_family<3>(A, gspr, n, r0, c0, kh, r[3], xs, vs, sf, flags);
-    tile_family<4>(A, gspr, n, r0, c0, kb, r[4], xs, vs, sf, flags);
-    tile_family<5>(A, gspr, n, r0, c0, kb, r[5], xs, vs, sf, flags);
+// Force on the vertex in slot ia of the loaded tile from the one in slot ib.
+__device__ __forceinline__ f3 tile_spring(const float4* xs, const float4* vs, int ia, int ib, float rest, float k, float kd) {
+    const float4 pa = xs[ia], va = vs[ia], pb = xs[ib], vb = vs[ib];
+    return spring(mk(pa.x, pa.y, pa.z), mk(va.x, va.y, va.z), mk(pb.x, pb.y, pb.z), mk(vb.x, vb.y, vb.z), rest, k, kd);
 }
 
-// The 12 stencil springs of vertex (row, col) at (ty, tx) in its tile, in
-// grid_stencil's order, from the tile's table: the table's force for the
-// springs whose first end is the vertex, its negation for the others (but
-// for the components the flags keep).
-__device__ __forceinline__ f3 tile_force(f3 force, int N, int row, int col, int ty, int tx, const float* sf,
-                                         const unsigned char* flags) {
-    auto add = [&](u32 i, bool neg) {
-        f3 F = mk(sf[i], sf[TILE_SPRINGS + i], sf[2 * TILE_SPRINGS + i]);
-        if (neg) {
-            const u32 fl = flags[i];
-            F = mk((fl & 1u) ? F.x : -F.x, (fl & 2u) ? F.y : -F.y, (fl & 4u) ? F.z : -F.z);
-        }
-        force = force + F;
-    };
-    const u32 y = (u32)ty, x = (u32)tx;
-    if (col > 0) add(TS_SX + y * 17 + x, true);
-    if (col < N - 1) add(TS_SX + y * 17 + x + 1, false);
-    if (row > 0) add(TS_SY + y * 16 + x, true);
-    if (row < N - 1) add(TS_SY + (y + 1) * 16 + x, false);
-    if (col > 0 && row > 0) add(TS_HA + y * 17 + x, true);
-    if (col < N - 1 && row > 0) add(TS_HB + y * 17 + x + 1, true);
-    if (col > 0 && row < N - 1) add(TS_HB + (y + 1) * 17 + x, false);
-    if (col < N - 1 && row < N - 1) add(TS_HA + (y + 1) * 17 + x + 1, false);
-    if (col > 1) add(TS_BX + y * 18 + x, true);
-    if (col < N - 2) add(TS_BX + y * 18 + x + 2, false);
-    if (row > 1) add(TS_BY + y * 16 + x, true);
-    if (row < N - 2) add(TS_BY + (y + 2) * 16 + x, false);
-    return force;
+// The spring of family FAM whose first end is this thread's vertex (row, col),
+// at (ty, tx) in the tile: into the table, and returned.  Zero off the mesh.
+template <int FAM>
+__device__ __forceinline__ f3 tile_own(const StepArgs& A, const TileMesh& T, u32 gspr, u32 n, int row, int col, int ty, int tx,
+                                       const float4* xs, const float4* vs, float* sf) {
+    f3 F = mk(0.f, 0.f, 0.f);
+    if ((u32)(row + ts_dr(FAM)) < n && (u32)(col + ts_dc(FAM)) < n && (u32)row < n && (u32)col < n) {
+        float k, rest;
+        tile_spring_kL(A, T, gspr, FAM, n, (u32)row, (u32)col, k, rest);
+        const int ia = (ty + 2) * HALO_W + tx + 2;
+        F = tile_spring(xs, vs, ia, ia + ts_dr(FAM) * HALO_W + ts_dc(FAM), rest, k, A.kd);
+    }
+    const u32 i = ts_base(FAM) + (u32)((ty - ts_row0(FAM)) * ts_width(FAM) + tx - ts_col0(FAM));
+    sf[i] = F.x;
+    sf[TILE_SPRINGS + i] = F.y;
+    sf[2 * TILE_SPRINGS + i] = F.z;
+    return F;
+}
+
+// The spring of family FAM whose second end is the vertex at (ty, tx).
+template <int FAM>
+__device__ __forceinline__ f3 tile_into(int ty, int tx, const float* sf) {
+    const u32 i = ts_base(FAM) + (u32)((ty - ts_dr(FAM) - ts_row0(FAM)) * ts_width(FAM) + tx - ts_dc(FAM) - ts_col0(FAM));
+    return mk(sf[i], sf[TILE_SPRINGS + i], sf[2 * TILE_SPRINGS + i]);
+}
+
+__device__ __forceinline__ bool has_neg_zero(f3 a) {
+    return (__float_as_uint(a.x) == 0x80000000u) | (__float_as_uint(a.y) == 0x80000000u) |
+           (__float_as_uint(a.z) == 0x80000000u);
+}
+__device__ __noinline__ f3 vertex_force_call(const StepArgs& A, const MeshDev& M, u32 g, f3 pos, f3 vel, float mass) {
+    return vertex_force(A, M, g, pos, vel, mass);
 }
 
 // Warp-aggregated add of v into ctr[0] and the running total ctr[3].
@@ -455,8 +450,9 @@ __device__ __forceinline__ void warp_count(unsigned long long* ctr, u32 v) {
 // the next state's velocities; k_fused applies the contacts to it.  The forces
 // need no tree, so these kernels run beside the refit, and the query's warps
 // neither carry the springs' code nor idle lanes through them.
-__device__ __forceinline__ void put_velocity(const StepArgs& A, u32 g, f3 vel, f3 force, float mass) {
-    vel = vel + ((force * A.subh) / mass) * A.mask[g];
+__device__ __forceinline__ void put_velocity(const StepArgs& A, u32 g, f3 vel, f3 force, float mass,
+                                             float mask) {
+    vel = vel + ((force * A.subh) / mass) * mask;
     A.vn[g] = make_float4(vel.x, vel.y, vel.z, 0.f);
 }
 
@@ -468,30 +464,96 @@ __global__ void __launch_bounds__(128) k_force_vertices(StepArgs A) {
     if (!(M.flags & MF_CLOTH) || ((M.flags & MF_GRID) && M.tmap != NO_PAIR)) return;
     const f3 vel = ld(A.v, g);
     const float mass = A.mass[g];
-    put_velocity(A, g, vel, vertex_force(A, M, g, ld(A.x, g), vel, mass), mass);
+    put_velocity(A, g, vel, vertex_force(A, M, g, ld(A.x, g), vel, mass), mass, A.mask[g]);
 }
 
-// The grid cloths, one 16 x 8 tile per CTA (see "grid-cloth tiles" above).
-__global__ void __launch_bounds__(TILE_W * TILE_H) k_force_tiles(StepArgs A) {
+// The grid cloths' tiles (see "grid-cloth tiles" above), gridDim.x apart per
+// CTA: the next tile's loads are in flight while this one is computed.  Bound
+// by instructions and the springs' dependent chains (0.68 issued a cycle).  A
+// million vertices in 48 cloths (10,339 tiles): 79 us with the springs dealt
+// out family by family and a flag byte each, one tile per CTA; 64 us so.
+__global__ void __launch_bounds__(TILE_W * TILE_H, TILE_CTAS) k_force_tiles(const __grid_constant__ StepArgs A, u32 ntiles) {
     __shared__ float sf[3 * TILE_SPRINGS];
-    __shared__ unsigned long long bar;
-    __shared__ __align__(128) float4 xs[TILE_SMEM / sizeof(float4)];
-    const uint2 t = A.ftiles[blockIdx.x];
-    const MeshDev& M = A.meshes[t.x];
-    const int r0 = (int)(t.y >> 16), c0 = (int)(t.y & 0xFFFFu), N = (int)M.grid_n;
-    if (threadIdx.x == 0) tile_load(xs, A.tmaps + M.tmap + A.xbuf, A.tmaps + M.tmap + 3 + A.vbuf, r0, c0, &bar);
-    __syncthreads();  // the barrier is initialised
-    if (!tile_wait(&bar) && threadIdx.x == 0) atomicOr(A.status, ST_ITER_CAP);
-    unsigned char* flags = reinterpret_cast<unsigned char*>(xs + 2 * HALO_W * HALO_H);
-    tile_springs(A, M, r0, c0, xs, xs + HALO_W * HALO_H, sf, flags);
-    __syncthreads();
-    const int ty = (int)threadIdx.x / TILE_W, tx = (int)threadIdx.x % TILE_W, row = r0 + ty, col = c0 + tx;
-    if (row >= N || col >= N) return;
-    const u32 g = M.voff + (u32)(row * N + col);
-    const float4 v4 = xs[HALO_W * HALO_H + (ty + 2) * HALO_W + tx + 2];
-    const f3 vel = mk(v4.x, v4.y, v4.z);
-    const float mass = A.mass[g];
-    put_velocity(A, g, vel, tile_force(base_force(A, g, vel, mass), N, row, col, ty, tx, sf, flags), mass);
+    __shared__ unsigned long long bars[2];
+    __shared__ __align__(128) float4 tiles[2][2 * HALO_W * HALO_H];
+    __shared__ TileMesh meshes[2];
+    auto load = [&](u32 i, u32 b) {
+        const uint2 t = A.ftiles[i];
+        const MeshDev& M = A.meshes[t.x];
+        if (threadIdx.x >= 32 && threadIdx.x < 38) {
+            const u32 f = threadIdx.x - 32;
+            meshes[b].k[f] = f < 2 ? M.kstretch : (f < 4 ? M.kshear : M.kbend);
+            meshes[b].rest[f] = M.rest[f];
+        }
+        if (threadIdx.x == 0)
+            tile_load(tiles[b], A.tmaps + M.tmap + A.xbuf, A.tmaps + M.tmap + 3 + A.vbuf, (int)(t.y >> 16),
+                      (int)(t.y & 0xFFFFu), bars + b);
+    };
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + 1)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    load(blockIdx.x, 0u);
+    const u32 hw = threadIdx.x < TILE_HALO_N ? TILE_HALO.e[threadIdx.x] : 0u;
+    const int ty = (int)threadIdx.x / TILE_W, tx = (int)threadIdx.x % TILE_W;
+    __syncthreads();  // the barriers are initialised
+    u32 b = 0, phase = 0;
+    for (u32 i = blockIdx.x; i < ntiles; i += gridDim.x) {
+        if (i + gridDim.x < ntiles) load(i + gridDim.x, b ^ 1u);
+        const uint2 t = A.ftiles[i];
+        const MeshDev& M = A.meshes[t.x];
+        const int r0 = (int)(t.y >> 16), c0 = (int)(t.y & 0xFFFFu), row = r0 + ty, col = c0 + tx;
+        const u32 n = M.grid_n, gspr = M.gspr;
+        const bool on = (u32)row < n && (u32)col < n;
+        const u32 g = M.voff + (u32)row * n + (u32)col;
+        const float mass = on ? A.mass[g] : 1.f, mask = on ? A.mask[g] : 0.f;
+        const float4 *xs = tiles[b], *vs = xs + HALO_W * HALO_H;
+        const TileMesh& T = meshes[b];
+        if (!tile_wait(bars + b, phase) && threadIdx.x == 0) atomicOr(A.status, ST_ITER_CAP);
+        const f3 sx = tile_own<0>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        const f3 sy = tile_own<1>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        const f3 ha = tile_own<2>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        const f3 hb = tile_own<3>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        const f3 bx = tile_own<4>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        const f3 by = tile_own<5>(A, T, gspr, n, row, col, ty, tx, xs, vs, sf);
+        if (threadIdx.x < TILE_HALO_N) {
+            const int fam = (int)(hw & 7u), lr = (int)((hw >> 3) & 15u), lc = (int)((hw >> 7) & 31u);
+            const int ar = r0 - 2 + lr, ac = c0 - 2 + lc;
+            f3 F = mk(0.f, 0.f, 0.f);
+            if ((u32)ar < n && (u32)ac < n && (u32)ar + ((hw >> 28) & 3u) < n && (u32)(ac + (int)(hw >> 30) - 1) < n) {
+                float k, rest;
+                tile_spring_kL(A, T, gspr, fam, n, (u32)ar, (u32)ac, k, rest);
+                const int ia = lr * HALO_W + lc;
+                F = tile_spring(xs, vs, ia, ia + (int)((hw >> 22) & 63u), rest, k, A.kd);
+            }
+            const u32 s = (hw >> 12) & 1023u;
+            sf[s] = F.x;
+            sf[TILE_SPRINGS + s] = F.y;
+            sf[2 * TILE_SPRINGS + s] = F.z;
+        }
+        __syncthreads();
+        if (on) {
+            const float4 v4 = vs[(ty + 2) * HALO_W + tx + 2];
+            const f3 vel = mk(v4.x, v4.y, v4.z);
+            f3 force = base_force(A, g, vel, mass);
+            if (has_neg_zero(force)) {
+                const float4 x4 = xs[(ty + 2) * HALO_W + tx + 2];
+                force = vertex_force_call(A, M, g, mk(x4.x, x4.y, x4.z), vel, mass);
+            } else {
+                force = force - tile_into<0>(ty, tx, sf) + sx;
+                force = force - tile_into<1>(ty, tx, sf) + sy;
+                force = force - tile_into<2>(ty, tx, sf) - tile_into<3>(ty, tx, sf) + hb + ha;
+                force = force - tile_into<4>(ty, tx, sf) + bx;
+                force = force - tile_into<5>(ty, tx, sf) + by;
+            }
+            put_velocity(A, g, vel, force, mass, mask);
+        }
+        __syncthreads();  // the table, this tile's buffer and its parameters are read
+        b ^= 1u;
+        phase ^= b ^ 1u;
+    }
 }
 
 // ------------------------------------------------------------------ fused
@@ -1559,7 +1621,7 @@ struct ys_scene {
     std::vector<u32> act_aoff;       // per mesh: first slot in vorder, or NO_PAIR (not working)
     DBuf<CUtensorMap> tmaps;         // 5 per grid cloth: X[0..2], V[0..1]
     DBuf<uint2> ftiles;              // tiles of the grid cloths with maps (StepArgs::ftiles)
-    u32 nftiles = 0;
+    u32 nftiles = 0, tile_ctas = 0;  // and the CTAs that are resident at once
     bool force_vertices = false;     // some cloth has no tiles
     cudaStream_t side = nullptr;     // the force kernels run here, beside the refit
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -2013,6 +2075,10 @@ ys_status encode_tile_maps(ys_scene* s) {
         for (u32 r = 0; r < n; r += TILE_H)
             for (u32 c = 0; c < n; c += TILE_W) tiles.push_back(make_uint2((u32)m, (r << 16) | c));
     }
+    int dev = 0, sms = 0;
+    YS_CK(cudaGetDevice(&dev));
+    YS_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    s->tile_ctas = (u32)(sms * TILE_CTAS);
     s->nftiles = (u32)tiles.size();
     if (!tiles.empty()) {
         YS_CK(s->ftiles.alloc(tiles.size()));
@@ -2050,7 +2116,8 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
 
 // The force kernels of every cloth.
 void launch_forces(ys_scene* s, const StepArgs& A, cudaStream_t st) {
-    if (s->nftiles) k_force_tiles<<<s->nftiles, TILE_W * TILE_H, 0, st>>>(A);
+    if (s->nftiles)
+        k_force_tiles<<<std::min(s->nftiles, s->tile_ctas), TILE_W * TILE_H, 0, st>>>(A, s->nftiles);
     if (s->force_vertices) k_force_vertices<<<ceil_div(s->nV, 128), 128, 0, st>>>(A);
 }
 
