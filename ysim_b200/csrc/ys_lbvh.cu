@@ -1521,6 +1521,7 @@ __global__ void __launch_bounds__(GROUP_THREADS) k_refit_groups(const GroupJob* 
     __shared__ u32 shk[32][6], shb[32][6], sh_ext[GROUP_THREADS / 32];
     const GroupJob& J = jobs[blkJob[blockIdx.x]];
     const u32 b = blockIdx.x - J.block0, w = threadIdx.x >> 5, flags = J.flags, n = J.n;
+    if (blockIdx.x == 0 && threadIdx.x < B.nctr) B.ctr[threadIdx.x] = 0ull;
     if (flags & GJ_VERTS) {
         u32 r[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
 #pragma unroll

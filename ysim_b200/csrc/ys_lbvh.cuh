@@ -273,6 +273,8 @@ struct GroupBufs {
     float4 *l0, *l1, *l2;  // boxes of leaves, runs of 32 and of 1024 (pairs; a tree's first leaf is a multiple of 1024)
     float4* rec;           // 4 per leaf
     u32 *top, *root;       // 8 words per run of 32768 / per mesh
+    unsigned long long* ctr;  // the launch sets the first nctr of these to 0
+    u32 nctr;
 };
 static constexpr u32 GROUP_BLOCK = 1024;    // leaves (or vertices) per block
 static constexpr u32 GROUP_TOP = 32768;

@@ -132,7 +132,10 @@ struct StepArgs {
     u32 xbuf, vbuf;
     const CUtensorMap* tmaps;
     u32* status;
-    unsigned long long* counters;  // [0] broad rows, [1] contacts, [2] pool fill, [3] [4] running totals of 0, 1
+    // [0] broad rows, [1] contacts, [2] pool fill, [3] [4] running totals of 0, 1, [6] blocks done (k_fused)
+    unsigned long long* counters;
+    u32* clear;   // this launch's last block sets the first nclear words to 0 (0: none)
+    u32 nclear;
     // fused record pool
     VContact* pool;
     u32* vstart;
@@ -1098,6 +1101,21 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
             if (Cn) { atomicAdd(&A.counters[1], Cn); atomicAdd(&A.counters[4], Cn); }
         }
     }
+    // What the substep's refit reduced into is zero again for the next one.  A
+    // memset before the refit stood 5 us before the end of the substep's
+    // first kernel (2.5 us to it, 0.7 us, 2 us on to the refit): a 64 x 64
+    // cloth's substep took 20.5 us of which the kernels are 15.
+    if (A.nclear && threadIdx.x < 32) {  // every warp of the block has read its boxes: the counters' barrier
+        u32 last = 0;
+        if (lane == 0) {
+            __threadfence();
+            last = atomicAdd(&A.counters[6], 1ull) == gridDim.x - 1u ? 1u : 0u;
+        }
+        if (__shfl_sync(FULL_MASK, last, 0)) {
+            for (u32 i = lane; i < A.nclear; i += 32u) A.clear[i] = 0u;
+            if (lane == 0) A.counters[6] = 0ull;
+        }
+    }
     if (st) atomicOr(A.status, st);
 }
 
@@ -1535,12 +1553,14 @@ struct ys_scene {
     // sorted-leaf groups of the fused path (cube layout; GroupJob): boxes,
     // records, tops and roots.  gzero holds, in this order, what a substep
     // reduces into (the grid extents, the tops and roots of the meshes refit
-    // every substep, the counters: cleared by one memset), the running totals,
-    // and the tops and roots of the other meshes, written at their build.
+    // every substep), the counters, and the tops and roots of the other meshes,
+    // written at their build.  The former are zero between substeps unless
+    // gdirty: the last block of k_fused clears them.
     DBuf<float4> gl0, gl1, gl2, grec;
     DBuf<u32> gzero;
     DView<u32> maxext, gacc;                    // grid extents; all tops and roots (8 words each)
     size_t gclear = 0;                          // words of gzero before the counters
+    bool gdirty = false;                        // they were written with no k_fused to clear them
     DBuf<GroupJob> gjobs;                       // per mesh build jobs, then the substep's jobs
     DBuf<u32> gblk;                             // job of each block of the substep's refit
     std::vector<GroupJob> hgbuild;              // per mesh: its build job (flags 0: none)
@@ -1606,6 +1626,9 @@ struct ys_scene {
     // refit + fused substep replayed without host launch overhead
     bool use_graphs = true;
     cudaGraphExec_t graphs[18] = {};
+    // and one per rotation state at a frame's start: the frame's substeps
+    cudaGraphExec_t frame_graphs[18] = {};
+    u32 frames_seen[18] = {};        // frames started from each state since the graphs were dropped
     uint64_t graph_epoch = 0;        // counts what made captured substeps stale (drop_graphs)
     int fused_min_blocks = 8;        // k_fused register cap (ys_scene_set_fused_variant / ys_scene_autotune)
     // fused-kernel thread order (ys_scene_set_thread_order): working vertices
@@ -1655,7 +1678,7 @@ ys_status check_scene(ys_scene* s) {
 }
 
 GroupBufs group_bufs(ys_scene* s) {
-    return GroupBufs{s->gl0.p, s->gl1.p, s->gl2.p, s->grec.p, s->gacc.p, s->gacc.p};
+    return GroupBufs{s->gl0.p, s->gl1.p, s->gl2.p, s->grec.p, s->gacc.p, s->gacc.p, nullptr, 0u};
 }
 
 StepArgs make_args(ys_scene* s) {
@@ -1716,6 +1739,8 @@ StepArgs make_args(ys_scene* s) {
     A.cap = s->cap;
     A.status = s->status.p;
     A.counters = s->counters.p;
+    A.clear = s->gzero.p;
+    A.nclear = 0;
     A.pool = s->pool.p; A.vstart = s->vstart.p; A.vcount = s->vcount.p;
     A.rows = s->rows.p; A.contacts = s->contacts.p; A.f = s->Fbuf.p;
     A.bucket = s->bucket.p; A.csr_off = s->csr_off.p; A.csr = s->csr.p;
@@ -1821,6 +1846,11 @@ ys_status build_tree(ys_scene* s, HostMesh& H) {
 }
 
 void drop_graphs(ys_scene* s);
+// After a rebuild: substeps captured in the cube layout read the sorted-leaf
+// groups, whose launches a rebuild leaves as they are.
+void drop_refit_graphs(ys_scene* s) {
+    if (s->tree_layout != YS_TREE_CUBE) drop_graphs(s);
+}
 
 // Upload the 6 job tables (cur x cv) with the level-mode flag of the 4-wide jobs.
 ys_status upload_jobs(ys_scene* s, bool levels) {
@@ -1863,7 +1893,7 @@ ys_status build_levels(ys_scene* s) {
         u32 nbig[2] = {0, 0};
         YS_CK(cudaMemcpyAsync(nbig, s->bigCnt.p, 8, cudaMemcpyDeviceToHost, st));
         YS_CK(cudaStreamSynchronize(st));
-        drop_graphs(s);
+        drop_refit_graphs(s);
         s->nbig = nbig[0];
         s->nhuge = nbig[1];
         s->use_levels = true;
@@ -1874,7 +1904,7 @@ ys_status build_levels(ys_scene* s) {
     std::vector<u32> cnt(MAX_LEVELS + 2);
     YS_CK(cudaMemcpyAsync(cnt.data(), s->hcount.p, 4 * cnt.size(), cudaMemcpyDeviceToHost, st));
     YS_CK(cudaStreamSynchronize(st));
-    drop_graphs(s);
+    drop_refit_graphs(s);
     if (cnt[0] != 0) {  // a tree taller than MAX_LEVELS: climb instead
         s->use_levels = false;
         return upload_jobs(s, false);
@@ -2111,7 +2141,10 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
             if (s->cls_off[e + 1] > s->cls_off[e] && s->cls_variant[e] != s->cls_variant[c]) break;
         A.tbase = s->cls_off[c];
         A.tend = s->cls_off[e];
+        // the last launch: every reader of the refit's reductions is done
+        A.nclear = s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] ? (u32)s->gclear : 0u;
         launch_fused(A, s->stream, s->cls_variant[c]);
+        if (A.nclear) s->gdirty = false;
     }
 }
 
@@ -2160,6 +2193,7 @@ ys_status refit(ys_scene* s) {
         // the job table for the current (position, velocity) buffer pair
         const RefitJob* table = s->jobs.p + (size_t)(s->cur * 2 + s->cv) * s->njobs;
         YS_CK(cudaMemsetAsync(s->maxext.p, 0, s->maxext.n * 4, s->stream));
+        s->gdirty = true;
         launch_refit(table, s->njobs, s->refitLeaves, s->status.p, s->stream);
         if (s->use_levels && s->use_ranges) {
             launch_refit_ranges(table, s->njobs, s->bigEnt.p, (u32)s->bigEnt.n, s->nbig, s->nhuge, s->stream);
@@ -2171,21 +2205,34 @@ ys_status refit(ys_scene* s) {
     return YS_OK;
 }
 
+// The state that the fused substep's refit expects (StepArgs::nclear).
+ys_status clear_groups(ys_scene* s) {
+    if (!s->gdirty) return YS_OK;
+    YS_CK(cudaMemsetAsync(s->gzero.p, 0, 4 * s->gclear, s->stream));
+    s->gdirty = false;
+    return YS_OK;
+}
+
 // What the fused substep reads of the trees at the current positions: the
 // sorted-leaf groups (cube layout; the 4-wide trees then stay as they are
 // until someone asks for them, see refresh_wide) or the binary trees.  Clears
 // the substep's counters as well.
 ys_status refit_fused(ys_scene* s) {
-    const size_t cnt = s->record ? 24 : 16;  // counters [0] [1] ([2]: the record pool); [3] [4] keep running totals
+    const u32 cnt = s->record ? 3 : 2;  // counters [0] [1] ([2]: the record pool); [3] [4] keep running totals
     if (s->tree_layout != YS_TREE_CUBE) {
         ys_status r = refit(s);
         if (r) return r;
-        YS_CK(cudaMemsetAsync(s->counters.p, 0, cnt, s->stream));
+        YS_CK(cudaMemsetAsync(s->counters.p, 0, 8 * cnt, s->stream));
         return YS_OK;
     }
-    YS_CK(cudaMemsetAsync(s->gzero.p, 0, 4 * s->gclear + cnt, s->stream));
-    launch_refit_groups(s->gjobs.p + s->meshes.size(), s->gblk.p, s->ngblocks, s->X[s->cur].p, s->V[s->cv].p,
-                        group_bufs(s), s->stream);
+    ys_status r = clear_groups(s);
+    if (r) return r;
+    GroupBufs B = group_bufs(s);
+    B.ctr = s->counters.p;
+    B.nctr = cnt;
+    if (!s->ngblocks) YS_CK(cudaMemsetAsync(s->counters.p, 0, 8 * cnt, s->stream));
+    launch_refit_groups(s->gjobs.p + s->meshes.size(), s->gblk.p, s->ngblocks, s->X[s->cur].p, s->V[s->cv].p, B, s->stream);
+    s->gdirty = true;
     return YS_OK;
 }
 
@@ -2285,8 +2332,10 @@ ys_status system_update(ys_scene* s) {
 
 void drop_graphs(ys_scene* s) {
     ++s->graph_epoch;
-    for (auto& g : s->graphs)
-        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    for (auto* v : {s->graphs, s->frame_graphs})
+        for (int k = 0; k < 18; ++k)
+            if (v[k]) { cudaGraphExecDestroy(v[k]); v[k] = nullptr; }
+    for (u32& n : s->frames_seen) n = 0;
 }
 
 // Enqueue the device work of one fused substep (no preamble, no rotation).
@@ -2314,28 +2363,59 @@ cudaEvent_t next_event(ys_scene* s) {
     return s->evPool[s->evUsed++];
 }
 
+// The host state that substeps advance.
+struct ys_scene_clock {
+    int cur, prev, cv, stale;
+    bool snapshot;
+    u32 cursor;
+    uint64_t frame, run;
+};
+ys_scene_clock scene_clock(const ys_scene* s) {
+    return {s->cur, s->prev, s->cv, s->refit_stale, s->snapshot_pending, s->cursor, s->frame, s->substeps_run};
+}
+void set_clock(ys_scene* s, const ys_scene_clock& c) {
+    s->cur = c.cur; s->prev = c.prev; s->cv = c.cv; s->refit_stale = c.stale; s->snapshot_pending = c.snapshot;
+    s->cursor = c.cursor; s->frame = c.frame; s->substeps_run = c.run;
+}
+
+// Host state after a fused substep.
+void advance(ys_scene* s) {
+    mark_refit(s);
+    s->snapshot_pending = true;
+    rotate(s);
+}
+
+// Replay `n` substeps as the graph of the current rotation state; captured
+// when there is none.
+ys_status replay(ys_scene* s, cudaGraphExec_t* graphs, u32 n) {
+    ys_status r = clear_groups(s);  // not part of a captured substep
+    if (r) return r;
+    cudaGraphExec_t& exec = graphs[(s->cur * 3 + s->prev) * 2 + s->cv];
+    if (!exec) {
+        const ys_scene_clock before = scene_clock(s);
+        cudaGraph_t g = nullptr;
+        YS_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+        for (u32 i = 0; i < n && !r; ++i)
+            if (!(r = enqueue_fused(s))) advance(s);
+        cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
+        set_clock(s, before);
+        if (r || ce != cudaSuccess) s->gdirty = true;
+        if (r) { if (g) cudaGraphDestroy(g); return r; }
+        if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+        ce = cudaGraphInstantiate(&exec, g, 0);
+        cudaGraphDestroy(g);
+        if (ce != cudaSuccess) { exec = nullptr; return fail(YS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)); }
+    }
+    YS_CK(cudaGraphLaunch(exec, s->stream));
+    for (u32 i = 0; i < n; ++i) advance(s);
+    return YS_OK;
+}
+
 ys_status fused_substep(ys_scene* s) {
     ys_status r = preamble(s);
     if (r) return r;
-    if (s->use_graphs && !s->timing && !s->record) {
-        const int key = (s->cur * 3 + s->prev) * 2 + s->cv;
-        if (!s->graphs[key]) {
-            cudaGraph_t g = nullptr;
-            YS_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-            ys_status er = enqueue_fused(s);
-            cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
-            if (er) { if (g) cudaGraphDestroy(g); return er; }
-            if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-            ce = cudaGraphInstantiate(&s->graphs[key], g, 0);
-            cudaGraphDestroy(g);
-            if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-        }
-        YS_CK(cudaGraphLaunch(s->graphs[key], s->stream));
-        mark_refit(s);
-        s->snapshot_pending = true;
-        rotate(s);
-        return YS_OK;
-    }
+    if (s->use_graphs && !s->timing && !s->record) return replay(s, s->graphs, 1);
+    if ((r = clear_groups(s))) return r;
     if (s->record) {
         r = ensure_record(s);
         if (r) return r;
@@ -2357,10 +2437,27 @@ ys_status fused_substep(ys_scene* s) {
         YS_CK(cudaGetLastError());
         YS_CK(cudaEventRecord(next_event(s), s->stream));
     }
-    mark_refit(s);
-    s->snapshot_pending = true;
-    rotate(s);
+    advance(s);
     if (s->record) s->last_contacts = 2;
+    return YS_OK;
+}
+
+// A whole frame from its start as one graph: with a launch per substep 3 to 4
+// us lay between a 64 x 64 cloth's substeps of 17 us.  The first frames from a
+// rotation state are enqueued kernel by kernel, at about the device's pace: a
+// capture takes 1 ms (10 substeps; 0.1 ms each), what some ten frames save.
+static constexpr u32 FRAME_GRAPH_MAX = 32, FRAME_GRAPH_AFTER = 8;
+ys_status fused_frame(ys_scene* s) {
+    ys_status r = preamble(s);
+    if (r) return r;
+    u32& seen = s->frames_seen[(s->cur * 3 + s->prev) * 2 + s->cv];
+    if (seen == FRAME_GRAPH_AFTER) return replay(s, s->frame_graphs, s->P.substeps);
+    ++seen;
+    if ((r = clear_groups(s))) return r;
+    for (u32 i = 0; i < s->P.substeps; ++i) {
+        if ((r = enqueue_fused(s))) return r;
+        advance(s);
+    }
     return YS_OK;
 }
 
@@ -2977,8 +3074,13 @@ ys_status ys_scene_step_staged(ys_scene* s, uint32_t n) {
 ys_status ys_scene_step(ys_scene* s, uint32_t n) {
     ys_status r = check_scene(s);
     if (r) return r;
-    for (u32 i = 0; i < n; ++i)
-        if ((r = fused_substep(s))) return r;
+    const u32 f = s->P.substeps;
+    const bool frames = s->use_graphs && !s->timing && !s->record && f > 1 && f <= FRAME_GRAPH_MAX;
+    while (n) {
+        const bool frame = frames && s->cursor == 0 && n >= f;
+        if ((r = frame ? fused_frame(s) : fused_substep(s))) return r;
+        n -= frame ? f : 1u;
+    }
     return YS_OK;
 }
 
@@ -3689,11 +3791,14 @@ ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
         G.exec = nullptr;
     }
     const uint64_t run0 = s->substeps_run;
+    const ys_status rc = clear_groups(s);  // not part of the captured pass
+    if (rc) return rc;
     if (!G.exec) {
         cudaGraph_t g = nullptr;
         YS_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         const ys_status er = enqueue();
         cudaError_t ce = cudaStreamEndCapture(st, &g);
+        if (er || ce != cudaSuccess) s->gdirty = true;
         if (er) { if (g) cudaGraphDestroy(g); return er; }
         if (ce != cudaSuccess) return fail(YS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
         ce = cudaGraphInstantiate(&G.exec, g, 0);
@@ -3713,9 +3818,7 @@ ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
 ys_status adj_substep(ys_scene* s) {
     const ys_status r = enqueue_fused(s);
     if (r) return r;
-    mark_refit(s);
-    s->snapshot_pending = true;
-    rotate(s);
+    advance(s);
     if (s->record) s->last_contacts = 2;
     return YS_OK;
 }
