@@ -96,7 +96,9 @@ __global__ void k_sh_order(const ShBox* __restrict__ tris, const u32* __restrict
 // entries (contiguous in the output, the counts being scanned), lane by
 // entry, each lane finding its triangle by a search over the lanes' first
 // entries; cell ordinal o of a triangle is cell (x, y, z) with x fastest.
-// A triangle's loop of 1 to MAX_CELLS cells no longer holds its warp.
+// A triangle's loop of 1 to MAX_CELLS cells no longer holds its warp.  Bound by
+// its instructions: 9.3M entries 75 us with two integer divisions an entry, 57
+// with the reciprocals' products.
 __global__ void k_sh_emit(const ShBox* __restrict__ tris, const u32* __restrict__ off, u32 nF, float inv, u32 mask,
                           u32* __restrict__ ebucket, u32* __restrict__ etri, u32* __restrict__ big,
                           u32* __restrict__ nbig) {
@@ -107,6 +109,9 @@ __global__ void k_sh_emit(const ShBox* __restrict__ tris, const u32* __restrict_
     const u32 tEnd = min(t0 + 32u, nF);
     const u32 start = off[t0], total = off[tEnd] - start;
     int lo[3] = {0, 0, 0}, hi[3] = {-1, -1, -1};
+    // o / n for o < 4096 as floor((o + 0.5) / n): half a step from the next
+    // integer, 2^11 times what the reciprocal and the product can be off
+    float rx = 1.f, ry = 1.f;
     u32 rel = total;  // this lane's first entry, relative to the warp's
     if (t < nF) {
         const u32 base = off[t], end = off[t + 1];
@@ -116,8 +121,11 @@ __global__ void k_sh_emit(const ShBox* __restrict__ tris, const u32* __restrict_
             big[i] = t;
         } else {
             cell_range(tris[t], inv, lo, hi);
+            rx = __frcp_rn((float)(hi[0] - lo[0] + 1));
+            ry = __frcp_rn((float)(hi[1] - lo[1] + 1));
         }
     }
+    const u32 nx0 = (u32)(hi[0] - lo[0] + 1), ny0 = (u32)(hi[1] - lo[1] + 1);
     for (u32 e0 = 0; e0 < total; e0 += 32u) {
         const u32 e = e0 + lane;
         // the last lane whose first entry is <= e (first entries are non-decreasing)
@@ -130,11 +138,11 @@ __global__ void k_sh_emit(const ShBox* __restrict__ tris, const u32* __restrict_
         const u32 rj = __shfl_sync(0xFFFFFFFFu, rel, (int)j);
         const int lx = __shfl_sync(0xFFFFFFFFu, lo[0], (int)j), ly = __shfl_sync(0xFFFFFFFFu, lo[1], (int)j),
                   lz = __shfl_sync(0xFFFFFFFFu, lo[2], (int)j);
-        const int hx = __shfl_sync(0xFFFFFFFFu, hi[0], (int)j), hy = __shfl_sync(0xFFFFFFFFu, hi[1], (int)j);
+        const u32 nx = __shfl_sync(0xFFFFFFFFu, nx0, (int)j), ny = __shfl_sync(0xFFFFFFFFu, ny0, (int)j);
+        const float ix = __shfl_sync(0xFFFFFFFFu, rx, (int)j), iy = __shfl_sync(0xFFFFFFFFu, ry, (int)j);
         if (e < total) {
-            const u32 o = e - rj, nx = (u32)(hx - lx + 1), ny = (u32)(hy - ly + 1);
-            const u32 q = o / nx;
-            ebucket[start + e] = cell_bucket(lx + (int)(o - q * nx), ly + (int)(q % ny), lz + (int)(q / ny), mask);
+            const u32 o = e - rj, q = (u32)(((float)o + 0.5f) * ix), z = (u32)(((float)q + 0.5f) * iy);
+            ebucket[start + e] = cell_bucket(lx + (int)(o - q * nx), ly + (int)(q - z * ny), lz + (int)z, mask);
             etri[start + e] = t0 + j;
         }
     }
@@ -146,14 +154,21 @@ __global__ void k_sh_emit(const ShBox* __restrict__ tris, const u32* __restrict_
 // slots stay below 2^28 - 1 (MAX_ENTRIES).
 static constexpr u32 RUN_LONG = 15;
 static constexpr u32 MAX_ENTRIES = (1u << 28) - 2;
-__global__ void k_sh_mark(const u32* __restrict__ skey, u32 nE, u32* __restrict__ bstart) {
-    const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nE) return;
-    const u32 b = skey[k];
-    if (k != 0 && skey[k - 1] == b) return;
-    u32 c = 1;
-    while (c < RUN_LONG && k + c < nE && skey[k + c] == b) ++c;
-    bstart[b] = (k << 4) | c;
+__global__ void __launch_bounds__(256) k_sh_mark(const u32* __restrict__ skey, u32 nE, u32* __restrict__ bstart) {
+    const u32 k = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const u32 b = k < nE ? skey[k] : 0xFFFFFFFFu;  // a bucket is below 2^31
+    u32 before = __shfl_up_sync(0xFFFFFFFFu, b, 1);
+    if (lane == 0) before = k && k < nE ? skey[k - 1] : 0xFFFFFFFFu;
+    const bool head = k < nE && (k == 0 || before != b);
+    // the run ends at the warp's next key that differs from the one before it;
+    // the warp's last run is followed beyond the warp
+    const unsigned ends = __ballot_sync(0xFFFFFFFFu, lane != 0 && before != b);
+    if (!head) return;
+    const unsigned after = ends & (0xFFFFFFFEu << lane);
+    u32 c = after ? (u32)__ffs(after) - 1u - lane : 32u - lane;
+    if (!after)
+        while (c < RUN_LONG && k + c < nE && skey[k + c] == b) ++c;
+    bstart[b] = (k << 4) | min(c, RUN_LONG);
 }
 
 __device__ __forceinline__ bool box_hit(f3 qmn, f3 qmx, const ShBox& r) {
@@ -324,19 +339,24 @@ ys_status ys_shash_build(ys_shash* h, const float* d_x, const uint32_t* d_facets
     // and scanning a table sized for the capacity cost more than the build
     u32 T = 1;
     while (T < 2u * std::max(nE, 1u) && T < h->tableCap) T <<= 1;
-    h->mask = T - 1;
     int bits = 0;
     while ((1u << bits) < T) ++bits;
+    // a bit that the sort would spend a pass of its own on is not worth it (9.3M
+    // entries, 25 -> 24 bits: a pass of 63 us and 10 us of clearing against 17
+    // us of a query of 1M points)
+    if (bits > 8 && bits % 8 == 1) { T >>= 1; --bits; }
+    h->mask = T - 1;
     YS_CK3(cudaMemsetAsync(h->bstart, 0xFF, 4 * ((size_t)T + 1), s));
     YS_CK3(cudaMemsetAsync(h->nbig, 0, 4, s));
-    k_sh_emit<<<ceil_div(nF, 256), 256, 0, s>>>(h->sbox, h->counts, nF, h->inv, h->mask, h->ebucket, h->etri,
-                                                 h->big, h->nbig);
+    u32 *ekey = h->ebucket, *eval = h->etri;
+    sort_input(ekey, eval, nE, h->sortScratch, 0, bits);
+    k_sh_emit<<<ceil_div(nF, 256), 256, 0, s>>>(h->sbox, h->counts, nF, h->inv, h->mask, ekey, eval, h->big, h->nbig);
     // entries grouped by bucket with a stable radix sort of (bucket,
     // triangle) in place of per-entry atomics on bucket counters (random
     // atomics into a table of up to 2^31 buckets); the triangle rides along
     // as the value, so no gather follows
     if (nE) {
-        YS_CK3(radix_sort_pairs(h->ebucket, h->etri, nE, h->sortScratch, 0, bits, s));
+        YS_CK3(radix_sort_staged(h->ebucket, h->etri, nE, h->sortScratch, 0, bits, s));
         k_sh_mark<<<ceil_div(nE, 256), 256, 0, s>>>(h->ebucket, nE, h->bstart);
     }
     YS_CK3(cudaGetLastError());

@@ -359,28 +359,47 @@ static void sort_passes(u32* keys, u32* vals, u32 n, u32* head, W* look, u32* k2
     }
 }
 
+static int sort_pass_count(int beginBit, int endBit) { return (endBit - beginBit + 7) / 8; }
+
+// Scratch: head (counts, tickets), look-back words (8-byte aligned), the other halves.
+struct SortScratch {
+    u32 *head, *look, *k2, *v2;
+    size_t words;  // of look
+};
+static SortScratch sort_scratch(void* scratch, u32 n, bool large) {
+    SortScratch S;
+    S.head = (u32*)(((uintptr_t)scratch + 7) & ~(uintptr_t)7);
+    S.look = S.head + SORT_HEAD;
+    S.words = (size_t)look_words(sort_tiles(n, large)) * (n >= (1u << 28) ? 2 : 1);
+    S.k2 = S.look + S.words;
+    S.v2 = S.k2 + n;
+    return S;
+}
+
 // Sort keys/vals in place.  scratch must hold sort_scratch_bytes(n) bytes
-// (large: of sort_large tiles only, see the allocation-free sort).
+// (large: of sort_large tiles only, see the allocation-free sort).  staged: the
+// pairs are where sort_input says.
 static cudaError_t sort_in(u32* keys, u32* vals, u32 n, void* scratch, int beginBit, int endBit, bool large,
-                           cudaStream_t s) {
+                           cudaStream_t s, bool staged = false) {
     if (n <= 1 || endBit <= beginBit) return cudaSuccess;
-    const int passes = (endBit - beginBit + 7) / 8;
+    const int passes = sort_pass_count(beginBit, endBit);
     if (n <= SMALL) {
         k_sort_small<<<1, MT, 0, s>>>(keys, vals, n, beginBit, beginBit + 8 * passes);
         return cudaGetLastError();
     }
     const bool wide = n >= (1u << 28);
-    // head (counts, tickets), look-back words (8-byte aligned), the other halves
-    u32* head = (u32*)(((uintptr_t)scratch + 7) & ~(uintptr_t)7);
-    u32* look = head + SORT_HEAD;
-    const size_t words = (size_t)look_words(sort_tiles(n, large)) * (wide ? 2 : 1);
-    u32 *k2 = look + words, *v2 = k2 + n;
-    cudaError_t e = cudaMemsetAsync(head, 0, 4 * (SORT_HEAD + words), s);
+    const SortScratch S = sort_scratch(scratch, n, large);
+    u32 *head = S.head, *look = S.look, *k2 = S.k2, *v2 = S.v2;
+    cudaError_t e = cudaMemsetAsync(head, 0, 4 * (SORT_HEAD + S.words), s);
     if (e != cudaSuccess) return e;
+    if (staged && (passes & 1)) {  // the last pass ends in the caller's arrays
+        std::swap(keys, k2);
+        std::swap(vals, v2);
+    }
     if (wide) sort_passes<LT, LI, u64>(keys, vals, n, head, (u64*)look, k2, v2, beginBit, passes, s);
     else if (large) sort_passes<LT, LI, u32>(keys, vals, n, head, look, k2, v2, beginBit, passes, s);
     else sort_passes<ST, SI, u32>(keys, vals, n, head, look, k2, v2, beginBit, passes, s);
-    if (passes & 1) {
+    if ((passes & 1) && !staged) {
         cudaMemcpyAsync(keys, k2, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(vals, v2, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);
     }
@@ -389,6 +408,17 @@ static cudaError_t sort_in(u32* keys, u32* vals, u32 n, void* scratch, int begin
 
 cudaError_t radix_sort_pairs(u32* keys, u32* vals, u32 n, void* scratch, int beginBit, int endBit, cudaStream_t s) {
     return sort_in(keys, vals, n, scratch, beginBit, endBit, sort_large(n), s);
+}
+
+void sort_input(u32*& keys, u32*& vals, u32 n, void* scratch, int beginBit, int endBit) {
+    if (n <= SMALL || !(sort_pass_count(beginBit, endBit) & 1)) return;
+    const SortScratch S = sort_scratch(scratch, n, sort_large(n));
+    keys = S.k2;
+    vals = S.v2;
+}
+
+cudaError_t radix_sort_staged(u32* keys, u32* vals, u32 n, void* scratch, int beginBit, int endBit, cudaStream_t s) {
+    return sort_in(keys, vals, n, scratch, beginBit, endBit, sort_large(n), s, true);
 }
 
 }  // namespace ys
