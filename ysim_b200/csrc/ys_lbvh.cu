@@ -851,12 +851,17 @@ __global__ void __launch_bounds__(256) k_refit_bin_faces(RefitJob J, const u32* 
 // its range stays in the block.  Leaves whose bit in reach is clear take no
 // part in the unions (midpoint split; nodes inside runs are written by
 // k_refit_bin_runs afterwards).
+//
+// The boxes of every window of 1, 2, 4, 8, 16 and 64 leaves of the block are
+// in shared memory, and a union may take a leaf twice, so two or four windows
+// give any range.  Walking the range (single leaves up to the 16-leaf groups
+// inside it, then groups) held each warp for its longest range: 44 us of a
+// million leaves, 28 so.
+static constexpr u32 WINDOWS = 6;  // of 1, 2, 4, 8, 16, 64 leaves
 __global__ void __launch_bounds__(256) k_refit_bin_leaves(RefitJob J, const uint2* __restrict__ range,
                                                           const float4* __restrict__ lbox,
                                                           const u32* __restrict__ reach) {
-    __shared__ float sh_leaf[6][256];
-    __shared__ float sh_g16[6][16];
-    __shared__ float sh_box[8][6];
+    __shared__ float sh[WINDOWS][6][256];  // box of the window that starts at a leaf (cut at the block's end)
     const u32 n = J.n;
     const u32 i0 = blockIdx.x * 256u, i = i0 + threadIdx.x;
     const bool has = i < n;
@@ -882,55 +887,52 @@ __global__ void __launch_bounds__(256) k_refit_bin_leaves(RefitJob J, const uint
     const bool on = has && (!reach || ((reach[i >> 5] >> (i & 31u)) & 1u));
     float v[6] = {on ? lo.x : inf, on ? lo.y : inf, on ? lo.z : inf,
                   on ? hi.x : -inf, on ? hi.y : -inf, on ? hi.z : -inf};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) sh_leaf[k][threadIdx.x] = v[k];
-    const u32 lane = threadIdx.x & 31u;
-#pragma unroll
-    for (int off = 8; off >= 1; off >>= 1) {
+    auto join = [&](u32 w, u32 at) {
+        at = min(at, 255u);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            v[k] = fminf(v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], off));
-            v[3 + k] = fmaxf(v[3 + k], __shfl_xor_sync(0xFFFFFFFFu, v[3 + k], off));
+            v[k] = fminf(v[k], sh[w][k][at]);
+            v[3 + k] = fmaxf(v[3 + k], sh[w][3 + k][at]);
         }
-    }
-    if ((lane & 15u) == 0) {
-        store_box(J.bb16 + (i >> 4), mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]));
+    };
+    auto put = [&](u32 w) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) sh_g16[k][threadIdx.x >> 4] = v[k];
-    }
+        for (int k = 0; k < 6; ++k) sh[w][k][threadIdx.x] = v[k];
+        __syncthreads();
+    };
+    put(0);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        v[k] = fminf(v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], 16));
-        v[3 + k] = fmaxf(v[3 + k], __shfl_xor_sync(0xFFFFFFFFu, v[3 + k], 16));
+    for (u32 w = 1; w < 5; ++w) {
+        join(w - 1, threadIdx.x + (1u << (w - 1)));
+        put(w);
     }
-    if (lane == 0)
-        for (int k = 0; k < 6; ++k) sh_box[threadIdx.x >> 5][k] = v[k];
-    __syncthreads();
+    if ((threadIdx.x & 15u) == 0) store_box(J.bb16 + (i >> 4), mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]));
+    join(4, threadIdx.x + 16u);
+    join(4, threadIdx.x + 32u);
+    join(4, threadIdx.x + 48u);
+    put(5);
     if (threadIdx.x == 0) {
-        for (u32 w = 1; w < 8; ++w)
-            for (int k = 0; k < 3; ++k) {
-                v[k] = fminf(v[k], sh_box[w][k]);
-                v[3 + k] = fmaxf(v[3 + k], sh_box[w][3 + k]);
-            }
+        join(5, 64u);
+        join(5, 128u);
+        join(5, 192u);
         store_box(J.bb256 + (i0 >> 8), mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]));
     }
     if (i + 1 >= n) return;  // no internal node i
     const uint2 r = range[i];
     if ((r.x >> 8) != (i0 >> 8) || (r.y >> 8) != (i0 >> 8) || r.x > r.y) return;  // a big node
-    float b[6] = {inf, inf, inf, -inf, -inf, -inf};
-    const u32 L = r.x - i0, e = r.y - i0 + 1;
-    u32 s16 = (L + 15u) & ~15u, e16 = e & ~15u;
-    if (s16 >= e16) { s16 = e; e16 = e; }
-    for (u32 l = L; l < s16; ++l)
+    const u32 L = r.x - i0, e = r.y - i0 + 1, len = e - L;
+    // the largest window that fits; four of them where two may not cover
+    const u32 w = len >= 64u ? 5u : min(31u - (u32)__clz((int)len), 4u), size = w == 5u ? 64u : 1u << w;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { b[k] = fminf(b[k], sh_leaf[k][l]); b[3 + k] = fmaxf(b[3 + k], sh_leaf[3 + k][l]); }
-    for (u32 q = s16 >> 4; q < (e16 >> 4); ++q)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { b[k] = fminf(b[k], sh_g16[k][q]); b[3 + k] = fmaxf(b[3 + k], sh_g16[3 + k][q]); }
-    for (u32 l = e16; l < e; ++l)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { b[k] = fminf(b[k], sh_leaf[k][l]); b[3 + k] = fmaxf(b[3 + k], sh_leaf[3 + k][l]); }
-    store_box(&nodes[i], mk(b[0], b[1], b[2]), mk(b[3], b[4], b[5]));
+    for (int k = 0; k < 3; ++k) {
+        v[k] = fminf(sh[w][k][L], sh[w][k][e - size]);
+        v[3 + k] = fmaxf(sh[w][3 + k][L], sh[w][3 + k][e - size]);
+    }
+    if (len > 2u * size) {
+        join(w, L + size);
+        join(w, e - 2u * size);
+    }
+    store_box(&nodes[i], mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]));
 }
 
 // Big nodes (ranges across blocks): 8 lanes per node of big, then a block
