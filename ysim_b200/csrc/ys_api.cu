@@ -224,6 +224,7 @@ ys_status ys_lbvh_build(ys_lbvh* t, const float* x, uint32_t nV, const uint32_t*
         }
         launch_leaf_rank(t->idx, nF, t->rank, t->stream);
     } else {
+        launch_leaf_nodes(t->idx, nF, t->nodes, t->stream);
         YS_CK2(launch_claims(t->nodes, nF, t->claimOff, t->claims, t->karrasScratch, t->stream));
         t->claimed = true;
     }

@@ -183,9 +183,13 @@ __global__ void __launch_bounds__(256) k_karras(const u32* __restrict__ codes, c
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int)n) return;
     KarrasView K{codes, idx, (int)n};
-    Node* L = nodes + (n - 1 + i);
-    L->a = -1;
-    L->b = (i32)idx[i];
+    // with ranges the refit writes whole leaf nodes (launch_leaf_nodes writes
+    // these two words where the tree is climbed after all)
+    if (!R.range) {
+        Node* L = nodes + (n - 1 + i);
+        L->a = -1;
+        L->b = (i32)idx[i];
+    }
     if (i + 1 >= (int)n) return;
     visits[i] = 0;
     int d = (K.delta(i, i + 1) - K.delta(i, i - 1) >= 0) ? 1 : -1;
@@ -259,6 +263,16 @@ __global__ void __launch_bounds__(256) k_karras(const u32* __restrict__ codes, c
             atomicMax(&R.count[3], (u32)(last - first) + 1u);
         }
     }
+}
+
+__global__ void k_leaf_nodes(const u32* __restrict__ idx, u32 n, Node* __restrict__ nodes) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    nodes[n - 1 + i].a = -1;
+    nodes[n - 1 + i].b = (i32)idx[i];
+}
+void launch_leaf_nodes(const u32* idx, u32 n, Node* nodes, cudaStream_t s) {
+    if (n) k_leaf_nodes<<<ceil_div(n, 256), 256, 0, s>>>(idx, n, nodes);
 }
 
 size_t karras_scratch_bytes(u32 n) { return scan_scratch_bytes(n ? 2 * n : 1); }

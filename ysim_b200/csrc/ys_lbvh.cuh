@@ -151,6 +151,8 @@ struct BinRanges {
 };
 void launch_run_reach(const Node* nodes, u32 n, const uint2* range, const u32* codes, const u32* runs, u32 nruns,
                       u32* reach, cudaStream_t s);
+// The child words of the leaves (launch_karras leaves them out with ranges).
+void launch_leaf_nodes(const u32* idx, u32 n, Node* nodes, cudaStream_t s);
 // Claimant lists of a built tree (for the climb).
 cudaError_t launch_claims(const Node* nodes, u32 n, u32* claimOff, i32* claims, void* scratch, cudaStream_t s);
 cudaError_t launch_karras(const u32* codes, const u32* idx, u32 n, Node* nodes, i32* parent, u32* claimOff,
