@@ -13,7 +13,7 @@ sort, Karras), amortised into the timed steps as it comes.
 
 Prints one JSON line (rank 0).  value = substeps/s over all ranks, timed on the
 device with CUDA events on the scene's stream around each substep (one CUDA
-graph launch: refit and fused kernel), the L2 flushed (a 256 MiB write)
+graph launch: refit, forces and fused kernel), the L2 flushed (a 256 MiB write)
 between timed substeps and excluded from the timed intervals; the roofline's
 per-kernel durations come from bursts of further substeps interleaved with
 the timed ones, with events around each kernel.  e2e =
@@ -503,12 +503,12 @@ def run_ours(args, rank, world, local):
     peak, peak_kind = measured_peak()
     ach = ab["fused"] / (fused_ms / 1000.0) / 1e9
     traffic = measured_traffic(args)
-    roof = {"bound": "hbm", "kernel": "k_fused (query+narrow+contacts+forces+integrate)", "achieved": ach,
+    roof = {"bound": "hbm", "kernel": "k_force_vertices + k_fused (forces, query+narrow+contacts+integrate)", "achieved": ach,
             "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": ach / peak,
             "traffic": traffic.get("k_fused"), "algorithmic_bytes": ab["fused"], "avg_launch_ms": fused_ms,
             "refit_kernel": {"achieved": ab["refit"] / (refit_ms / 1000.0) / 1e9, "algorithmic_bytes": ab["refit"],
                              "avg_launch_ms": refit_ms, "traffic": traffic.get("refit"),
-                             "launches_per_substep": "range refit: leaf pass (sorted-leaf order, block boxes) + one pass for the nodes whose range crosses a 256-leaf block and the root"},
+                             "launches_per_substep": "one: the boxes of runs of 32, 1024 and 32768 sorted leaves, face records, grid extent and root box"},
             "traffic_source": traffic.get("source")}
     # The kernel is issue- and latency-bound, not bandwidth-bound: the same
     # launch against the SMs' instruction-issue peak (148 SMs x 4 schedulers x
@@ -547,12 +547,9 @@ def run_ours(args, rank, world, local):
         scene.close()  # room for the 16M-triangle microbenchmark
         run_collide(args, collide.append)
 
-    # launches in the timed loop: per substep the refit's leaf kernel, its
-    # level kernels and its top-level kernel, and k_fused (one CUDA graph);
-    # kt counts the refit as one timed stage, so the level launches are taken
-    # from the kernel list of the recorded substeps: 6 refit launches on C2
-    refit_launches = 6 if spec.meshes[0].behavior == 0 and spec.params.self_mode else 1
-    launches = int(round((kt[1] * refit_launches + kt[3]) / ksteps * args.steps))
+    # launches in the timed loop: per substep the refit, the forces and k_fused
+    # (one CUDA graph); kt counts the forces and k_fused as one timed stage
+    launches = int(round((kt[1] + 2 * kt[3]) / ksteps * args.steps))
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -744,7 +741,8 @@ def measure_batched(args, rank, world, local, steps=100):
         q.set_fused_variant(ch["ctas_per_sm"] if ch else tuned)
         if ch:
             q.set_thread_order(ch["thread_order"])
-        q.step(20)
+        for _ in range(20):
+            q.step(1)
     for q in plain:
         q.sync()
     if world > 1:

@@ -1560,7 +1560,8 @@ struct ys_scene {
     DBuf<u32> gzero;
     DView<u32> maxext, gacc;                    // grid extents; all tops and roots (8 words each)
     size_t gclear = 0;                          // words of gzero before the counters
-    bool gdirty = false;                        // they were written with no k_fused to clear them
+    bool gdirty = false;                        // they were written, and no k_fused has cleared them
+    bool fused_clears = false;                  // whether a substep's k_fused does (what its graphs were captured with)
     DBuf<GroupJob> gjobs;                       // per mesh build jobs, then the substep's jobs
     DBuf<u32> gblk;                             // job of each block of the substep's refit
     std::vector<GroupJob> hgbuild;              // per mesh: its build job (flags 0: none)
@@ -2134,6 +2135,12 @@ ys_status refresh_wide(ys_scene* s);
 // first: the few long warps of a small class then run beside the large
 // class's instead of before them (48 FastGrid instances of 16^2 to 256^2
 // vertices: 27 + 58 + 231 us one after another).
+// Up to this many blocks the fused kernel's last one clears for the next
+// substep; each block's ticket costs it about a microsecond at its end, which
+// above this is more than the memset and its gaps (8,208 blocks, 48 cloths:
+// 213.7 us a substep with tickets, 209.9 with the memset; 2,048 blocks: equal;
+// 512: 18.4 against 20.5).
+static constexpr int CLEAR_BLOCKS = 4096;
 void launch_fused_classes(ys_scene* s, StepArgs A) {
     const size_t n = s->cls_off.size() ? s->cls_off.size() - 1 : 0;
     for (size_t c = 0, e = 0; c < n; c = e) {
@@ -2142,7 +2149,10 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
         A.tbase = s->cls_off[c];
         A.tend = s->cls_off[e];
         // the last launch: every reader of the refit's reductions is done
-        A.nclear = s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] ? (u32)s->gclear : 0u;
+        const u32 vpw = A.wide ? vertices_per_warp(A.tend - A.tbase) : 32u;
+        A.nclear = s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] &&
+                           ceil_div(A.tend - A.tbase, FUSED_WARPS * vpw) <= CLEAR_BLOCKS
+                       ? (u32)s->gclear : 0u;
         launch_fused(A, s->stream, s->cls_variant[c]);
         if (A.nclear) s->gdirty = false;
     }
@@ -2207,7 +2217,7 @@ ys_status refit(ys_scene* s) {
 
 // The state that the fused substep's refit expects (StepArgs::nclear).
 ys_status clear_groups(ys_scene* s) {
-    if (!s->gdirty) return YS_OK;
+    if (!s->gdirty || s->tree_layout != YS_TREE_CUBE) return YS_OK;
     YS_CK(cudaMemsetAsync(s->gzero.p, 0, 4 * s->gclear, s->stream));
     s->gdirty = false;
     return YS_OK;
@@ -2350,6 +2360,7 @@ ys_status enqueue_fused(ys_scene* s) {
     YS_CK(cudaStreamWaitEvent(s->stream, s->join, 0));
     if (r) return r;
     launch_fused_classes(s, A);
+    s->fused_clears = !s->gdirty;
     YS_CK(cudaGetLastError());
     return YS_OK;
 }
@@ -2407,6 +2418,7 @@ ys_status replay(ys_scene* s, cudaGraphExec_t* graphs, u32 n) {
         if (ce != cudaSuccess) { exec = nullptr; return fail(YS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)); }
     }
     YS_CK(cudaGraphLaunch(exec, s->stream));
+    s->gdirty = !s->fused_clears;
     for (u32 i = 0; i < n; ++i) advance(s);
     return YS_OK;
 }
@@ -3808,6 +3820,7 @@ ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
         G.frame = s->frame; G.cursor = s->cursor; G.cur = s->cur; G.prev = s->prev; G.cv = s->cv; G.stale = s->refit_stale;
     }
     YS_CK(cudaGraphLaunch(G.exec, st));
+    s->gdirty = !s->fused_clears;
     s->frame = G.frame; s->cursor = G.cursor; s->cur = G.cur; s->prev = G.prev; s->cv = G.cv; s->refit_stale = G.stale;
     s->snapshot_pending = false;
     s->substeps_run = run0 + substeps;
