@@ -6,11 +6,11 @@
 // with identical results:
 //   staged -- one kernel group per reference stage: swept refit, broad rows,
 //             narrow contacts, per-vertex CSR, forces, integrate;
-//   fused  -- swept refit, then ONE kernel per substep in which the thread of
-//             a vertex traverses the trees, runs the narrow test on every
-//             candidate, keeps its contacts in canonical order in local
-//             memory, gathers its spring forces and integrates.  Broad rows,
-//             contacts and forces never touch HBM.
+//   fused  -- a refit of the sorted-leaf groups, the spring forces beside it,
+//             then one kernel in which a warp traverses the trees for its
+//             vertices, tests the candidates, and each vertex keeps its
+//             contacts in canonical order in local memory and integrates.
+//             Broad rows, contacts and forces never touch HBM.
 // xPrev is not copied: positions live in three rotating buffers (current,
 // previous, next), so SymplecticSystem::snapshotXPrev becomes a pointer
 // rotation.
