@@ -1663,6 +1663,7 @@ struct ys_scene {
     DBuf<VContact> csr, pool;
     DBuf<u32> bucket, csr_off, vstart, vcount;
     bool staged_ready = false, record = false, record_ready = false;
+    bool rows_stored = false;  // counters[0] counts what a detect wrote to rows, not a fused substep's
     int last_contacts = 0;  // 0 none, 1 staged csr, 2 fused pool
     // progress
     uint64_t frame = 0, substeps_run = 0;
@@ -2274,6 +2275,7 @@ ys_status ensure_staged(ys_scene* s) {
     YS_CK(s->csr_off.alloc(s->nV + 1));
     YS_CK(s->Fbuf.alloc(s->nV));
     YS_CK(cudaMemsetAsync(s->Fbuf.p, 0, s->nV * sizeof(float4), s->stream));
+    YS_CK(cudaMemsetAsync(s->csr_off.p, 0, (s->nV + 1) * 4, s->stream));  // an update before any narrow: no contacts
     YS_CK(s->scanScratch.alloc(scan_scratch_bytes(s->nV + 1)));
     s->staged_ready = true;
     return YS_OK;
@@ -2297,6 +2299,7 @@ ys_status detect(ys_scene* s) {
     StepArgs A = make_args(s);
     k_detect_rows<<<ceil_div(s->nV, 128), 128, 0, s->stream>>>(A);
     YS_CK(cudaGetLastError());
+    s->rows_stored = true;
     return YS_OK;
 }
 
@@ -2306,6 +2309,7 @@ ys_status narrow_and_sort(ys_scene* s) {
     unsigned long long cnt[2];
     YS_CK(cudaMemcpyAsync(cnt, s->counters.p, 16, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
+    if (!s->rows_stored) cnt[0] = 0;
     u32 nrows = (u32)std::min<unsigned long long>(cnt[0], s->cap);
     s->last_rows = cnt[0];
     YS_CK(cudaMemsetAsync(s->counters.p + 1, 0, 8, s->stream));
@@ -2392,6 +2396,7 @@ void set_clock(ys_scene* s, const ys_scene_clock& c) {
 // Host state after a fused substep.
 void advance(ys_scene* s) {
     mark_refit(s);
+    s->rows_stored = false;
     s->snapshot_pending = true;
     rotate(s);
 }
@@ -3453,7 +3458,7 @@ ys_status ys_scene_clear_flags(ys_scene* s) {
 ys_status ys_scene_rows(ys_scene* s, void* out, uint64_t cap, uint64_t* n_out) {
     ys_status r = check_scene(s);
     if (r) return r;
-    if (!s->staged_ready) { if (n_out) *n_out = 0; return YS_OK; }
+    if (!s->rows_stored) { if (n_out) *n_out = 0; return YS_OK; }
     unsigned long long cnt;
     YS_CK(cudaMemcpyAsync(&cnt, s->counters.p, 8, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
@@ -3823,6 +3828,7 @@ ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
     s->gdirty = !s->fused_clears;
     s->frame = G.frame; s->cursor = G.cursor; s->cur = G.cur; s->prev = G.prev; s->cv = G.cv; s->refit_stale = G.stale;
     s->snapshot_pending = false;
+    s->rows_stored = false;
     s->substeps_run = run0 + substeps;
     return YS_OK;
 }
