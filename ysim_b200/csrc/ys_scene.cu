@@ -2166,7 +2166,8 @@ void launch_forces(ys_scene* s, const StepArgs& A, cudaStream_t st) {
     if (s->force_vertices) k_force_vertices<<<ceil_div(s->nV, 128), 128, 0, st>>>(A);
 }
 
-ys_status preamble(ys_scene* s) {
+// refits: the caller goes on with a refit.
+ys_status preamble(ys_scene* s, bool refits = true) {
     if (s->cursor != 0) return YS_OK;
     {
         ys_status r = refresh_shapes(s);
@@ -2174,8 +2175,11 @@ ys_status preamble(ys_scene* s) {
     }
     if (s->P.rebuild_frames && s->frame % s->P.rebuild_frames == 0) {
         bool rebuilt = false;
-        ys_status rw = refresh_wide(s);  // trees not rebuilt below keep the last substep's boxes
-        if (rw) return rw;
+        if (!refits) {  // trees not rebuilt below keep the last substep's boxes
+            ys_status r = refresh_wide(s);
+            if (r) return r;
+        }
+        s->refit_stale = -1;
         for (auto& H : s->meshes) {
             if (H.built && H.d.behavior == YS_FLOAT) continue;
             if (!H.needs_tree) continue;  // its root box comes from the root-only refit
@@ -2251,11 +2255,12 @@ void mark_refit(ys_scene* s) {
     if (s->tree_layout == YS_TREE_CUBE) s->refit_stale = s->cur * 2 + s->cv;
 }
 
-// The 4-wide trees as the last fused substep's refit would have left them
-// (that substep's buffers hold its positions and velocities until the next
-// one).  Called by whoever reads the wide trees or overwrites those buffers.
+// The 4-wide trees, root boxes and grid extents as the last fused substep's
+// refit would have left them (that substep's buffers hold its positions and
+// velocities until the next one).  Called by whoever reads them or overwrites
+// those buffers without a refit of its own.
 ys_status refresh_wide(ys_scene* s) {
-    if (s->refit_stale < 0 || s->njobs == 0) return YS_OK;
+    if (s->refit_stale < 0) return YS_OK;
     const int cur = s->cur, cv = s->cv;
     s->cur = s->refit_stale / 2;
     s->cv = s->refit_stale % 2;
@@ -2294,7 +2299,7 @@ ys_status ensure_record(ys_scene* s) {
 
 ys_status detect(ys_scene* s) {
     ys_status r = ensure_staged(s);
-    if (r) return r;
+    if (r || (r = refresh_wide(s))) return r;
     YS_CK(cudaMemsetAsync(s->counters.p, 0, 8, s->stream));
     StepArgs A = make_args(s);
     k_detect_rows<<<ceil_div(s->nV, 128), 128, 0, s->stream>>>(A);
@@ -2305,7 +2310,7 @@ ys_status detect(ys_scene* s) {
 
 ys_status narrow_and_sort(ys_scene* s) {
     ys_status r = ensure_staged(s);
-    if (r) return r;
+    if (r || (r = refresh_wide(s))) return r;  // the analytic markers read root boxes
     unsigned long long cnt[2];
     YS_CK(cudaMemcpyAsync(cnt, s->counters.p, 16, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
@@ -2334,7 +2339,7 @@ ys_status narrow_and_sort(ys_scene* s) {
 
 ys_status system_update(ys_scene* s) {
     ys_status r = ensure_staged(s);
-    if (r) return r;
+    if (r || (r = refresh_wide(s))) return r;  // it overwrites the last substep's velocities
     StepArgs A = make_args(s);
     k_forces<<<ceil_div(s->nV, 128), 128, 0, s->stream>>>(A);
     k_integrate<<<ceil_div(s->nV, 128), 128, 0, s->stream>>>(A);
@@ -3065,7 +3070,7 @@ ys_status ys_scene_pack(ys_scene* s) {
     return YS_OK;
 }
 
-ys_status ys_frame_preamble(ys_scene* s) { ys_status r = check_scene(s); return r ? r : preamble(s); }
+ys_status ys_frame_preamble(ys_scene* s) { ys_status r = check_scene(s); return r ? r : preamble(s, false); }
 ys_status ys_broad_refit(ys_scene* s) { ys_status r = check_scene(s); return r ? r : refit(s); }
 ys_status ys_broad_detect(ys_scene* s) { ys_status r = check_scene(s); return r ? r : detect(s); }
 ys_status ys_narrow_and_sort(ys_scene* s) { ys_status r = check_scene(s); return r ? r : narrow_and_sort(s); }
@@ -3543,6 +3548,7 @@ ys_status ys_scene_tree(ys_scene* s, int mesh, void* nodes, int32_t* parent, uin
     }
     const size_t nn = 2 * (size_t)n - 1;
     if (nodes && s->tree_layout == YS_TREE_CUBE) {
+        if ((r = refresh_wide(s))) return r;  // before the root box below takes the place of its root box
         // the cube layout refits the wide form only; give the binary form the
         // boxes of a refit from the current state (swept for moving meshes)
         RefitJob J;
@@ -3768,8 +3774,9 @@ struct ys_adjoint {
 
 namespace {
 
+// A substep follows, whose refit takes the place of the one left undone.
 void restore_state(ys_scene* s, const float4* x, const float4* xp, const float4* v, uint64_t frame, u32 cursor) {
-    refresh_wide(s);
+    s->refit_stale = -1;
     const size_t bytes = sizeof(float4) * s->nV;
     cudaMemcpyAsync(s->X[s->cur].p, x, bytes, cudaMemcpyDeviceToDevice, s->stream);
     cudaMemcpyAsync(s->X[s->prev].p, xp, bytes, cudaMemcpyDeviceToDevice, s->stream);
@@ -4338,12 +4345,11 @@ ys_status ys_adjoint_forward(ys_adjoint* a, float* d_xT) {
         YS_CK(cudaGetLastError());
         return YS_OK;
     }
-    ys_status r = refresh_wide(s);
-    if (r) return r;
     s->cur = 0; s->prev = 1; s->cv = 0;
     restore_state(s, a->x0.p, a->x0.p, a->v0.p, 0, 0);
     const bool rec = s->record;
     s->record = false;
+    ys_status r = YS_OK;
     auto pass = [&](auto&& substep) -> ys_status {
         for (u32 t = 0; t < a->T; ++t) {
             if (t % a->K == 0) {
@@ -4398,10 +4404,9 @@ ys_status ys_adjoint_backward(ys_adjoint* a, const float* d_dLdx, float* d_gk, f
     float *gk = whole ? a->gk.p : d_gk, *gL = whole ? a->gL.p : d_gL;
     YS_CK(cudaMemsetAsync(a->ax.p, 0, bytes, st));
     k_mesh_pack4<<<ceil_div(a->nV, 256), 256, 0, st>>>(d_dLdx, a->ax.p, a->voff, a->nV);
-    ys_status r = refresh_wide(s);
-    if (r) return r;
     const bool rec = s->record;
-    if ((r = ensure_record(s))) return r;
+    ys_status r = ensure_record(s);
+    if (r) return r;
     VContact* keep_pool = s->pool.p;
     u32 *keep_vs = s->vstart.p, *keep_vc = s->vcount.p;
     s->cur = 0; s->prev = 1; s->cv = 0;
