@@ -58,6 +58,9 @@ __device__ __forceinline__ dd3 ldf(const float4* p, u32 i) {
 struct __align__(32) DContact { double nx, ny, nz, d; };
 
 static constexpr u32 D64_CAP = 16;    // contacts kept per vertex and step
+// Bound on one warp's search in one obstacle, per vertex: candidates tested
+// and runs of 32 leaves opened; past it the search stops and the rollout fails.
+static constexpr u32 D64_STEPS = 1u << 24;
 // Block size of the per-vertex kernels (32 measured the same on the
 // 128x128 rollout: the step kernel is bound by its divergent descents).
 static constexpr u32 D64_BLOCK = 128;
@@ -314,6 +317,7 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_cand(A64 A) {
             shi.z < (double)rl[2] || slo.z > (double)rh[2])
             continue;
         const u32 n = T.nF, n1 = (n + 31u) / 32u, n2 = (n + 1023u) / 1024u;
+        u32 steps = 0;
         const float4* __restrict__ L0 = A.grp.l0 + 2 * (size_t)T.boxL0;
         const float4* __restrict__ L1 = A.grp.l1 + 2 * (size_t)(T.boxL0 / 32u);
         const float4* __restrict__ L2 = A.grp.l2 + 2 * (size_t)(T.boxL0 / 1024u);
@@ -351,9 +355,15 @@ __global__ void __launch_bounds__(D64_BLOCK) k_d64_cand(A64 A) {
                         qn += (u32)__popc(hm);
                         if (qn >= 32u) {
                             qn -= 32u;
+                            steps += 32u;
                             drain(qn, 32);
                         }
                     } while (vm);
+                }
+                if ((steps += 32u) > D64_STEPS * A.vpw) {  // at most 2^29
+                    st |= YS_FLAG_STACK_OVF;
+                    m2 = 0;
+                    q2 = n2;
                 }
             }
         }

@@ -12,6 +12,10 @@ static constexpr int STACK_DEPTH = 64;          // queryAABB stack (bvh.metal:13
 // descent that reaches 2^16 is reported (YS_FLAG_STACK_OVF) and stopped so a
 // degenerate tree cannot keep a kernel busy for minutes.
 static constexpr u32 VISIT_CAP = 1u << 16;
+// The same bound for a warp's descent of the sorted-leaf groups of one tree,
+// per vertex of the warp: candidates found (VISIT_CAP wide nodes hold up to
+// three leaves each) and runs of 32 leaves opened.
+static constexpr u32 GROUP_STEPS = 4 * VISIT_CAP;
 
 // intersectAABB (bvh.metal:1285-1290): inclusive box overlap.
 __device__ __forceinline__ bool overlap(f3 qmn, f3 qmx, float4 n0, float4 n1) {

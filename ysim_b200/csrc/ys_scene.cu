@@ -844,6 +844,7 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
                 Q.vhi[lane] = make_float4(bhi.x, bhi.y, bhi.z, 0.f);
                 __syncwarp();
                 const LaneBox LB = lane_box(blo, bhi);
+                u32 steps = 0;  // candidates tested and runs of 32 opened, 32 at a time (GROUP_STEPS)
                 f3 alo, ahi;  // the union of all, of those that meet a run of 32768, of 1024
                 lane_union(LB, in, alo, ahi);
                 const unsigned inm = __ballot_sync(FULL_MASK, in);
@@ -915,9 +916,15 @@ __global__ void __launch_bounds__(128, MINB) k_fused(StepArgs A) {
                                     qn += (u32)__popc(hm);
                                     if (qn >= 32u) {
                                         qn -= 32u;
+                                        steps += 32u;
                                         drain(qn, 32);
                                     }
                                 }
+                            }
+                            if ((steps += 32u) > GROUP_STEPS * A.vpw) {  // nothing more of this tree
+                                st |= ST_STACK_OVF;
+                                m2 = m3 = 0;
+                                q3 = n3;
                             }
                         }
                     }
@@ -3986,6 +3993,7 @@ ys_status d64_status(ys_adjoint* a) {
     YS_CK(cudaMemcpyAsync(&f, a->dstatus.p, 4, cudaMemcpyDeviceToHost, a->s->stream));
     YS_CK(cudaStreamSynchronize(a->s->stream));
     if (f & YS_FLAG_CONTACT_OVF) return fail(YS_ERR_CAPACITY, "FP64 rollout: more than 16 contacts at a vertex");
+    if (f & YS_FLAG_STACK_OVF) return fail(YS_ERR_CAPACITY, "FP64 rollout: contact search past its bound");
     return YS_OK;
 }
 
