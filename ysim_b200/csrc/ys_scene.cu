@@ -17,6 +17,7 @@
 #include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (the entry point comes from the runtime)
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <string>
 #include <type_traits>
@@ -1158,10 +1159,12 @@ void launch_fused_t(const StepArgs& A, int g, cudaStream_t st, int minBlocks) {
 u32 vertices_per_warp(u32 n) {
     return n <= 9472u ? 2u : n <= 18944u ? 4u : n <= 75776u ? 8u : n <= 151552u ? 16u : 32u;
 }
+// A.vpw on entry: what the other scenes' load asks for (note_load).
+u32 launch_vpw(const StepArgs& A) { return A.wide ? std::max(A.vpw, vertices_per_warp(A.tend - A.tbase)) : 32u; }
 
 void launch_fused(StepArgs A, cudaStream_t st, int minBlocks) {
     if (A.tend <= A.tbase) return;
-    A.vpw = A.wide ? vertices_per_warp(A.tend - A.tbase) : 32u;
+    A.vpw = launch_vpw(A);
     const int g = ceil_div(A.tend - A.tbase, FUSED_WARPS * A.vpw);
     if (A.analytic) launch_fused_t<true>(A, g, st, minBlocks);
     else launch_fused_t<false>(A, g, st, minBlocks);
@@ -1659,6 +1662,10 @@ struct ys_scene {
     cudaEvent_t fork = nullptr, join = nullptr;
     std::vector<int> mesh_class;     // per mesh, or -1 (not working)
     DBuf<char> oscratch;
+    // this scene's share of its device's load (note_load)
+    uint64_t load_seen = 0;          // Load::stepped after this scene's last step call
+    u32 load_pending = 0;            // vertices counted in Load::pending
+    u32 load_vpw = 0, load_votes = 0;  // vertices per warp for that load (0: alone); calls in a row that want another
     int tree_layout = YS_TREE_CUBE;  // Morton normalisation of the scene trees
     int tree_builder = YS_BUILD_KARRAS;
     DBuf<char> aggScratch;           // Apetrei range ends and root slot
@@ -1741,6 +1748,7 @@ StepArgs make_args(ys_scene* s) {
     A.vbuf = (u32)s->cv;
     A.tbase = 0;
     A.tend = s->nact;
+    A.vpw = s->load_vpw;
     A.grp = group_bufs(s);
     A.lvid = s->lvid.p;
     A.self_mode = s->P.self_mode;
@@ -2157,9 +2165,8 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
         A.tbase = s->cls_off[c];
         A.tend = s->cls_off[e];
         // the last launch: every reader of the refit's reductions is done
-        const u32 vpw = A.wide ? vertices_per_warp(A.tend - A.tbase) : 32u;
         A.nclear = s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] &&
-                           ceil_div(A.tend - A.tbase, FUSED_WARPS * vpw) <= CLEAR_BLOCKS
+                           ceil_div(A.tend - A.tbase, FUSED_WARPS * launch_vpw(A)) <= CLEAR_BLOCKS
                        ? (u32)s->gclear : 0u;
         launch_fused(A, s->stream, s->cls_variant[c]);
         if (A.nclear) s->gdirty = false;
@@ -2367,13 +2374,18 @@ void drop_graphs(ys_scene* s) {
 // Enqueue the device work of one fused substep (no preamble, no rotation).
 ys_status enqueue_fused(ys_scene* s) {
     const StepArgs A = make_args(s);
-    // the forces beside the refit, on the scene's second stream
-    YS_CK(cudaEventRecord(s->fork, s->stream));
-    YS_CK(cudaStreamWaitEvent(s->side, s->fork, 0));
-    launch_forces(s, A, s->side);
-    YS_CK(cudaEventRecord(s->join, s->side));
+    // the forces beside the refit, on the scene's second stream; in turn
+    // where other scenes fill the gaps (a graph with branches takes the host
+    // twice as long to launch)
+    const bool fork = !s->load_vpw;
+    if (fork) {
+        YS_CK(cudaEventRecord(s->fork, s->stream));
+        YS_CK(cudaStreamWaitEvent(s->side, s->fork, 0));
+    }
+    launch_forces(s, A, fork ? s->side : s->stream);
+    if (fork) YS_CK(cudaEventRecord(s->join, s->side));
     ys_status r = refit_fused(s);
-    YS_CK(cudaStreamWaitEvent(s->stream, s->join, 0));
+    if (fork) YS_CK(cudaStreamWaitEvent(s->stream, s->join, 0));
     if (r) return r;
     launch_fused_classes(s, A);
     s->fused_clears = !s->gdirty;
@@ -2403,6 +2415,51 @@ ys_scene_clock scene_clock(const ys_scene* s) {
 void set_clock(ys_scene* s, const ys_scene_clock& c) {
     s->cur = c.cur; s->prev = c.prev; s->cv = c.cv; s->refit_stale = c.stale; s->snapshot_pending = c.snapshot;
     s->cursor = c.cursor; s->frame = c.frame; s->substeps_run = c.run;
+}
+
+// Step calls on a device, for vertices_per_warp, which takes a chip that is
+// idle but for this launch: 256 grid cloths stepped in turn on their own
+// streams take 1.72 ms a round at their own sizes' vertices per warp and 0.83
+// at their sum's.  stepped: working vertices of every step call so far;
+// pending: those of the scenes that have stepped and not synchronised since.
+// The states do not depend on it.
+struct Load {
+    std::atomic<uint64_t> stepped{0};
+    std::atomic<int64_t> pending{0};
+};
+static constexpr int LOAD_DEVICES = 64;
+static constexpr u32 LOAD_VOTES = 4;  // captured substeps hold the vertices per warp: not for every call
+Load g_load[LOAD_DEVICES];
+
+// A step call: what runs beside it is what other scenes have enqueued since
+// this one's last call and not waited for.
+void note_load(ys_scene* s) {
+    if (s->device < 0 || s->device >= LOAD_DEVICES || s->tree_layout != YS_TREE_CUBE) return;
+    Load& L = g_load[s->device];
+    const uint64_t before = L.stepped.fetch_add(s->nact, std::memory_order_relaxed);
+    const uint64_t calls = before - s->load_seen;
+    s->load_seen = before + s->nact;
+    if (!s->load_pending) {
+        s->load_pending = s->nact;
+        L.pending.fetch_add(s->nact, std::memory_order_relaxed);
+    }
+    const int64_t pending = L.pending.load(std::memory_order_relaxed) - (int64_t)s->load_pending;
+    const uint64_t others = std::min(calls, (uint64_t)std::max<int64_t>(pending, 0));
+    const u32 vpw = vertices_per_warp((u32)std::min<uint64_t>(s->nact + others, 0xFFFFFFFFu));
+    const u32 want = vpw > vertices_per_warp(s->nact) ? vpw : 0u;
+    if (want == s->load_vpw) s->load_votes = 0;
+    else if (++s->load_votes >= LOAD_VOTES) {
+        s->load_vpw = want;
+        s->load_votes = 0;
+        drop_graphs(s);
+    }
+}
+
+// The scene's stream has been waited for.
+void settle_load(ys_scene* s) {
+    if (!s->load_pending) return;
+    g_load[s->device].pending.fetch_sub(s->load_pending, std::memory_order_relaxed);
+    s->load_pending = 0;
 }
 
 // Host state after a fused substep.
@@ -2632,6 +2689,7 @@ ys_status ys_scene_destroy(ys_scene* s) {
     if (!s) return YS_OK;
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
+    settle_load(s);
     for (auto& b : s->X) b.free();
     for (auto& b : s->V) b.free();
     s->Fbuf.free(); s->mass.free(); s->mask.free(); s->vobj.free(); s->targets.free(); s->spr_off.free();
@@ -3103,8 +3161,11 @@ ys_status ys_scene_step_staged(ys_scene* s, uint32_t n) {
 ys_status ys_scene_step(ys_scene* s, uint32_t n) {
     ys_status r = check_scene(s);
     if (r) return r;
+    if (n) note_load(s);
     const u32 f = s->P.substeps;
-    const bool frames = s->use_graphs && !s->timing && !s->record && f > 1 && f <= FRAME_GRAPH_MAX;
+    // beside other scenes a frame's gaps are filled, and capturing it or
+    // enqueueing its kernels one by one is host time they wait for
+    const bool frames = s->use_graphs && !s->timing && !s->record && f > 1 && f <= FRAME_GRAPH_MAX && !s->load_vpw;
     while (n) {
         const bool frame = frames && s->cursor == 0 && n >= f;
         if ((r = frame ? fused_frame(s) : fused_substep(s))) return r;
@@ -3326,6 +3387,7 @@ ys_status ys_scene_set_graphs(ys_scene* s, int on) {
 ys_status ys_scene_sync(ys_scene* s) {
     if (!s) return fail(YS_ERR_BAD_ARG, "null scene");
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     return YS_OK;
 }
 
@@ -3351,6 +3413,7 @@ ys_status ys_scene_get_state(ys_scene* s, int which, float* out) {
     k_unpack4<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(src, s->scratch3.p, s->nV);
     YS_CK(cudaMemcpyAsync(out, s->scratch3.p, 12 * (size_t)s->nV, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     return YS_OK;
 }
 
@@ -3376,6 +3439,7 @@ ys_status ys_scene_set_state(ys_scene* s, int which, const float* in) {
     k_pack4_static<<<ceil_div(s->nV, 256), 256, 0, s->stream>>>(s->scratch3.p, dst, o1, o2, s->vobj.p, s->dmeshes.p, s->nV);
     YS_CK(cudaGetLastError());
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     return YS_OK;
 }
 
@@ -3387,6 +3451,7 @@ ys_status ys_scene_stats(ys_scene* s, uint64_t out[8]) {
     YS_CK(cudaMemcpyAsync(cnt, s->counters.p, 24, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaMemcpyAsync(&st, s->status.p, 4, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     out[0] = s->frame;
     out[1] = s->cursor;
     out[2] = cnt[0];
@@ -3455,6 +3520,7 @@ ys_status ys_scene_totals(ys_scene* s, uint64_t out[2]) {
     unsigned long long c[2];
     YS_CK(cudaMemcpyAsync(c, s->counters.p + 3, 16, cudaMemcpyDeviceToHost, s->stream));
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     out[0] = c[0]; out[1] = c[1];
     return YS_OK;
 }
@@ -3484,6 +3550,7 @@ ys_status ys_scene_contacts(ys_scene* s, uint32_t* off, void* out, uint64_t cap,
     ys_status r = check_scene(s);
     if (r) return r;
     YS_CK(cudaStreamSynchronize(s->stream));
+    settle_load(s);
     if (s->last_contacts == 1) {
         std::vector<u32> o(s->nV + 1);
         YS_CK(cudaMemcpy(o.data(), s->csr_off.p, 4 * (size_t)(s->nV + 1), cudaMemcpyDeviceToHost));
