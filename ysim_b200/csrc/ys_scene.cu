@@ -26,6 +26,7 @@
 #include "ys_analytic.cuh"
 #include "ys_collide.cuh"
 #include "ys_common.cuh"
+#include "ys_groups.cuh"
 #include "ys_lbvh.cuh"
 #include "ys_scan.cuh"
 #include "ys_sort.cuh"
@@ -306,6 +307,7 @@ __device__ __forceinline__ f3 vertex_force(const StepArgs& A, const MeshDev& M, 
 static constexpr int TILE_W = 16, TILE_H = 8;
 static constexpr int HALO_W = TILE_W + 4, HALO_H = TILE_H + 4;  // the stencil reaches 2 vertices out
 static constexpr int TILE_CTAS = 8;  // resident per SM
+static constexpr u32 REFIT_FORCE_CTAS = 2;  // of k_refit_forces
 static constexpr u32 TILE_BOX_BYTES = HALO_W * HALO_H * 16;      // one float4 buffer's tile
 // the tile's table: first spring, row length, first row and column of each
 // family, and the step from a to b
@@ -460,9 +462,8 @@ __device__ __forceinline__ void put_velocity(const StepArgs& A, u32 g, f3 vel, f
     A.vn[g] = make_float4(vel.x, vel.y, vel.z, 0.f);
 }
 
-// Every cloth vertex that no tile covers, one thread each, in vertex order.
-__global__ void __launch_bounds__(128) k_force_vertices(StepArgs A) {
-    const u32 g = blockIdx.x * blockDim.x + threadIdx.x;
+// A cloth vertex that no tile covers.
+__device__ __forceinline__ void force_vertex(const StepArgs& A, u32 g) {
     if (g >= A.nV) return;
     const MeshDev& M = A.meshes[A.vobj[g]];
     if (!(M.flags & MF_CLOTH) || ((M.flags & MF_GRID) && M.tmap != NO_PAIR)) return;
@@ -471,13 +472,15 @@ __global__ void __launch_bounds__(128) k_force_vertices(StepArgs A) {
     put_velocity(A, g, vel, vertex_force(A, M, g, ld(A.x, g), vel, mass), mass, A.mask[g]);
 }
 
-// The grid cloths' tiles (see "grid-cloth tiles" above), gridDim.x apart per
-// CTA: the next tile's loads are in flight while this one is computed.  Bound
-// by instructions and the springs' dependent chains (0.68 issued a cycle).  A
-// million vertices in 48 cloths (10,339 tiles): 79 us with the springs dealt
-// out family by family and a flag byte each, one tile per CTA; 64 us so; 56 us
-// with the branch-free unit vector.
-__global__ void __launch_bounds__(TILE_W * TILE_H, TILE_CTAS) k_force_tiles(const __grid_constant__ StepArgs A, u32 ntiles) {
+// Every cloth vertex that no tile covers, one thread each, in vertex order.
+__global__ void __launch_bounds__(128) k_force_vertices(StepArgs A) {
+    force_vertex(A, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Tiles first, first + step, ... of the grid cloths (see "grid-cloth tiles"
+// above) by TILE_W * TILE_H threads: the next tile's loads are in flight while
+// this one is computed.
+__device__ __forceinline__ void force_tiles(const StepArgs& A, u32 first, u32 step, u32 ntiles) {
     __shared__ float sf[3 * TILE_SPRINGS];
     __shared__ unsigned long long bars[2];
     __shared__ __align__(128) float4 tiles[2][2 * HALO_W * HALO_H];
@@ -500,13 +503,13 @@ __global__ void __launch_bounds__(TILE_W * TILE_H, TILE_CTAS) k_force_tiles(cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    load(blockIdx.x, 0u);
+    load(first, 0u);
     const u32 hw = threadIdx.x < TILE_HALO_N ? TILE_HALO.e[threadIdx.x] : 0u;
     const int ty = (int)threadIdx.x / TILE_W, tx = (int)threadIdx.x % TILE_W;
     __syncthreads();  // the barriers are initialised
     u32 b = 0, phase = 0;
-    for (u32 i = blockIdx.x; i < ntiles; i += gridDim.x) {
-        if (i + gridDim.x < ntiles) load(i + gridDim.x, b ^ 1u);
+    for (u32 i = first; i < ntiles; i += step) {
+        if (i + step < ntiles) load(i + step, b ^ 1u);
         const uint2 t = A.ftiles[i];
         const MeshDev& M = A.meshes[t.x];
         const int r0 = (int)(t.y >> 16), c0 = (int)(t.y & 0xFFFFu), row = r0 + ty, col = c0 + tx;
@@ -558,6 +561,34 @@ __global__ void __launch_bounds__(TILE_W * TILE_H, TILE_CTAS) k_force_tiles(cons
         __syncthreads();  // the table, this tile's buffer and its parameters are read
         b ^= 1u;
         phase ^= b ^ 1u;
+    }
+}
+
+// The grid cloths' tiles, gridDim.x apart per CTA.  Bound
+// by instructions and the springs' dependent chains (0.68 issued a cycle).  A
+// million vertices in 48 cloths (10,339 tiles): 79 us with the springs dealt
+// out family by family and a flag byte each, one tile per CTA; 64 us so; 56 us
+// with the branch-free unit vector.
+__global__ void __launch_bounds__(TILE_W * TILE_H, TILE_CTAS) k_force_tiles(const __grid_constant__ StepArgs A, u32 ntiles) {
+    force_tiles(A, blockIdx.x, gridDim.x, ntiles);
+}
+
+// Small scenes: the groups' refit in the first blocks, a tile of a grid cloth
+// in each of the next, the other cloth vertices in the last (128 of a block's
+// threads: a scheduler's warps would only wait for one another).  One node of a
+// graph without branches, where the refit and the forces beside it are two and
+// a fork: a rollout of 100 steps is captured in 5 ms instead of 15, and a
+// substep saves 0.2 (64 x 64 grid cloth) to 2 us (97 x 97 triangle cloth).
+__global__ void __launch_bounds__(GROUP_THREADS) k_refit_forces(const GroupJob* __restrict__ jobs,
+                                                                const u32* __restrict__ blkJob, u32 refitBlocks,
+                                                                GroupBufs B, const __grid_constant__ StepArgs A,
+                                                                u32 ntiles) {
+    if (blockIdx.x < refitBlocks) {
+        refit_groups_block(jobs, blkJob, A.x, A.v, B);
+    } else if (threadIdx.x < TILE_W * TILE_H) {
+        const u32 t = blockIdx.x - refitBlocks;
+        if (t < ntiles) force_tiles(A, t, ntiles, ntiles);
+        else force_vertex(A, (t - ntiles) * (TILE_W * TILE_H) + threadIdx.x);
     }
 }
 
@@ -1656,7 +1687,7 @@ struct ys_scene {
     std::vector<u32> act_aoff;       // per mesh: first slot in vorder, or NO_PAIR (not working)
     DBuf<CUtensorMap> tmaps;         // 5 per grid cloth: X[0..2], V[0..1]
     DBuf<uint2> ftiles;              // tiles of the grid cloths with maps (StepArgs::ftiles)
-    u32 nftiles = 0, tile_ctas = 0;  // and the CTAs that are resident at once
+    u32 nftiles = 0, sms = 0;        // the tiles; SMs of the device
     bool force_vertices = false;     // some cloth has no tiles
     cudaStream_t side = nullptr;     // the force kernels run here, beside the refit
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -2126,7 +2157,7 @@ ys_status encode_tile_maps(ys_scene* s) {
     int dev = 0, sms = 0;
     YS_CK(cudaGetDevice(&dev));
     YS_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    s->tile_ctas = (u32)(sms * TILE_CTAS);
+    s->sms = (u32)sms;
     s->nftiles = (u32)tiles.size();
     if (!tiles.empty()) {
         YS_CK(s->ftiles.alloc(tiles.size()));
@@ -2176,7 +2207,7 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
 // The force kernels of every cloth.
 void launch_forces(ys_scene* s, const StepArgs& A, cudaStream_t st) {
     if (s->nftiles)
-        k_force_tiles<<<std::min(s->nftiles, s->tile_ctas), TILE_W * TILE_H, 0, st>>>(A, s->nftiles);
+        k_force_tiles<<<std::min(s->nftiles, s->sms * TILE_CTAS), TILE_W * TILE_H, 0, st>>>(A, s->nftiles);
     if (s->force_vertices) k_force_vertices<<<ceil_div(s->nV, 128), 128, 0, st>>>(A);
 }
 
@@ -2242,27 +2273,43 @@ ys_status clear_groups(ys_scene* s) {
     return YS_OK;
 }
 
+// The groups as a substep's refit takes them: it sets the counters of the
+// substep to 0, [0] [1] ([2]: the record pool); [3] [4] keep running totals.
+GroupBufs substep_groups(ys_scene* s) {
+    GroupBufs B = group_bufs(s);
+    B.ctr = s->counters.p;
+    B.nctr = s->record ? 3u : 2u;
+    return B;
+}
+
 // What the fused substep reads of the trees at the current positions: the
 // sorted-leaf groups (cube layout; the 4-wide trees then stay as they are
 // until someone asks for them, see refresh_wide) or the binary trees.  Clears
 // the substep's counters as well.
 ys_status refit_fused(ys_scene* s) {
-    const u32 cnt = s->record ? 3 : 2;  // counters [0] [1] ([2]: the record pool); [3] [4] keep running totals
+    const GroupBufs B = substep_groups(s);
     if (s->tree_layout != YS_TREE_CUBE) {
         ys_status r = refit(s);
         if (r) return r;
-        YS_CK(cudaMemsetAsync(s->counters.p, 0, 8 * cnt, s->stream));
+        YS_CK(cudaMemsetAsync(B.ctr, 0, 8 * B.nctr, s->stream));
         return YS_OK;
     }
     ys_status r = clear_groups(s);
     if (r) return r;
-    GroupBufs B = group_bufs(s);
-    B.ctr = s->counters.p;
-    B.nctr = cnt;
-    if (!s->ngblocks) YS_CK(cudaMemsetAsync(s->counters.p, 0, 8 * cnt, s->stream));
+    if (!s->ngblocks) YS_CK(cudaMemsetAsync(B.ctr, 0, 8 * B.nctr, s->stream));
     launch_refit_groups(s->gjobs.p + s->meshes.size(), s->gblk.p, s->ngblocks, s->X[s->cur].p, s->V[s->cv].p, B, s->stream);
     s->gdirty = true;
     return YS_OK;
+}
+
+// Blocks of k_refit_forces, or 0 where the refit and the forces are kernels of
+// their own: more than are resident at once (65,000 cloth vertices: 25.4 us a
+// substep apart, 28.4 in one), beside other scenes (its blocks use a quarter
+// of their threads for the forces), or with nothing to refit.
+u32 refit_force_blocks(const ys_scene* s) {
+    if (s->tree_layout != YS_TREE_CUBE || !s->ngblocks || s->load_vpw) return 0;
+    const u32 n = s->ngblocks + s->nftiles + (s->force_vertices ? (u32)ceil_div(s->nV, TILE_W * TILE_H) : 0u);
+    return n <= REFIT_FORCE_CTAS * s->sms ? n : 0u;
 }
 
 void mark_refit(ys_scene* s) {
@@ -2374,6 +2421,17 @@ void drop_graphs(ys_scene* s) {
 // Enqueue the device work of one fused substep (no preamble, no rotation).
 ys_status enqueue_fused(ys_scene* s) {
     const StepArgs A = make_args(s);
+    if (const u32 blocks = refit_force_blocks(s)) {
+        ys_status r = clear_groups(s);
+        if (r) return r;
+        k_refit_forces<<<blocks, GROUP_THREADS, 0, s->stream>>>(s->gjobs.p + s->meshes.size(), s->gblk.p, s->ngblocks,
+                                                                substep_groups(s), A, s->nftiles);
+        s->gdirty = true;
+        launch_fused_classes(s, A);
+        s->fused_clears = !s->gdirty;
+        YS_CK(cudaGetLastError());
+        return YS_OK;
+    }
     // the forces beside the refit, on the scene's second stream; in turn
     // where other scenes fill the gaps (a graph with branches takes the host
     // twice as long to launch)
