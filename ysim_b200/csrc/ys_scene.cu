@@ -2419,7 +2419,8 @@ void drop_graphs(ys_scene* s) {
 }
 
 // Enqueue the device work of one fused substep (no preamble, no rotation).
-ys_status enqueue_fused(ys_scene* s) {
+// in_turn: the forces before the refit, not beside it.
+ys_status enqueue_fused(ys_scene* s, bool in_turn = false) {
     const StepArgs A = make_args(s);
     if (const u32 blocks = refit_force_blocks(s)) {
         ys_status r = clear_groups(s);
@@ -2435,7 +2436,7 @@ ys_status enqueue_fused(ys_scene* s) {
     // the forces beside the refit, on the scene's second stream; in turn
     // where other scenes fill the gaps (a graph with branches takes the host
     // twice as long to launch)
-    const bool fork = !s->load_vpw;
+    const bool fork = !s->load_vpw && !in_turn;
     if (fork) {
         YS_CK(cudaEventRecord(s->fork, s->stream));
         YS_CK(cudaStreamWaitEvent(s->side, s->fork, 0));
@@ -3849,12 +3850,10 @@ __global__ void k_mesh_unpack4(const float4* __restrict__ in, float* __restrict_
 
 #include "ys_adj64.cuh"
 
-// A whole pass of the binary32 rollout as a graph, from the second pass on (a
-// capture costs about one pass: 100 steps 12 ms, against 3 ms that it saves
-// each later one).  It starts from the first
-// buffers (cur 0, prev 1, velocity 0), so the buffers of every step are fixed;
-// epoch: the scene's captured-substep epoch it belongs to; the rest: the
-// scene's host state after the pass.
+// A whole pass of the binary32 rollout as a graph (adj_whole says when).  It
+// starts from the first buffers (cur 0, prev 1, velocity 0), so the buffers of
+// every step are fixed; epoch: the scene's captured-substep epoch it belongs
+// to; the rest: the scene's host state after the pass.
 struct AdjGraph {
     cudaGraphExec_t exec = nullptr;
     uint64_t runs = 0, epoch = 0, frame = 0;
@@ -3922,17 +3921,25 @@ void restore_state(ys_scene* s, const float4* x, const float4* xp, const float4*
     s->snapshot_pending = false;
 }
 
-// No substep of the rollout rebuilds a tree or reads a collider's pose, so a
-// pass is the same sequence of launches every time; up to ADJ_GRAPH_STEPS of
-// them go into one graph (a substep is four nodes; longer passes launch a graph
-// per substep).
-static constexpr u32 ADJ_GRAPH_STEPS = 1024;
-bool adj_capturable(const ys_adjoint* a) {
+// No substep of the rollout rebuilds a tree or reads a collider's pose: a pass
+// is the same sequence of launches every time.
+bool adj_plain(const ys_adjoint* a) {
     const ys_scene* s = a->s;
-    if (!s->use_graphs || s->timing || a->T > ADJ_GRAPH_STEPS || !s->shape_mesh.empty()) return false;
+    if (s->timing || !s->shape_mesh.empty()) return false;
     for (auto& H : s->meshes)
         if (H.needs_tree && !(H.built && H.d.behavior == YS_FLOAT)) return false;
     return true;
+}
+
+// Such a pass, after `runs` others, goes through one graph of up to
+// ADJ_GRAPH_STEPS substeps (two to four nodes each) once what capturing it
+// costs is about what it has not yet saved.  100 steps of small scenes: 3 ms
+// against 3 ms a pass (128 x 128: 10.2 enqueued, 6.9 replayed), so from the
+// second pass on; of those whose substeps have branches: 14 ms against 3 (200 x
+// 200: 11.7, 8.9), from the fifth.
+static constexpr u32 ADJ_GRAPH_STEPS = 1024;
+bool adj_whole(const ys_adjoint* a, uint64_t runs) {
+    return a->s->use_graphs && a->T <= ADJ_GRAPH_STEPS && adj_plain(a) && runs >= (refit_force_blocks(a->s) ? 1u : 4u);
 }
 
 // Run a pass through its graph; enqueue() issues the pass from the first
@@ -3972,14 +3979,17 @@ ys_status adj_graph(ys_adjoint* a, AdjGraph& G, u32 substeps, Fn&& enqueue) {
     return YS_OK;
 }
 
-// One substep of a pass under capture.
-ys_status adj_substep(ys_scene* s) {
-    const ys_status r = enqueue_fused(s);
+// One substep of a plain pass, under capture or enqueued: with a host call per
+// launch, fork and join the branches cost more than they save.
+ys_status adj_substep(ys_scene* s, bool captured) {
+    const ys_status r = enqueue_fused(s, !captured);
     if (r) return r;
     advance(s);
     if (s->record) s->last_contacts = 2;
     return YS_OK;
 }
+ys_status adj_captured(ys_scene* s) { return adj_substep(s, true); }
+ys_status adj_enqueued(ys_scene* s) { return adj_substep(s, false); }
 
 // ---- 64-bit mode
 void d64_drop_graphs(ys_adjoint* a);
@@ -4500,7 +4510,8 @@ ys_status ys_adjoint_forward(ys_adjoint* a, float* d_xT) {
         }
         return YS_OK;
     };
-    r = (a->c_fwd.runs++ && adj_capturable(a)) ? adj_graph(a, a->c_fwd, a->T, [&] { return pass(adj_substep); }) : pass(fused_substep);
+    if (adj_whole(a, a->c_fwd.runs++)) r = adj_graph(a, a->c_fwd, a->T, [&] { return pass(adj_captured); });
+    else r = pass(adj_plain(a) ? adj_enqueued : fused_substep);
     s->record = rec;
     if (r) return r;
     if (d_xT) k_mesh_unpack4<<<ceil_div(a->nV, 256), 256, 0, s->stream>>>(s->X[s->cur].p, d_xT, a->voff, a->nV);
@@ -4529,7 +4540,7 @@ ys_status ys_adjoint_backward(ys_adjoint* a, const float* d_dLdx, float* d_gk, f
         return YS_OK;
     }
     const size_t bytes = sizeof(float4) * s->nV;
-    const bool whole = a->c_bwd.runs++ && adj_capturable(a);
+    const bool whole = adj_whole(a, a->c_bwd.runs++);
     if (whole && !a->gk.p) {
         YS_CK(a->gk.alloc(a->S));
         YS_CK(a->gL.alloc(a->S));
@@ -4587,14 +4598,14 @@ ys_status ys_adjoint_backward(ys_adjoint* a, const float* d_dLdx, float* d_gk, f
         return q;
     };
     if (whole) {
-        r = adj_graph(a, a->c_bwd, a->T, [&] { return pass(adj_substep); });
+        r = adj_graph(a, a->c_bwd, a->T, [&] { return pass(adj_captured); });
         s->last_contacts = 2;
         if (!r) {
             YS_CK(cudaMemcpyAsync(d_gk, gk, 4 * (size_t)a->S, cudaMemcpyDeviceToDevice, st));
             YS_CK(cudaMemcpyAsync(d_gL, gL, 4 * (size_t)a->S, cudaMemcpyDeviceToDevice, st));
         }
     } else {
-        r = pass(fused_substep);
+        r = pass(adj_plain(a) ? adj_enqueued : fused_substep);
     }
     s->pool.p = keep_pool; s->vstart.p = keep_vs; s->vcount.p = keep_vc;  // also after a failed substep
     // dL/dv0 lies where T swaps put it; the buffers' names go back for the next pass
