@@ -173,20 +173,20 @@ ys_status ys_system_update(ys_scene* s);
 /* ---- Whole substeps ---------------------------------------------------- */
 /* n substeps through the staged kernels above (one launch group per stage). */
 ys_status ys_scene_step_staged(ys_scene* s, uint32_t n);
-/* n substeps through the fused path: refit + one kernel doing detect,
- * narrow, per-vertex contacts, spring forces and integration (same results
- * as the staged path). */
+/* n substeps through the fused path: refit, spring forces, and one kernel
+ * doing detect, narrow, per-vertex contacts and integration (same results as
+ * the staged path). */
 ys_status ys_scene_step(ys_scene* s, uint32_t n);
 /* Record the fused path's per-vertex contacts for inspection (slower). */
 ys_status ys_scene_set_record(ys_scene* s, int record);
-/* Replay each fused substep as a captured CUDA graph (default on; substeps
- * that rebuild trees, record contacts or time kernels run eagerly). */
+/* Replay fused substeps, and whole frames and rollout passes that recur, as
+ * captured CUDA graphs (default on; substeps that record contacts or time
+ * kernels run eagerly). */
 ys_status ys_scene_set_graphs(ys_scene* s, int on);
 /* Register cap of the fused substep kernel, as CTAs per SM (8: 64 registers,
  * 7: 72, 4: uncapped).  The results are the same for every value; the speed
- * depends on the scene (the self-colliding 262k-vertex cloth runs fastest at 7,
- * the batched FastGrid instances at 8).  No counterpart in the reference (its Metal pipelines have
- * fixed threadgroup sizes). */
+ * depends on the scene (ys_scene_autotune).  No counterpart in the reference
+ * (its Metal pipelines have fixed threadgroup sizes). */
 ys_status ys_scene_set_fused_variant(ys_scene* s, int min_blocks);
 /* Thread order of the fused substep kernel, for every size class.  Its
  * threads take the working vertices (cloth, moving or querying; static
@@ -209,22 +209,24 @@ ys_status ys_scene_set_thread_order(ys_scene* s, int order);
  * reports it (*chosen) and the mean milliseconds per variant (ms_out[3], in
  * the order 8, 7, 4; may be null).  No counterpart in the reference. */
 ys_status ys_scene_autotune(ys_scene* s, uint32_t reps, int* chosen, float* ms_out);
-/* The fused substep runs one launch per size class of the working meshes
- * (cloth, moving or querying meshes with at most 4096, 16384, 65536 vertices,
- * and larger; a batch of instances of mixed sizes spans several).  Each
- * class has its own register-cap variant and thread order. */
+/* The fused substep's working meshes fall into size classes (cloth, moving or
+ * querying meshes with at most 4096, 16384, 65536 vertices, and larger; a
+ * batch of instances of mixed sizes spans several).  Each class has its own
+ * register-cap variant and thread order; neighbouring classes of one variant
+ * share a launch. */
 typedef struct ys_fused_class {
     uint32_t max_mesh_vertices;  /* the class's bound on a mesh's vertex count */
     uint32_t meshes, vertices;   /* working meshes and vertices in the class */
     int32_t ctas_per_sm;         /* chosen variant (8, 7 or 4) */
     int32_t thread_order;        /* chosen thread order: YS_ORDER_VERTEX, _MORTON or _TILE */
-    float ms[3][3];              /* mean ms per launch: [vertex, Morton, tile order][8, 7, 4] */
+    float ms[3][3];              /* mean ms of a launch of the class alone: [vertex, Morton, tile order][8, 7, 4] */
 } ys_fused_class;
-/* Per-class autotuner: times every variant under each thread order on each
- * class's launch over the current state (the scene does not advance), keeps
- * the fastest pair per class and reports the classes (out: up to cap
- * records; *nclasses: the number of classes, 4).  No counterpart in the
- * reference. */
+/* Per-class autotuner: times every variant under each thread order on a launch
+ * of each class over the current state (the scene does not advance), then, as
+ * a substep makes them, the launches of each class's fastest pair and of one
+ * variant for every class, keeps the fastest of these and reports the classes
+ * (out: up to cap records; *nclasses: the number of classes, 4).  No
+ * counterpart in the reference. */
 ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* out, uint32_t cap,
                                     uint32_t* nclasses);
 /* Analytic collider (GeneralMesh::colliderKind and transform): kind

@@ -2188,7 +2188,7 @@ ys_status refresh_wide(ys_scene* s);
 // 213.7 us a substep with tickets, 209.9 with the memset; 2,048 blocks: equal;
 // 512: 18.4 against 20.5).
 static constexpr int CLEAR_BLOCKS = 4096;
-void launch_fused_classes(ys_scene* s, StepArgs A) {
+void launch_fused_classes(ys_scene* s, StepArgs A, bool clears = true) {
     const size_t n = s->cls_off.size() ? s->cls_off.size() - 1 : 0;
     for (size_t c = 0, e = 0; c < n; c = e) {
         for (e = c + 1; e < n; ++e)
@@ -2196,7 +2196,7 @@ void launch_fused_classes(ys_scene* s, StepArgs A) {
         A.tbase = s->cls_off[c];
         A.tend = s->cls_off[e];
         // the last launch: every reader of the refit's reductions is done
-        A.nclear = s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] &&
+        A.nclear = clears && s->tree_layout == YS_TREE_CUBE && A.tend > A.tbase && A.tend == s->cls_off[n] &&
                            ceil_div(A.tend - A.tbase, FUSED_WARPS * launch_vpw(A)) <= CLEAR_BLOCKS
                        ? (u32)s->gclear : 0u;
         launch_fused(A, s->stream, s->cls_variant[c]);
@@ -3357,7 +3357,10 @@ ys_status ys_scene_autotune(ys_scene* s, uint32_t reps, int* chosen, float* ms_o
 
 // Per size class: time each register-cap variant under each thread order on
 // the current state (the kernel writes only the next-state buffers; the
-// running totals are restored) and keep the fastest pair for the class.
+// running totals are restored).  Kept is the fastest of four sets of launches,
+// timed as a substep makes them (neighbouring classes of one cap share a
+// launch and its vertices per warp): every class its fastest pair, or one cap
+// for all, each with its fastest order.
 ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* out, uint32_t cap,
                                     uint32_t* nclasses) {
     ys_status r = check_scene(s);
@@ -3375,6 +3378,21 @@ ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* 
     YS_CK(cudaEventCreate(&e0));
     YS_CK(cudaEventCreate(&e1));
     float ms[NCLASS][3][3] = {};
+    std::vector<int> variant = s->cls_variant, orders = s->cls_order;
+    auto mean = [&](auto&& launch) {
+        launch();  // warm-up
+        float t = 0.f;
+        for (u32 k = 0; k < reps; ++k) {
+            cudaEventRecord(e0, st);
+            launch();
+            cudaEventRecord(e1, st);
+            cudaEventSynchronize(e1);
+            float m = 0.f;
+            cudaEventElapsedTime(&m, e0, e1);
+            t += m;
+        }
+        return t / (float)reps;
+    };
     for (int order = ORDER_VERTEX; order <= ORDER_TILE && !r; ++order) {
         for (auto& o : s->cls_order) o = order;
         if ((r = order_layout(s)) || (r = compute_order(s))) break;
@@ -3384,34 +3402,31 @@ ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* 
             A.tbase = s->cls_off[c];
             A.tend = s->cls_off[c + 1];
             if (A.tend <= A.tbase) continue;
-            for (int i = 0; i < 3; ++i) {
-                launch_fused(A, st, FUSED_VARIANTS[i]);  // warm-up
-                float t = 0.f;
-                for (u32 k = 0; k < reps; ++k) {
-                    cudaEventRecord(e0, st);
-                    launch_fused(A, st, FUSED_VARIANTS[i]);
-                    cudaEventRecord(e1, st);
-                    cudaEventSynchronize(e1);
-                    float m = 0.f;
-                    cudaEventElapsedTime(&m, e0, e1);
-                    t += m;
-                }
-                ms[c][order][i] = t / (float)reps;
-            }
+            for (int i = 0; i < 3; ++i)
+                ms[c][order][i] = mean([&] { launch_fused(A, st, FUSED_VARIANTS[i]); });
         }
+    }
+    float best = 1e30f;
+    for (int set = -1; set < 3 && !r; ++set) {  // -1: each class its fastest pair; else one cap
+        for (int c = 0; c < NCLASS; ++c) {
+            if (!s->cls_meshes[c]) continue;
+            int bo = ORDER_MORTON, bi = std::max(set, 0);
+            for (int o = ORDER_VERTEX; o <= ORDER_TILE; ++o)
+                for (int i = 0; i < 3; ++i)
+                    if ((set < 0 || i == set) && ms[c][o][i] < ms[c][bo][bi]) { bo = o; bi = i; }
+            s->cls_order[c] = bo;
+            s->cls_variant[c] = FUSED_VARIANTS[bi];
+        }
+        if ((r = order_layout(s)) || (r = compute_order(s))) break;
+        const StepArgs A = make_args(s);
+        const float t = mean([&] { launch_fused_classes(s, A, false); });
+        if (t < best) { best = t; variant = s->cls_variant; orders = s->cls_order; }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (!r) {
-        for (int c = 0; c < NCLASS; ++c) {
-            if (s->cls_off[c + 1] <= s->cls_off[c]) continue;
-            int bo = ORDER_MORTON, bi = 0;
-            for (int o = ORDER_VERTEX; o <= ORDER_TILE; ++o)
-                for (int i = 0; i < 3; ++i)
-                    if (ms[c][o][i] < ms[c][bo][bi]) { bo = o; bi = i; }
-            s->cls_order[c] = bo;
-            s->cls_variant[c] = FUSED_VARIANTS[bi];
-        }
+        s->cls_variant = variant;
+        s->cls_order = orders;
         if (!(r = order_layout(s))) r = compute_order(s);
     }
     YS_CK(cudaGetLastError());
