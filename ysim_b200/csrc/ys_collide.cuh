@@ -386,26 +386,33 @@ __device__ __forceinline__ bool narrow_one(f3 qcur, f3 qprev, f3 t0, f3 t1, f3 t
 // an ulp (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990).  A root of all ones is the exception that is
 // known there: its reciprocal may be off.  Root and reciprocal depend on |d|^2
-// alone; over every significand and both parities of the exponent they are
-// sqrtf's and the division's but for that exception.  The bounds on d keep
+// alone; the approximation's documented error would admit two significands
+// with a wrong root, so they rest on what this architecture's instruction
+// gives: over every significand and both parities of the exponent they are
+// sqrtf's and the division's but for that exception
+// (tests/test_gpu_unit_vector.py).  The bounds on d keep
 // every remainder exact.  One branch, where the root and the three divisions
 // have one each and so run one after another.  k_force_vertices on 262k
 // vertices of a triangle cloth: 33 -> 28 us.
-__device__ __forceinline__ bool unit_vector(f3 d, float& len, f3& u) {
-    const float s = dot(d, d);
+__device__ __forceinline__ void unit_root(float s, float& len, float& inv) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
     const float g = s * y;
     len = __fmaf_rn(__fmaf_rn(-g, g, s), 0.5f * y, g);
     y = __fmaf_rn(__fmaf_rn(-len, y, 1.f), y, y);
-    y = __fmaf_rn(__fmaf_rn(-len, y, 1.f), y, y);
-    auto quotient = [&](float a) {
-        float q = a * y;
-        q = __fmaf_rn(__fmaf_rn(-q, len, a), y, q);
-        q = __fmaf_rn(__fmaf_rn(-q, len, a), y, q);
-        return __uint_as_float((__float_as_uint(q) & 0x7FFFFFFFu) | (__float_as_uint(a) & 0x80000000u));  // -0 / len
-    };
-    u = mk(quotient(d.x), quotient(d.y), quotient(d.z));
+    inv = __fmaf_rn(__fmaf_rn(-len, y, 1.f), y, y);
+}
+__device__ __forceinline__ float unit_quotient(float a, float len, float inv) {
+    float q = a * inv;
+    q = __fmaf_rn(__fmaf_rn(-q, len, a), inv, q);
+    q = __fmaf_rn(__fmaf_rn(-q, len, a), inv, q);
+    return __uint_as_float((__float_as_uint(q) & 0x7FFFFFFFu) | (__float_as_uint(a) & 0x80000000u));  // -0 / len
+}
+__device__ __forceinline__ bool unit_vector(f3 d, float& len, f3& u) {
+    const float s = dot(d, d);
+    float y;
+    unit_root(s, len, y);
+    u = mk(unit_quotient(d.x, len, y), unit_quotient(d.y, len, y), unit_quotient(d.z, len, y));
     // 2^-60 <= s < 2^60, each component 0 or at least 2^-80, not all ones
     const u32 m = umin(umin(2u * __float_as_uint(d.x) - 1u, 2u * __float_as_uint(d.y) - 1u),
                        2u * __float_as_uint(d.z) - 1u);

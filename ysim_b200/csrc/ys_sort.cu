@@ -46,7 +46,10 @@ static constexpr int LT = 256, LI = 20;              // 5120 pairs
 static constexpr int ST = 256, SI = 8;               // 2048 pairs
 static constexpr int MT = 512, MI = 11;              // the one-CTA sort: what 48 KB of shared memory hold
 static constexpr u32 SMALL = MT * MI;
-static constexpr u32 LOOK_POLLS = 1u << 16;
+#ifndef YS_SORT_LOOK_POLLS  // a test builds this file with 0
+#define YS_SORT_LOOK_POLLS (1u << 16)
+#endif
+static constexpr u32 LOOK_POLLS = YS_SORT_LOOK_POLLS;
 static constexpr u32 LOOK = 8;         // words loaded together
 static constexpr u32 LOOK_GROUP = 16;  // tiles whose counts are summed into one word
 
