@@ -335,8 +335,11 @@ __global__ void __launch_bounds__(MT) k_sort_small(u32* __restrict__ keys, u32* 
 // Large tiles once there are enough of them to fill the chip (a pass of
 // 700,000 pairs 9.9 us in small tiles, of 1M 15.6 in small and 12.2 in large).
 static bool sort_large(u32 n) { return n >= 148u * LT * LI; }
-static u32 sort_tiles(u32 n, bool large) { return (u32)ceil_div(n, large ? LT * LI : ST * SI); }
-static u32 look_words(u32 tiles) { return 256u * (tiles + (u32)ceil_div(tiles, LOOK_GROUP)); }
+static constexpr u32 sort_tiles(u32 n, bool large) {
+    const u32 tile = large ? LT * LI : ST * SI;
+    return n / tile + (n % tile ? 1u : 0u);
+}
+static constexpr u32 look_words(u32 tiles) { return 256u * (tiles + (tiles + LOOK_GROUP - 1u) / LOOK_GROUP); }
 static constexpr size_t SORT_HEAD = 4 * 256 + 64;  // words: counts of 4 passes, tickets
 
 // Monotone in n: a scratch for n pairs serves every smaller sort.
@@ -444,7 +447,7 @@ ys_status fail(ys_status code, const std::string& msg);
 
 static constexpr u32 NOALLOC_MAX_PAIRS = 1u << 20;  // 1,048,576 pairs
 static constexpr size_t NOALLOC_SCRATCH_BYTES = 8651776;
-static_assert(4 * (SORT_HEAD + 256 * (NOALLOC_MAX_PAIRS / (LT * LI)) / LOOK_GROUP * (LOOK_GROUP + 1) + 2 * (size_t)NOALLOC_MAX_PAIRS) + 8 <=
+static_assert(4 * (SORT_HEAD + look_words(sort_tiles(NOALLOC_MAX_PAIRS, true)) + 2 * (size_t)NOALLOC_MAX_PAIRS) + 8 <=
                   NOALLOC_SCRATCH_BYTES,
               "the allocation-free sort's scratch holds the large tiles' words");
 static __device__ __align__(256) unsigned char g_noalloc_sort_scratch[NOALLOC_SCRATCH_BYTES];
