@@ -61,8 +61,7 @@ static constexpr u32 D64_CAP = 16;    // contacts kept per vertex and step
 // Bound on one warp's search in one obstacle, per vertex: candidates tested
 // and runs of 32 leaves opened; past it the search stops and the rollout fails.
 static constexpr u32 D64_STEPS = 1u << 24;
-// Block size of the per-vertex kernels (32 measured the same on the
-// 128x128 rollout: the step kernel is bound by its divergent descents).
+// Block size of the search, step and reverse kernels.
 static constexpr u32 D64_BLOCK = 128;
 
 // Order-preserving map of binary64 onto u64 (larger double, larger key), so

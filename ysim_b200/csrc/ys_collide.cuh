@@ -115,32 +115,6 @@ __device__ __forceinline__ u32 wide_step(const Wide4* __restrict__ w4, int w, f3
     return st;
 }
 
-// The same step with the pushes going through push(child), which returns
-// false when the stack is full.
-template <class Push, class Leaf>
-__device__ __forceinline__ u32 wide_step_p(const Wide4* __restrict__ w4, int w, f3 qmn, f3 qmx, Push&& push,
-                                           Leaf&& leaf) {
-    const float4* p = reinterpret_cast<const float4*>(w4 + w);
-    const float4 lx = __ldg(p), ly = __ldg(p + 1), lz = __ldg(p + 2);
-    const float4 hx = __ldg(p + 3), hy = __ldg(p + 4), hz = __ldg(p + 5);
-    const int4 ch = __ldg(reinterpret_cast<const int4*>(p + 6));
-    const float LX[4] = {lx.x, lx.y, lx.z, lx.w}, LY[4] = {ly.x, ly.y, ly.z, ly.w}, LZ[4] = {lz.x, lz.y, lz.z, lz.w};
-    const float HX[4] = {hx.x, hx.y, hx.z, hx.w}, HY[4] = {hy.x, hy.y, hy.z, hy.w}, HZ[4] = {hz.x, hz.y, hz.z, hz.w};
-    const int C[4] = {ch.x, ch.y, ch.z, ch.w};
-    u32 st = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int c = C[k];
-        if (c == W4_EMPTY || !overlap_xyz(qmn, qmx, LX[k], LY[k], LZ[k], HX[k], HY[k], HZ[k])) continue;
-        if (c < 0) {
-            leaf(k, (u32)~c);
-        } else if (!push(c)) {
-            st |= ST_STACK_OVF;
-        }
-    }
-    return st;
-}
-
 // Descent of the 4-wide form of a tree (same leaves as traverse on the binary
 // form): the root box first (binary root node), then wide nodes from 0.
 template <class Fn>

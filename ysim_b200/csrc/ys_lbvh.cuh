@@ -165,7 +165,8 @@ cudaError_t launch_karras(const u32* codes, const u32* idx, u32 n, Node* nodes, 
 // face-order pass computes the leaf boxes first, so the leaf pass reads them
 // in order instead of gathering facets and vertices; *nan becomes nonzero when
 // a leaf box has a NaN (the unions leave NaN out, a climb's tinym::min keeps
-// it or not by operand order).
+// it or not by operand order).  A minimum of zeros of both signs is -0 in a
+// union and the first operand's in a climb, a maximum +0; the values are equal.
 void launch_refit_bin(const RefitJob& J, const uint2* range, const u32* big, u32 nbig, const u32* huge, u32 nhuge,
                       const u32* rank, float4* lbox, cudaStream_t s, const u32* runs = nullptr, u32 nruns = 0,
                       const u32* reach = nullptr, u32* nan = nullptr);

@@ -2176,18 +2176,18 @@ ys_status encode_tile_maps(ys_scene* s) {
 
 ys_status refresh_wide(ys_scene* s);
 
-// The size classes' k_fused launches (classes do not interact: a launch
-// writes only its own vertices' next state).  Neighbouring classes of the same
-// register cap share one launch, smallest meshes
-// first: the few long warps of a small class then run beside the large
-// class's instead of before them (48 FastGrid instances of 16^2 to 256^2
-// vertices: 27 + 58 + 231 us one after another).
 // Up to this many blocks the fused kernel's last one clears for the next
 // substep; each block's ticket costs it about a microsecond at its end, which
 // above this is more than the memset and its gaps (8,208 blocks, 48 cloths:
 // 213.7 us a substep with tickets, 209.9 with the memset; 2,048 blocks: equal;
 // 512: 18.4 against 20.5).
 static constexpr int CLEAR_BLOCKS = 4096;
+// The size classes' k_fused launches (classes do not interact: a launch
+// writes only its own vertices' next state).  Neighbouring classes of the same
+// register cap share one launch, smallest meshes first: the few long warps of
+// a small class then run beside the large class's instead of before them (48
+// FastGrid instances of 16^2 to 256^2 vertices: 27 + 58 + 231 us one after
+// another).  clears: the last launch may clear for the next substep.
 void launch_fused_classes(ys_scene* s, StepArgs A, bool clears = true) {
     const size_t n = s->cls_off.size() ? s->cls_off.size() - 1 : 0;
     for (size_t c = 0, e = 0; c < n; c = e) {
@@ -2897,10 +2897,11 @@ ys_status ys_scene_pack(ys_scene* s) {
     }
     spr_off[nV] = (u32)spr_nbr.size();
     vaf_off[nV] = (u32)vaf.size();
-    // own-face windows: a vertex's faces, sorted, in at most two runs of 8
-    // ids each (a grid cloth's vertex: the two cell rows around it)
-    std::vector<uint2> ownw(nV, make_uint2(0u, 0u));
-    for (u32 gv = 0; gv < nV; ++gv) {
+    // own-face windows (the binary trees' descent): a vertex's faces, sorted, in
+    // at most two runs of 8 ids each (a grid cloth's vertex: the two cell rows
+    // around it)
+    std::vector<uint2> ownw(s->tree_layout == YS_TREE_REFERENCE ? nV : 0, make_uint2(0u, 0u));
+    for (u32 gv = 0; gv < ownw.size(); ++gv) {
         std::vector<u32> fs(vaf.begin() + vaf_off[gv], vaf.begin() + vaf_off[gv + 1]);
         if (fs.empty()) continue;
         std::sort(fs.begin(), fs.end());

@@ -335,8 +335,9 @@ ys_status ys_shash_build(ys_shash* h, const float* d_x, const uint32_t* d_facets
     YS_CK3(cudaStreamSynchronize(s));
     if (nE > h->maxEntries) return fail(YS_ERR_CAPACITY, "cell entries exceed the hash capacity");
     h->nE = nE;
-    // buckets for this build's entries (load factor at most 1/2): clearing
-    // and scanning a table sized for the capacity cost more than the build
+    // buckets for this build's entries (load factor at most 1/2, or 1 where it
+    // is halved below): clearing and scanning a table sized for the capacity
+    // cost more than the build
     u32 T = 1;
     while (T < 2u * std::max(nE, 1u) && T < h->tableCap) T <<= 1;
     int bits = 0;
