@@ -61,8 +61,8 @@ __device__ __forceinline__ void group_block(float4* __restrict__ l2, u32* __rest
 // Every box set, record, grid extent and root box of a substep in one launch:
 // the gathers of x (and v) are the dependent loads, every write is a
 // coalesced stream.  It replaces the 4-wide tree's refit in the fused
-// substep (leaf pass + range pass, 45 + 7.5 us on the 522,242-face cloth,
-// bound by its scattered slot writes; 21.8 us here).
+// substep (leaf pass + range pass, 48.8 + 10.9 us under ncu on the 522,242-face
+// cloth, bound by its scattered slot writes; 25.3 us here).
 __device__ __forceinline__ void refit_groups_block(const GroupJob* __restrict__ jobs, const u32* __restrict__ blkJob,
                                                    const float4* __restrict__ x, const float4* __restrict__ v,
                                                    const GroupBufs& B) {
