@@ -3360,8 +3360,9 @@ ys_status ys_scene_autotune(ys_scene* s, uint32_t reps, int* chosen, float* ms_o
 // the current state (the kernel writes only the next-state buffers; the
 // running totals are restored).  Kept is the fastest of four sets of launches,
 // timed as a substep makes them (neighbouring classes of one cap share a
-// launch and its vertices per warp): every class its fastest pair, or one cap
-// for all, each with its fastest order.
+// launch and its vertices per warp): every class its fastest pair, or, where
+// that is faster by more than the timings differ, one cap for all with each
+// class's fastest order.
 ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* out, uint32_t cap,
                                     uint32_t* nclasses) {
     ys_status r = check_scene(s);
@@ -3421,7 +3422,7 @@ ys_status ys_scene_autotune_classes(ys_scene* s, uint32_t reps, ys_fused_class* 
         if ((r = order_layout(s)) || (r = compute_order(s))) break;
         const StepArgs A = make_args(s);
         const float t = mean([&] { launch_fused_classes(s, A, false); });
-        if (t < best) { best = t; variant = s->cls_variant; orders = s->cls_order; }
+        if (t < 0.99f * best) { best = t; variant = s->cls_variant; orders = s->cls_order; }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
