@@ -2478,8 +2478,8 @@ void set_clock(ys_scene* s, const ys_scene_clock& c) {
 
 // Step calls on a device, for vertices_per_warp, which takes a chip that is
 // idle but for this launch: 256 grid cloths stepped in turn on their own
-// streams take 1.72 ms a round at their own sizes' vertices per warp and 0.83
-// at their sum's.  stepped: working vertices of every step call so far;
+// streams take 1.72 ms a turn at their own sizes' vertices per warp and 0.83 at
+// their sum's.  stepped: working vertices of every step call so far;
 // pending: those of the scenes that have stepped and not synchronised since.
 // The states do not depend on it.
 struct Load {
