@@ -565,7 +565,7 @@ __device__ __forceinline__ void force_tiles(const StepArgs& A, u32 first, u32 st
 }
 
 // The grid cloths' tiles, gridDim.x apart per CTA.  Bound
-// by instructions and the springs' dependent chains (0.68 issued a cycle).  A
+// by instructions and the springs' dependent chains (0.66 issued a cycle).  A
 // million vertices in 48 cloths (10,339 tiles): 79 us with the springs dealt
 // out family by family and a flag byte each, one tile per CTA; 64 us so; 56 us
 // with the branch-free unit vector.
