@@ -87,7 +87,7 @@ def _slots(tree):
 
 
 @pytest.mark.parametrize("scene", ["hash", "bvh"])
-@pytest.mark.parametrize("call", ["none", "update", "set", "rebuild", "tree"])
+@pytest.mark.parametrize("call", ["none", "update", "set", "set_again", "tune_set", "rebuild", "tree"])
 def test_trees_outlive_their_buffers(cuda_lib, scene, call):
     """Calls between the fused substep and the reading of its trees that write its buffers or rebuild some trees; the
     obstacle moves and is not rebuilt."""
@@ -99,16 +99,25 @@ def test_trees_outlive_their_buffers(cuda_lib, scene, call):
         spec.params.rebuild_frames = 1
     a, b = _pair(spec, "cube", spec.params.substeps)
     try:
+        if call == "tune_set":  # the tuner refits at the current state
+            a.autotune(reps=1)
+            b.broad_phase.refit_swept()
         for s in (a, b):
             if call == "update":
                 s.system.update()
-            elif call == "set":
-                for w in ("v", "xprev", "x"):
-                    s.set(w, s.get(w) + np.float32(0.25))
+            elif "set" in call:
+                for w in ("v", "xprev", "x") * (2 if call == "set_again" else 1):
+                    s.set(w, s.get(w) + np.float32(0.01))
             elif call == "rebuild":
                 s.broad_phase.build()
         if call == "tree":
             assert np.array_equal(a.tree(0)[0]["mn"], b.tree(0)[0]["mn"])
+        if "set" in call:
+            rows = []
+            for s in (a, b):
+                s.broad_phase.detect_collisions()
+                rows.append(canon_rows_full(s.rows()))
+            assert np.array_equal(rows[0], rows[1])
         for m in range(2):
             wa, wb = _slots(a.wide_tree(m)), _slots(b.wide_tree(m))
             assert len(wa) > 0 and np.array_equal(wa, wb)

@@ -1607,6 +1607,7 @@ struct ys_scene {
     DBuf<u32> gblk;                             // job of each block of the substep's refit
     std::vector<GroupJob> hgbuild;              // per mesh: its build job (flags 0: none)
     u32 ngjobs = 0, ngblocks = 0;
+    bool static_jobs = false;  // some refit job is a static mesh's
     int refit_stale = -1;  // buffer pair (cur * 2 + cv) of a refit that left the 4-wide trees behind, or -1
     DBuf<uint2> own;    // per vertex: its own faces as two 8-face windows (StepArgs::own)
     DBuf<Node> nodes;
@@ -2330,6 +2331,26 @@ ys_status refresh_wide(ys_scene* s) {
     s->cur = cur;
     s->cv = cv;
     return r;
+}
+
+// Before state `which` (0 x, 1 v, 2 xprev) is overwritten from outside: if the
+// refit left undone reads that buffer, its content moves to the one that the
+// next substep writes.  (The vertices of static meshes are written to every
+// buffer; a job of such a mesh needs its refit before.)
+ys_status keep_refit_buffers(ys_scene* s, int which) {
+    if (s->refit_stale < 0) return YS_OK;
+    const size_t bytes = sizeof(float4) * s->nV;
+    int x = s->refit_stale / 2, v = s->refit_stale % 2;
+    if (which == 1 && v == s->cv) {
+        YS_CK(cudaMemcpyAsync(s->V[1 - v].p, s->V[v].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+        v = 1 - v;
+    } else if (which != 1 && x == (which == 0 ? s->cur : s->prev)) {
+        const int next = 3 - s->cur - s->prev;
+        YS_CK(cudaMemcpyAsync(s->X[next].p, s->X[x].p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+        x = next;
+    }
+    s->refit_stale = x * 2 + v;
+    return YS_OK;
 }
 
 ys_status ensure_staged(ys_scene* s) {
@@ -3099,6 +3120,7 @@ ys_status ys_scene_pack(ys_scene* s) {
         if (!J.rootOnly && s->fpos.p) J.fpos = s->fpos.p + 3 * (size_t)H.foff;  // faces the fused kernel tests
         if (J.w4) { J.wrange = s->wrange.p + H.w4_off; J.idx = s->idx.p + H.foff; J.lvid = s->lvid.p + H.foff; }
         s->hjobs.push_back(J);
+        s->static_jobs = s->static_jobs || (H.flags & MF_STATIC);
         // every job's leaves start on a 256-leaf boundary (the range refit's
         // blocks then never hold two jobs)
         leaves = (leaves + J.n + 255u) & ~255u;
@@ -3498,7 +3520,7 @@ ys_status ys_scene_set_state(ys_scene* s, int which, const float* in) {
     if (r) return r;
     if (!in) return fail(YS_ERR_BAD_ARG, "null input");
     if (which < 0 || which > 2) return fail(YS_ERR_BAD_ARG, "bad state id");
-    if ((r = refresh_wide(s))) return r;
+    if ((r = which == 0 && s->static_jobs ? refresh_wide(s) : keep_refit_buffers(s, which))) return r;
     if (!s->scratch3.p) YS_CK(s->scratch3.alloc(3 * (size_t)s->nV));
     YS_CK(cudaMemcpyAsync(s->scratch3.p, in, 12 * (size_t)s->nV, cudaMemcpyHostToDevice, s->stream));
     // vertices of static meshes are never rewritten by a substep, so every
